@@ -697,16 +697,18 @@ extern "C" cudaError_t newt_pile_fused_prepare() {
 // One call's launches on `st`: the queue sort by last call's costs (when
 // `cost` and `queue` are given), then the gangs of launch shape `shape`.
 // `counter` must be zero when the gangs start (the caller clears it on `st`
-// first).  Every live world of the table advances `n_steps` env-steps.
+// first).  `before` (nullable) is recorded on `st` ahead of the gangs' launch.
+// Every live world of the table advances `n_steps` env-steps.
 extern "C" int newt_launch_pile_fused(const PileGroupDev* dG, const int* dwseg, int ng, int* queue, int n_items,
                                       int* counter, int n_steps, int grid, unsigned long long* work, unsigned* cost,
-                                      int nbm, int cm, int shape, cudaStream_t st) {
+                                      int nbm, int cm, int shape, cudaEvent_t before, cudaStream_t st) {
   if (n_items <= 0 || grid <= 0) return 0;
   int launches = 0;
   if (queue && cost) {
     pile_k_queue_sort<<<1, 1024, 0, st>>>(cost, n_items, queue);
     ++launches;
   }
+  if (before) cudaEventRecord(before, st);
   with_kernel(shape, [&](auto kern, int gang, int wpw) {
     kern<<<grid, 32 * gang, newt_pile_fused_smem_bytes(gang * wpw, nbm, cm), st>>>(dG, dwseg, ng, queue, n_items,
                                                                                    counter, n_steps, work, cost, nbm,

@@ -273,7 +273,7 @@ int newt_gpu_destroy(newt_gpu_ctx* ctx) {
   if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
   for (void* p : ctx->plan_bufs) cudaFree(p);
   for (void* p : ctx->plain_bufs) cudaFree(p);
-  if (ctx->side) cudaStreamDestroy(ctx->side);
+  for (cudaStream_t s : ctx->side) if (s) cudaStreamDestroy(s);
   for (int k = 0; k < 3; ++k) if (ctx->pside[k]) cudaStreamDestroy(ctx->pside[k]);
   for (int k = 0; k < 4; ++k) if (ctx->pev[k]) cudaEventDestroy(ctx->pev[k]);
   for (int b = 0; b < newt_gpu_ctx::PILE_BRANCHES; ++b) {

@@ -161,7 +161,7 @@ struct newt_gpu_ctx {
   bool graph_dirty = true;
   std::vector<void*> plan_bufs;  // device queues / group tables the graph reads
   int queue_items = 0;
-  cudaStream_t side = nullptr;   // second capture branch (tree persistent kernels)
+  cudaStream_t side[4] = {};     // capture branches of the tree launches, one per size bucket
   cudaStream_t pside[3] = {nullptr, nullptr, nullptr};  // pile island-class branches
   cudaEvent_t pev[4] = {nullptr, nullptr, nullptr, nullptr};
   // batched piles: world-range branches, each with its own main stream, three
@@ -250,7 +250,6 @@ int autotune_batched(newt_gpu_ctx* ctx, int n_steps, int horizon, int32_t* choic
 
 // kernel launchers (defined in the .cu kernel files)
 extern "C" int newt_tree_bucket(int L);
-extern "C" void newt_launch_tree_fused(const TreeGroupDev& g, int base, int count, int n_steps, cudaStream_t st);
 extern "C" void newt_launch_tree_plain(const TreeGroupDev& g, cudaStream_t st);
 extern "C" void newt_tc_offsets(int L, int nv, int ng, int maxc, int rpc, int* con, int* imp, int* misc);
 extern "C" size_t newt_tc_ws_bytes(int L, int nv, int ng, int maxc, int rpc);

@@ -21,9 +21,10 @@
     if (e_ != cudaSuccess) { ctx->err = std::string(#call ": ") + cudaGetErrorString(e_); return NEWT_E_CUDA; } \
   } while (0)
 
-extern "C" void newt_launch_tree_persistent(const TreeGroupDev* dgroups, const int* dqueue, int* dcounter, int n_items,
-                                            int bucket, int n_steps, int grid, cudaStream_t st);
-extern "C" int newt_tree_persistent_blocks_per_sm(int bucket);
+extern "C" void newt_launch_tree_lanes(const TreeGroupDev* dgroups, const int* dqueue, int n_items, int L, int serial,
+                                       int n_steps, int pct, cudaStream_t st);
+extern "C" cudaError_t newt_tree_lanes_prepare();
+extern "C" int newt_tree_item_worlds();
 extern "C" size_t newt_pile_ws_bytes(int nb, int np, int maxc);
 extern "C" int newt_launch_pile_step(const PileGroupDev* dG, const int* dwseg, int ng, int total_worlds,
                                      int total_slots, int* lists, int write_diag, cudaStream_t st,
@@ -33,7 +34,7 @@ extern "C" int newt_pile_fused_blocks_per_sm(int shape, int nbm, int cm);
 extern "C" int newt_pile_fused_worlds_per_block(int shape);
 extern "C" int newt_launch_pile_fused(const PileGroupDev* dG, const int* dwseg, int ng, int* queue, int n_items,
                                       int* counter, int n_steps, int grid, unsigned long long* work, unsigned* cost,
-                                      int nbm, int cm, int shape, cudaStream_t st);
+                                      int nbm, int cm, int shape, cudaEvent_t before, cudaStream_t st);
 extern "C" int newt_tc_prepare(newt_gpu_ctx* ctx, HostGroup* g, int n_steps);
 extern "C" size_t newt_pile_newton_bytes(int maxc);
 extern "C" int newt_launch_pile_solo_step(const PileGroupDev* dG, const int* dwseg, int ng, int total_worlds,
@@ -149,7 +150,9 @@ static void launch_pile_steps(newt_gpu_ctx* ctx, const PileTable& t, int n_steps
 static int ensure_pile_branches(newt_gpu_ctx* ctx) {
   if (ctx->pbs[0][0]) return NEWT_OK;
   for (int b = 0; b < newt_gpu_ctx::PILE_BRANCHES; ++b) {
-    for (int k = 0; k < 4; ++k) CKS(cudaStreamCreateWithFlags(&ctx->pbs[b][k], cudaStreamNonBlocking));
+    int least = 0, most = 0;  // the piles go before the tree launches beside them
+    CKS(cudaDeviceGetStreamPriorityRange(&least, &most));
+    for (int k = 0; k < 4; ++k) CKS(cudaStreamCreateWithPriority(&ctx->pbs[b][k], cudaStreamNonBlocking, most));
     for (int k = 0; k < 5; ++k) CKS(cudaEventCreateWithFlags(&ctx->pbe[b][k], cudaEventDisableTiming));
   }
   return NEWT_OK;
@@ -229,35 +232,37 @@ int step_plain(newt_gpu_ctx* ctx, int n_steps) {
 // ---------------------------------------------------------------------------
 static int capture(newt_gpu_ctx* ctx, int n_steps) {
   std::vector<void*> bufs;
-  // trees: one persistent launch per size bucket over a cost-sorted queue
-  struct TreeLaunch { int bucket; TreeGroupDev* dg; int* dq; int* dc; int items; int grid; };
+  // trees: one launch per size bucket over a cost-sorted queue, each on its
+  // own branch (the bucket's largest tree sizes the blocks' shared memory)
+  struct TreeLaunch { int L, serial; TreeGroupDev* dg; int* dq; int items; };
   std::vector<TreeLaunch> tls;
   const int buckets[4] = {8, 16, 32, 65};
   for (int bucket : buckets) {
-    struct It { long cost; int g, base, count; };
+    struct It { int cost, g, base, count; };
     std::vector<It> its;
     std::vector<TreeGroupDev> tg;
+    const int chunk = newt_tree_item_worlds();
+    int most = 0, serial = 1;
     for (auto& gp : ctx->groups) {
       HostGroup* g = gp.get();
       if (g->n == 0 || g->kind != GK_TREE || newt_tree_bucket(g->size) != bucket) continue;
+      for (int i = 1; i < g->size; ++i) serial &= g->topo[4 * i] == i - 1;
       int gi = (int)tg.size();
       tg.push_back(g->tree_dev());
-      const int chunk = 64;
-      for (int b = 0; b < g->n; b += chunk) its.push_back({(long)g->size, gi, b, std::min(chunk, g->n - b)});
+      most = std::max(most, g->size);
+      for (int b = 0; b < g->n; b += chunk) its.push_back({g->size, gi, b, std::min(chunk, g->n - b)});
     }
     if (its.empty()) continue;
     std::stable_sort(its.begin(), its.end(), [](const It& a, const It& b) { return a.cost > b.cost; });
     std::vector<int> q;
     for (auto& i : its) { q.push_back(i.g); q.push_back(i.base); q.push_back(i.count); }
-    TreeLaunch L{bucket, nullptr, nullptr, nullptr, (int)its.size(), 0};
+    TreeLaunch L{most, serial, nullptr, nullptr, (int)its.size()};
+    CKS(newt_tree_lanes_prepare());
     CKS(cudaMalloc(&L.dg, tg.size() * sizeof(TreeGroupDev)));
     CKS(cudaMemcpy(L.dg, tg.data(), tg.size() * sizeof(TreeGroupDev), cudaMemcpyHostToDevice));
     CKS(cudaMalloc(&L.dq, q.size() * sizeof(int)));
     CKS(cudaMemcpy(L.dq, q.data(), q.size() * sizeof(int), cudaMemcpyHostToDevice));
-    CKS(cudaMalloc(&L.dc, sizeof(int)));
-    bufs.push_back(L.dg); bufs.push_back(L.dq); bufs.push_back(L.dc);
-    const int full = newt_tree_persistent_blocks_per_sm(bucket) * sm_count(ctx);
-    L.grid = std::min(L.items, std::max(1, full * ctx->tune_tree_grid_pct / 100));
+    bufs.push_back(L.dg); bufs.push_back(L.dq);
     tls.push_back(L);
   }
   // facet-row PGS piles, largest worlds first; the piles solved apart
@@ -330,10 +335,13 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
     }
   if (!tcs.empty() && !ctx->tcstream) CKS(cudaStreamCreateWithFlags(&ctx->tcstream, cudaStreamNonBlocking));
 
-  cudaEvent_t fork = nullptr, join = nullptr, tjoin = nullptr;
-  if (!ctx->side) CKS(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+  cudaEvent_t fork = nullptr, pfork = nullptr, join[4] = {}, tjoin = nullptr;
   CKS(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
-  CKS(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+  CKS(cudaEventCreateWithFlags(&pfork, cudaEventDisableTiming));
+  for (size_t k = 0; k < tls.size(); ++k) {
+    if (!ctx->side[k]) CKS(cudaStreamCreateWithFlags(&ctx->side[k], cudaStreamNonBlocking));
+    CKS(cudaEventCreateWithFlags(&join[k], cudaEventDisableTiming));
+  }
   CKS(cudaEventCreateWithFlags(&tjoin, cudaEventDisableTiming));
   cudaGraph_t graph;
   if (ctx->profile && nbr > 0) {
@@ -345,12 +353,6 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
     if (t.ng > 0) ctx->graph_lists.push_back({t.lists, t.slots});
   CKS(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
   cudaEventRecord(fork, ctx->stream);
-  cudaStreamWaitEvent(ctx->side, fork, 0);
-  for (auto& L : tls) {
-    cudaMemsetAsync(L.dc, 0, sizeof(int), ctx->side);
-    newt_launch_tree_persistent(L.dg, L.dq, L.dc, L.items, L.bucket, n_steps, L.grid, ctx->side);
-  }
-  cudaEventRecord(join, ctx->side);
   int tc_timed = 0;
   const int64_t l0 = ctx->launches;
   if (!tcs.empty()) {
@@ -371,7 +373,7 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
     cudaMemsetAsync(ctx->fused_work, 0, 4 * sizeof(unsigned long long), fs);
     if (ctx->profile) cudaEventRecordWithFlags(ctx->fkev[0], fs, cudaEventRecordExternal);
     fused_launches = newt_launch_pile_fused(ft.dG, ft.dseg, ft.ng, fqueue, ft.worlds, fcounter, n_steps, fgrid,
-                                            ctx->fused_work, fcost, fnbm, fcm, ctx->tune_fused_shape, fs);
+                                            ctx->fused_work, fcost, fnbm, fcm, ctx->tune_fused_shape, pfork, fs);
     if (ctx->profile) cudaEventRecordWithFlags(ctx->fkev[1], fs, cudaEventRecordExternal);
     cudaEventRecord(ctx->pbe[0][4], fs);
     cudaStreamWaitEvent(ctx->stream, ctx->pbe[0][4], 0);
@@ -384,17 +386,28 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
     cudaEventRecord(ctx->pbe[b][4], bs[0]);
     cudaStreamWaitEvent(ctx->stream, ctx->pbe[b][4], 0);
   }
+  // The trees start once the persistent pile launch is under way: its blocks
+  // stay for the whole call, so one that found its SM set to the trees' large
+  // shared memory would keep the small L1 that goes with it (the uneven
+  // workload lost 5%).
+  for (size_t k = 0; k < tls.size(); ++k) {
+    const TreeLaunch& L = tls[k];
+    cudaStreamWaitEvent(ctx->side[k], fused && ft.ng > 0 ? pfork : fork, 0);
+    newt_launch_tree_lanes(L.dg, L.dq, L.items, L.L, L.serial, n_steps, ctx->tune_tree_grid_pct, ctx->side[k]);
+    cudaEventRecord(join[k], ctx->side[k]);
+  }
   const int pile_launches = (int)(ctx->launches - before) + fused_launches;
   ctx->launches = l0;
   ctx->graph_kev_steps = ctx->profile && nbr > 0 && pile_worlds > 0 ? n_steps : 0;
   ctx->graph_kev_branches = std::max(nbr, 1);
   ctx->graph_fused = fused && ft.ng > 0;
   ctx->graph_tc_steps = tc_timed;
-  cudaStreamWaitEvent(ctx->stream, join, 0);
+  for (size_t k = 0; k < tls.size(); ++k) cudaStreamWaitEvent(ctx->stream, join[k], 0);
   if (!tcs.empty()) cudaStreamWaitEvent(ctx->stream, tjoin, 0);
   cudaError_t ce = cudaStreamEndCapture(ctx->stream, &graph);
   cudaEventDestroy(fork);
-  cudaEventDestroy(join);
+  cudaEventDestroy(pfork);
+  for (size_t k = 0; k < tls.size(); ++k) cudaEventDestroy(join[k]);
   cudaEventDestroy(tjoin);
   if (ce != cudaSuccess) { ctx->err = cudaGetErrorString(ce); return NEWT_E_CUDA; }
   if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);

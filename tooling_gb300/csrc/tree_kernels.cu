@@ -11,12 +11,10 @@
 //   newt/src/aba.rs:803-1102    aba::run
 //   newt/src/tree.rs:1393-1475  euler_step_with_workspace / integrate_tree_positions
 //
-// Two forms:
-//   * fused  (`tree_fused_kernel`): the whole horizon in one launch; each
-//     thread keeps its world's state in registers/local memory and reads its
-//     model parameters (L1/L2-resident) every step.  Used by the batched path.
-//   * plain  (`tree_fk_kernel`, `tree_aba_kernel`, `tree_integrate_kernel`):
-//     one launch per stage per step with state round-tripping through HBM.
+// The plain form (`tree_aba_kernel`, `tree_integrate_kernel`): one launch per
+// stage per step with state round-tripping through HBM; also the stages
+// around the tree-contact solve.  The batched form of trees without contact
+// is tree_lanes.cu.
 #include "common.cuh"
 #include "groups.h"
 #include "../../include/newt_gpu.h"
@@ -251,59 +249,6 @@ __device__ __forceinline__ bool finite_all(const float* a, int n) {
 
 }  // namespace
 
-// One world's whole horizon with its state kept on-chip.
-template <int MAXL>
-__device__ __forceinline__ void tree_world_steps(const TreeGroupDev& g, int w, int n_steps) {
-  const int cap = g.cap, nq = g.nq, nv = g.nv;
-  float q[MAXL + 6], qd[MAXL + 5], qf[MAXL + 5], qdd[MAXL + 5];
-  for (int k = 0; k < nq; ++k) q[k] = g.q[k * cap + w];
-  for (int k = 0; k < nv; ++k) { qd[k] = g.qd[k * cap + w]; qf[k] = g.qfrc[k * cap + w]; qdd[k] = 0.f; }
-  LinkScratch scr[MAXL];
-  uint32_t st = 0;
-  const bool rk4 = is_rk4(g, w);
-  for (int s = 0; s < n_steps; ++s) {
-    if (rk4) {
-      if (!tree_rk4<MAXL>(g, w, q, qd, qf, qdd, scr)) st |= NEWT_WS_NOT_PD;
-      continue;
-    }
-    if (!tree_aba<MAXL>(g, w, q, qd, qf, qdd, scr, g.dtg[w])) st |= NEWT_WS_NOT_PD;
-    tree_integrate<MAXL>(g, w, q, qd, qdd);
-  }
-  if (!finite_all(q, nq) || !finite_all(qd, nv)) st |= NEWT_WS_NONFINITE;
-  for (int k = 0; k < nq; ++k) g.q[k * cap + w] = q[k];
-  for (int k = 0; k < nv; ++k) { g.qd[k * cap + w] = qd[k]; g.qacc[k * cap + w] = qdd[k]; }
-  if (st) g.status[w] |= st;
-}
-
-// Whole horizon in one launch over a contiguous range of one group.
-template <int MAXL>
-__global__ void __launch_bounds__(64) tree_fused_kernel(TreeGroupDev g, int base, int count, int n_steps) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= count) return;
-  const int w = base + t;
-  if (w >= g.n || !g.live[w]) return;
-  tree_world_steps<MAXL>(g, w, n_steps);
-}
-
-// Persistent form: blocks pull (group, base, count) items from a queue
-// sorted by size class (largest first) until it is drained.
-template <int MAXL>
-__global__ void __launch_bounds__(64) tree_persistent_kernel(const TreeGroupDev* groups, const int* queue,
-                                                             int* counter, int n_items, int n_steps) {
-  __shared__ int item;
-  for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) item = atomicAdd(counter, 1);
-    __syncthreads();
-    const int it = item;
-    if (it >= n_items) return;
-    const int gi = queue[3 * it], base = queue[3 * it + 1], count = queue[3 * it + 2];
-    const TreeGroupDev g = groups[gi];
-    const int w = base + (int)threadIdx.x;
-    if ((int)threadIdx.x < count && w < g.n && g.live[w]) tree_world_steps<MAXL>(g, w, n_steps);
-  }
-}
-
 // Plain form, stage 1+2: forward dynamics from HBM state into HBM qacc.
 template <int MAXL>
 __global__ void __launch_bounds__(128) tree_aba_kernel(TreeGroupDev g) {
@@ -367,37 +312,6 @@ __global__ void __launch_bounds__(128) tree_integrate_kernel(TreeGroupDev g) {
 #define NEWT_TREE_BUCKETS(X) X(8) X(16) X(32) X(65)
 
 extern "C" int newt_tree_bucket(int L) { return L <= 8 ? 8 : L <= 16 ? 16 : L <= 32 ? 32 : 65; }
-
-extern "C" void newt_launch_tree_fused(const TreeGroupDev& g, int base, int count, int n_steps, cudaStream_t st) {
-  const int B = 64;
-  int grid = (count + B - 1) / B;
-  if (grid == 0) return;
-  switch (newt_tree_bucket(g.L)) {
-#define X(M) case M: tree_fused_kernel<M><<<grid, B, 0, st>>>(g, base, count, n_steps); break;
-    NEWT_TREE_BUCKETS(X)
-#undef X
-  }
-}
-
-extern "C" void newt_launch_tree_persistent(const TreeGroupDev* dgroups, const int* dqueue, int* dcounter, int n_items,
-                                            int bucket, int n_steps, int grid, cudaStream_t st) {
-  if (grid <= 0 || n_items <= 0) return;
-  switch (bucket) {
-#define X(M) case M: tree_persistent_kernel<M><<<grid, 64, 0, st>>>(dgroups, dqueue, dcounter, n_items, n_steps); break;
-    NEWT_TREE_BUCKETS(X)
-#undef X
-  }
-}
-
-extern "C" int newt_tree_persistent_blocks_per_sm(int bucket) {
-  int nb = 1;
-  switch (bucket) {
-#define X(M) case M: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, tree_persistent_kernel<M>, 64, 0); break;
-    NEWT_TREE_BUCKETS(X)
-#undef X
-  }
-  return nb < 1 ? 1 : nb;
-}
 
 // The sensors' dynamics pass for trees without geoms (newt/src/sensor.rs:
 // 446-530, 834-1000): qddot from the explicit ABA at the world's current
