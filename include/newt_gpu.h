@@ -193,10 +193,10 @@ NEWT_API int newt_gpu_set_qfrc(newt_gpu_ctx* ctx, const int32_t* slots, int32_t 
  * mode NEWT_STEP_PLAIN: one launch per stage per step, fixed tiles.
  * mode NEWT_STEP_BATCHED: the whole call captured in one CUDA graph and
  *   replayed: trees run the horizon in one persistent launch per size bucket
- *   over a cost-sorted queue; pile worlds of every size run theirs in one
- *   world-persistent launch (a warp per world for the whole horizon, worlds
- *   pulled from a queue sorted by the previous call's cost, most costly
- *   first); tree-contact worlds run their three kernels per env-step on a
+ *   over a cost-sorted queue; pile worlds of every size run two launches per
+ *   env-step and size class (contacts, then sweeps and integration, over a
+ *   queue sorted by the previous call's cost, most costly first), each class
+ *   on a branch of the graph; tree-contact worlds run their three kernels per env-step on a
  *   branch of the graph.  newt_gpu_autotune may instead pick the
  *   island-class pipeline for piles (collide, island-class solvers on forked
  *   streams, integrate, per env-step).  Pile worlds under the Newton solver
@@ -355,10 +355,8 @@ NEWT_API int newt_gpu_flush_l2(newt_gpu_ctx* ctx);                              
 /* Kernel launches issued by this context since creation. */
 NEWT_API int64_t newt_gpu_launch_count(const newt_gpu_ctx* ctx);
 /* Times the batched step's launch choices on the live worlds (piles in the
- * world-persistent launch in each of its shapes -- gangs of 4 to 32 warps,
- * one to four gangs per SM, with or without a barrier between assembly and
- * sweeps, one or two worlds per warp --
- * or in the island-class pipeline with 1, 2 or 3 world-range branches; tree
+ * batched launches in each of their shapes -- 8, 16 or 32 lanes per world in
+ * the sweeps, 2, 4, 6 or 8 warps per block in the contact stage -- or in the island-class pipeline with 1, 2 or 3 world-range branches; tree
  * persistent grid at full or half residency), `n_steps` env-steps per trial,
  * and keeps the fastest for later NEWT_STEP_BATCHED calls.  `horizon` is how
  * many env-steps the caller means to run next (<= 0: 8 x n_steps): every
@@ -366,16 +364,16 @@ NEWT_API int64_t newt_gpu_launch_count(const newt_gpu_ctx* ctx);
  * horizon/2 and horizon env-steps later (falling piles land and their
  * islands grow) -- and judged by the trapezoid average over the horizon
  * (weights 1/4, 1/2, 1/4).  Every world's state is left as it was.
- * `choice` (nullable, 5 ints): pile branches (0 for the persistent launch),
+ * `choice` (nullable, 5 ints): pile branches (0 for the batched launches),
  * tree grid percent, the winner's averaged time per trial in microseconds,
- * 1 if piles use the persistent launch, its shape index (0: 16 warps; 1: 12
- * warps; 2: 12 warps, one barrier per env-step; 3: 8 warps; 4: 24 warps; 5:
- * 32 warps).  No counterpart in newt. */
+ * 1 if piles use the batched launches, their shape index 0..11 (9..11 leave
+ * the lanes to the worlds' size and number; 10 is the default).  No
+ * counterpart in newt. */
 NEWT_API int newt_gpu_autotune(newt_gpu_ctx* ctx, int32_t n_steps, int32_t horizon, int32_t* choice);
 /* Sets the batched step's launch choices directly, in newt_gpu_autotune's
  * `choice` layout: [0] pile world-range branches of the island-class
  * pipeline (0: by world count), [1] tree persistent grid percent, [2]
- * ignored, [3] 1 for the world-persistent pile launch, 0 for the pipeline,
+ * ignored, [3] 1 for the batched pile launches, 0 for the pipeline,
  * [4] its shape index (newt_gpu_autotune).  No counterpart in newt. */
 NEWT_API int newt_gpu_set_launch_choice(newt_gpu_ctx* ctx, const int32_t* choice);
 /* Device bytes the world groups hold (capacity x bytes per world: model,

@@ -378,7 +378,7 @@ class Engine:
     def set_launch_choice(self, persistent: bool = True, persistent_shape: int = 10, pile_branches: int = 0,
                           tree_grid_pct: int = 100):
         """Pin the batched step's launch choices (what autotune() would pick):
-        piles in the world-persistent launch of shape `persistent_shape`, or
+        piles in the batched launches of shape `persistent_shape`, or
         in the island-class pipeline with `pile_branches` world-range
         branches (0: by world count)."""
         c = np.array([pile_branches, tree_grid_pct, 0, int(bool(persistent)), persistent_shape], np.int32)
@@ -401,9 +401,9 @@ class Engine:
         return dict(zip(TC_KERNELS, ms.tolist()))
 
     def fused_profile(self):
-        """(device ms of the last batched call's world-persistent pile launch,
-        or 0 when it was not timed; {contacts, rounds, levels, worlds} summed
-        over that launch's worlds and env-steps)."""
+        """(device ms of the last batched call's pile launches, all env-steps,
+        or 0 when they were not timed; {contacts, rounds, levels, worlds}
+        summed over their worlds and env-steps)."""
         ms = C.c_float()
         w = np.zeros(4, np.uint64)
         self._ck(self.L.newt_gpu_pile_fused_profile(self.ctx, C.byref(ms), _p(w)))

@@ -165,7 +165,10 @@ static __device__ __noinline__ int np_round_pair(int sa, int sb, GPose pa, GPose
   return 0;
 }
 
-NEWT_D void collide(const WsLay& L, float* wf, int* wi, int lane) {
+// `put(c, pos, n, pen, mu, ga, gb, ea, eb)` takes contact c (world geoms ga <
+// gb, entities ea, eb: bodies below nb, planes from it on).
+template <class Put>
+NEWT_D void collide(const WsLay& L, float* wf, int* wi, int lane, Put put) {
   const int ng = L.ng, nb = L.nb, W = L.words;
   // AABBs per geom index (newt/src/broadphase.rs:708-756); planes unbounded
   for (int k = lane; k < ng; k += 32) {
@@ -319,13 +322,9 @@ NEWT_D void collide(const WsLay& L, float* wf, int* wi, int lane) {
     for (int k = 0; k < cnt; ++k) {
       int c = off + k;
       if (c >= L.maxc) { overflow = 1; break; }
-      float* cf = wf + L.con + CF * c;
-      int* cc = wi + L.ci + CI * c;
       V3 n = flip ? -res[k].n : res[k].n;
-      st3(cf + C_POS, res[k].pos); st3(cf + C_N, n); cf[C_PEN] = res[k].pen;
       int ea = wi[L.gent + ga], eb = wi[L.gent + gb];
-      cf[C_MU] = fminf(wf[L.fric + ea], wf[L.fric + eb]);
-      cc[0] = ga; cc[1] = gb; cc[2] = ea; cc[3] = eb;
+      put(c, res[k].pos, n, res[k].pen, fminf(wf[L.fric + ea], wf[L.fric + eb]), ga, gb, ea, eb);
     }
     nc += __shfl_sync(0xffffffffu, incl, 31);
   }
@@ -338,5 +337,15 @@ NEWT_D void collide(const WsLay& L, float* wf, int* wi, int lane) {
   __syncwarp();
 }
 
+// The same into the scratch record's contacts.
+NEWT_D void collide(const WsLay& L, float* wf, int* wi, int lane) {
+  collide(L, wf, wi, lane, [&](int c, V3 pos, V3 n, float pen, float mu, int ga, int gb, int ea, int eb) {
+    float* cf = wf + L.con + CF * c;
+    int* cc = wi + L.ci + CI * c;
+    st3(cf + C_POS, pos); st3(cf + C_N, n); cf[C_PEN] = pen;
+    cf[C_MU] = mu;
+    cc[0] = ga; cc[1] = gb; cc[2] = ea; cc[3] = eb;
+  });
+}
 
 }  // namespace pile

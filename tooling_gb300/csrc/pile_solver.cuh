@@ -1,7 +1,7 @@
 // Free-body contact pipeline: the per-row and per-body pieces that every
 // pile solver shares (the per-class kernels of pile_kernels.cu and the
-// world-persistent kernel of pile_fused.cu), so both run the same
-// arithmetic for soft-constraint parameters, PGS row steps and integration.
+// batched kernels of pile_batched.cu), so both run the same arithmetic for
+// soft-constraint parameters and integration.
 //
 // Restates, for FP32 on sm_103a:
 //   newt/src/solver.rs:301-326    impedance_at_position (effective_solimp)
@@ -71,6 +71,10 @@ NEWT_D int find_seg(const int* seg, int ng, int t) {
 // ---------------------------------------------------------------------------
 // K4: integration + write-back (world.rs:1790-1817, 3223-3245)
 // ---------------------------------------------------------------------------
+struct BodyState { V3 p; Q4 q; V3 v, w; };  // position, orientation, linear and (body-frame) angular velocity
+// the body's model and the sweeps' velocity changes (world frame)
+struct BodyPush { S3 inert, iinv; V3 dv, dw; };
+
 // One body's RK4 step under the solver's wrench held constant over the four
 // stages (newt/src/world.rs:1705-1788, stage derivative world.rs:3223-3245,
 // stage states world.rs:3258-3271).  The wrench comes back from the velocity
@@ -78,12 +82,12 @@ NEWT_D int find_seg(const int* seg, int ng, int t) {
 // R0 Ib R0^T dw / dt.  Stage orientations are not renormalised; the final one
 // is, by division (newt/src/math.rs:591-598).  Returns true on a non-finite
 // result.
-__device__ __forceinline__ bool pile_rk4_body(float* wf, const WsLay& L, int b, float dt, V3 grav) {
-  const V3 p0 = ld3(wf + L.pos + 3 * b), v0 = ld3(wf + L.vel + 3 * b), w0 = ld3(wf + L.omg + 3 * b);
-  const Q4 q0 = ld4(wf + L.quat + 4 * b);
-  const S3 Ib = lds(wf + L.inertb + 6 * b), Ibi = lds(wf + L.iinvb + 6 * b);
-  const V3 alin = grav + ld3(wf + L.dv + 3 * b) / dt;
-  const V3 tau = qrot(q0, smv(Ib, qrot_inv(q0, ld3(wf + L.dw + 3 * b)))) / dt;
+__device__ __forceinline__ bool body_rk4(BodyState& s, const BodyPush& f, float dt, V3 grav) {
+  const V3 p0 = s.p, v0 = s.v, w0 = s.w;
+  const Q4 q0 = s.q;
+  const S3 Ib = f.inert, Ibi = f.iinv;
+  const V3 alin = grav + f.dv / dt;
+  const V3 tau = qrot(q0, smv(Ib, qrot_inv(q0, f.dw))) / dt;
   auto dang_at = [&](Q4 q, V3 om) {
     const V3 gyro = -cross(om, smv(Ib, om));
     return smv(Ibi, qrot_inv(q, tau) + gyro);
@@ -120,10 +124,25 @@ __device__ __forceinline__ bool pile_rk4_body(float* wf, const WsLay& L, int b, 
   Q4 nq = qstep(q0, dq, dt);
   const float n = sqrtf(nq.x * nq.x + nq.y * nq.y + nq.z * nq.z + nq.w * nq.w);
   nq = n == 0.f ? Q4{0.f, 0.f, 0.f, 1.f} : Q4{nq.x / n, nq.y / n, nq.z / n, nq.w / n};
-  st3(wf + L.pos + 3 * b, p); st3(wf + L.vel + 3 * b, lv); st3(wf + L.omg + 3 * b, av);
-  wf[L.quat + 4 * b] = nq.x; wf[L.quat + 4 * b + 1] = nq.y; wf[L.quat + 4 * b + 2] = nq.z; wf[L.quat + 4 * b + 3] = nq.w;
+  s = BodyState{p, nq, lv, av};
   return !(isfinite(p.x) && isfinite(p.y) && isfinite(p.z) && isfinite(lv.x) && isfinite(lv.y) && isfinite(lv.z) &&
            isfinite(av.x) && isfinite(av.y) && isfinite(av.z) && isfinite(nq.w));
+}
+
+// One body's semi-implicit Euler step; returns true on a non-finite result.
+__device__ __forceinline__ bool body_euler(BodyState& s, const BodyPush& f, float dt, V3 grav) {
+  Q4 q = s.q;
+  V3 om = s.w;
+  V3 iw = smv(f.inert, om);
+  V3 gyro = -cross(om, iw);
+  V3 dang = smv(f.iinv, gyro);
+  V3 lv = s.v + grav * dt + f.dv;
+  V3 av = om + dang * dt + qrot_inv(q, f.dw);
+  V3 p = s.p + lv * dt;
+  Q4 nq = q_integrate(q, av, dt);
+  s = BodyState{p, nq, lv, av};
+  return !(isfinite(p.x) && isfinite(p.y) && isfinite(p.z) && isfinite(lv.x) && isfinite(lv.y) && isfinite(lv.z) &&
+           isfinite(av.x) && isfinite(av.y) && isfinite(av.z));
 }
 
 // Semi-implicit Euler (or RK4 under the solver's wrench held over the
@@ -136,23 +155,11 @@ NEWT_D bool pile_integrate_world(float* wf, const WsLay& L, bool rk4, int lane) 
   const V3 grav = v3(wf[L.dtg + 1], wf[L.dtg + 2], wf[L.dtg + 3]);
   bool bad = false;
   for (int b = lane; b < L.nb; b += 32) {
-    if (rk4) {
-      bad |= pile_rk4_body(wf, L, b, dt, grav);
-      continue;
-    }
-    Q4 q = ld4(wf + L.quat + 4 * b);
-    V3 om = ld3(wf + L.omg + 3 * b);
-    V3 iw = smv(lds(wf + L.inertb + 6 * b), om);
-    V3 gyro = -cross(om, iw);
-    V3 dang = smv(lds(wf + L.iinvb + 6 * b), gyro);
-    V3 lv = ld3(wf + L.vel + 3 * b) + grav * dt + ld3(wf + L.dv + 3 * b);
-    V3 av = om + dang * dt + qrot_inv(q, ld3(wf + L.dw + 3 * b));
-    V3 p = ld3(wf + L.pos + 3 * b) + lv * dt;
-    Q4 nq = q_integrate(q, av, dt);
-    st3(wf + L.pos + 3 * b, p); st3(wf + L.vel + 3 * b, lv); st3(wf + L.omg + 3 * b, av);
-    wf[L.quat + 4 * b] = nq.x; wf[L.quat + 4 * b + 1] = nq.y; wf[L.quat + 4 * b + 2] = nq.z; wf[L.quat + 4 * b + 3] = nq.w;
-    bad |= !(isfinite(p.x) && isfinite(p.y) && isfinite(p.z) && isfinite(lv.x) && isfinite(lv.y) && isfinite(lv.z) &&
-             isfinite(av.x) && isfinite(av.y) && isfinite(av.z));
+    BodyState s{ld3(wf + L.pos + 3 * b), ld4(wf + L.quat + 4 * b), ld3(wf + L.vel + 3 * b), ld3(wf + L.omg + 3 * b)};
+    const BodyPush f{lds(wf + L.inertb + 6 * b), lds(wf + L.iinvb + 6 * b), ld3(wf + L.dv + 3 * b), ld3(wf + L.dw + 3 * b)};
+    bad |= rk4 ? body_rk4(s, f, dt, grav) : body_euler(s, f, dt, grav);
+    st3(wf + L.pos + 3 * b, s.p); st3(wf + L.vel + 3 * b, s.v); st3(wf + L.omg + 3 * b, s.w);
+    wf[L.quat + 4 * b] = s.q.x; wf[L.quat + 4 * b + 1] = s.q.y; wf[L.quat + 4 * b + 2] = s.q.z; wf[L.quat + 4 * b + 3] = s.q.w;
   }
   bad = __any_sync(0xffffffffu, bad);
   __syncwarp();

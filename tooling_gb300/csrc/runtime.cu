@@ -604,15 +604,15 @@ int newt_gpu_autotune(newt_gpu_ctx* ctx, int32_t n_steps, int32_t horizon, int32
   return rc;
 }
 
-extern "C" int newt_pile_fused_shapes();
+extern "C" int newt_pile_batched_shapes();
 
 int newt_gpu_set_launch_choice(newt_gpu_ctx* ctx, const int32_t* choice) {
   if (!ctx || !choice) return NEWT_E_INVALID;
   const int branches = choice[0], tree_pct = choice[1], fused = choice[3], shape = choice[4];
   if (branches < 0 || branches > newt_gpu_ctx::PILE_BRANCHES || tree_pct < 1 || tree_pct > 100 || fused < 0 ||
-      fused > 1 || shape < 0 || shape >= newt_pile_fused_shapes()) {
+      fused > 1 || shape < 0 || shape >= newt_pile_batched_shapes()) {
     ctx->err = "newt_gpu_set_launch_choice: pile branches 0..3, tree grid percent 1..100, persistent flag 0 or 1, "
-               "persistent shape 0.." + std::to_string(newt_pile_fused_shapes() - 1);
+               "persistent shape 0.." + std::to_string(newt_pile_batched_shapes() - 1);
     return NEWT_E_INVALID;
   }
   ctx->tune_branches = branches;

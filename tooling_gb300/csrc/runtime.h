@@ -170,13 +170,12 @@ struct newt_gpu_ctx {
   // launch choices of the batched form (newt_gpu_autotune): pile branches
   // (0: by world count), tree persistent grid in percent of full residency
   int tune_branches = 0, tune_tree_grid_pct = 100;
-  // pile worlds in the batched form: 1 = one world-persistent launch over a
-  // cost-sorted queue (pile_fused.cu), 0 = the island-class pipeline per
-  // env-step; the persistent launch's shape (gang size and barriers, an
-  // index into pile_fused.cu's shape table) and grid in percent of full
-  // residency (default: gangs of 8 warps, two per SM, meeting once per
-  // env-step, the fastest shape on 8192 sixteen-body piles)
-  int tune_pile_fused = 1, tune_fused_shape = 10, tune_fused_pct = 100;
+  // pile worlds in the batched form: 1 = two launches per env-step over a
+  // cost-sorted queue (pile_batched.cu), 0 = the island-class pipeline per
+  // env-step; the launches' shape (an index into pile_batched.cu's table;
+  // default: lanes by the worlds' size and number, eight warps per block in
+  // the contact stage, the fastest on 8192 sixteen-body piles)
+  int tune_pile_fused = 1, tune_fused_shape = 10;
   // the persistent launch of the captured graph: its timing events (external
   // records when profiling), its work counters (device: contacts, rounds,
   // levels, worlds) and whether the graph holds one; `last_fused` tells the

@@ -5,10 +5,10 @@
 // Batched form: the whole call is captured once in a CUDA graph and
 // replayed.  Trees run their horizon in one persistent launch per size
 // bucket, pulling work items from a device queue sorted by size class;
-// pile worlds of every size run theirs in one world-persistent launch over
-// a size-sorted queue (pile_fused.cu; the island-class pipeline, one launch
+// pile worlds run two launches per env-step and size class over a
+// cost-sorted queue (pile_batched.cu; the island-class pipeline, one launch
 // per stage per env-step, stays available to the autotuner); tree-contact
-// worlds run their per-env-step kernels on a third branch of the same graph.
+// worlds run their per-env-step kernels on another branch of the same graph.
 #include <algorithm>
 #include <cstdio>
 #include <vector>
@@ -30,11 +30,14 @@ extern "C" int newt_launch_pile_step(const PileGroupDev* dG, const int* dwseg, i
                                      int total_slots, int* lists, int write_diag, cudaStream_t st,
                                      const cudaStream_t* side, cudaEvent_t* ev, cudaEvent_t* kev);
 extern "C" void newt_pile_init();
-extern "C" int newt_pile_fused_blocks_per_sm(int shape, int nbm, int cm);
-extern "C" int newt_pile_fused_worlds_per_block(int shape);
-extern "C" int newt_launch_pile_fused(const PileGroupDev* dG, const int* dwseg, int ng, int* queue, int n_items,
-                                      int* counter, int n_steps, int grid, unsigned long long* work, unsigned* cost,
-                                      int nbm, int cm, int shape, cudaEvent_t before, cudaStream_t st);
+struct PileBatchedPlan { int lanes, warps, stride, space, nbm; };  // pile_batched.cu
+extern "C" int newt_pile_batched_class(int nb);
+extern "C" cudaError_t newt_pile_batched_plan(int shape, int worlds, int sms, int nbm, int cm, int stride,
+                                              PileBatchedPlan* p);
+extern "C" int newt_pile_batched_words(const PileGroupDev* g);
+extern "C" int newt_launch_pile_batched(const PileGroupDev* dG, const int* dwseg, int ng, int* queue, int n,
+                                        int n_steps, unsigned long long* work, unsigned* cost,
+                                        const PileBatchedPlan* p, cudaStream_t st);
 extern "C" int newt_tc_prepare(newt_gpu_ctx* ctx, HostGroup* g, int n_steps);
 extern "C" size_t newt_pile_newton_bytes(int maxc);
 extern "C" int newt_launch_pile_solo_step(const PileGroupDev* dG, const int* dwseg, int ng, int total_worlds,
@@ -288,13 +291,16 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
   }
   std::stable_sort(piles.begin(), piles.end(), [](HostGroup* a, HostGroup* b) { return a->size > b->size; });
   const bool fused = ctx->tune_pile_fused != 0;
-  // fused: one table over every pile group; its flat world order is the
-  // queue (groups by size, largest first)
-  PileTable ft;
-  int* fcounter = nullptr;
-  int* fqueue = nullptr;
-  unsigned* fcost = nullptr;
-  int fgrid = 0, fnbm = 0, fcm = 0;
+  // fused: two launches per env-step and size class, each class with its own
+  // table, whose flat world order is the first queue (groups by size, largest
+  // first), and on its own branch
+  struct BatchedLaunch {
+    PileTable t;
+    PileBatchedPlan plan;
+    int* queue;
+    unsigned* cost;
+  };
+  std::vector<BatchedLaunch> bls;
   const int nbr = fused ? 0
                         : (ctx->tune_branches > 0 ? std::min(ctx->tune_branches, newt_gpu_ctx::PILE_BRANCHES)
                                                   : (int)std::max<long>(1, std::min<long>(2, pile_worlds / 4096)));
@@ -304,22 +310,34 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
     if (rc != NEWT_OK) return rc;
   }
   if (fused && pile_worlds > 0) {
-    int rc = build_pile_table(ctx, piles, ft, bufs, 0, 1);
-    if (rc != NEWT_OK) return rc;
-    CKS(cudaMalloc(&fcounter, sizeof(int)));
-    CKS(cudaMalloc(&fqueue, sizeof(int) * (size_t)ft.worlds));
-    CKS(cudaMalloc(&fcost, sizeof(unsigned) * (size_t)ft.worlds));
-    CKS(cudaMemset(fcost, 0, sizeof(unsigned) * (size_t)ft.worlds));  // first call: any order
-    bufs.push_back(fcounter);
-    bufs.push_back(fqueue);
-    bufs.push_back(fcost);
     if (!ctx->fused_work) CKS(cudaMalloc(&ctx->fused_work, 4 * sizeof(unsigned long long)));
     if (!ctx->fkev[0])
       for (int k = 0; k < 2; ++k) CKS(cudaEventCreate(&ctx->fkev[k]));
-    for (HostGroup* g : piles) { fnbm = std::max(fnbm, g->size); fcm = std::max(fcm, g->maxc); }
-    const int wpb = newt_pile_fused_worlds_per_block(ctx->tune_fused_shape);
-    const int full = newt_pile_fused_blocks_per_sm(ctx->tune_fused_shape, fnbm, fcm) * sm_count(ctx);
-    fgrid = std::min((ft.worlds + wpb - 1) / wpb, std::max(1, full * ctx->tune_fused_pct / 100));
+    for (int cls : {2, 1, 0}) {
+      std::vector<HostGroup*> gs;
+      BatchedLaunch L{};
+      int nbm = 0, stride = 0, cm = 0;
+      for (HostGroup* g : piles)
+        if (newt_pile_batched_class(g->size) == cls) {
+          gs.push_back(g);
+          nbm = std::max(nbm, g->size);
+          cm = std::max(cm, g->maxc);
+          const PileGroupDev d = g->pile_dev();
+          stride = std::max(stride, newt_pile_batched_words(&d));
+        }
+      if (gs.empty()) continue;
+      int rc = build_pile_table(ctx, gs, L.t, bufs, 0, 1);
+      if (rc != NEWT_OK) return rc;
+      CKS(newt_pile_batched_plan(ctx->tune_fused_shape, L.t.worlds, sm_count(ctx), nbm, cm, stride, &L.plan));
+      if (L.t.worlds > 8 * sm_count(ctx)) {  // several waves: the costly worlds first
+        CKS(cudaMalloc(&L.queue, sizeof(int) * (size_t)L.t.worlds));
+        CKS(cudaMalloc(&L.cost, sizeof(unsigned) * (size_t)L.t.worlds));
+        CKS(cudaMemset(L.cost, 0, sizeof(unsigned) * (size_t)L.t.worlds));  // first call: any order
+        bufs.push_back(L.queue);
+        bufs.push_back(L.cost);
+      }
+      bls.push_back(L);
+    }
   }
   for (int b = 0; b < nbr; ++b) {
     int rc = build_pile_table(ctx, piles, pts[b], bufs, b, nbr);
@@ -335,9 +353,8 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
     }
   if (!tcs.empty() && !ctx->tcstream) CKS(cudaStreamCreateWithFlags(&ctx->tcstream, cudaStreamNonBlocking));
 
-  cudaEvent_t fork = nullptr, pfork = nullptr, join[4] = {}, tjoin = nullptr;
+  cudaEvent_t fork = nullptr, join[4] = {}, tjoin = nullptr;
   CKS(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
-  CKS(cudaEventCreateWithFlags(&pfork, cudaEventDisableTiming));
   for (size_t k = 0; k < tls.size(); ++k) {
     if (!ctx->side[k]) CKS(cudaStreamCreateWithFlags(&ctx->side[k], cudaStreamNonBlocking));
     CKS(cudaEventCreateWithFlags(&join[k], cudaEventDisableTiming));
@@ -365,17 +382,26 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
   for (int s = 0; s < n_steps && nt.ng > 0; ++s)
     ctx->launches += newt_launch_pile_solo_step(nt.dG, nt.dseg, nt.ng, nt.worlds, nt.slots, nt.lists,
                                                 s == n_steps - 1, solo_kinds, ctx->stream);
-  int fused_launches = 0;
-  if (fused && ft.ng > 0) {
-    cudaStream_t fs = ctx->pbs[0][0];
-    cudaStreamWaitEvent(fs, fork, 0);
-    cudaMemsetAsync(fcounter, 0, sizeof(int), fs);
-    cudaMemsetAsync(ctx->fused_work, 0, 4 * sizeof(unsigned long long), fs);
-    if (ctx->profile) cudaEventRecordWithFlags(ctx->fkev[0], fs, cudaEventRecordExternal);
-    fused_launches = newt_launch_pile_fused(ft.dG, ft.dseg, ft.ng, fqueue, ft.worlds, fcounter, n_steps, fgrid,
-                                            ctx->fused_work, fcost, fnbm, fcm, ctx->tune_fused_shape, pfork, fs);
-    if (ctx->profile) cudaEventRecordWithFlags(ctx->fkev[1], fs, cudaEventRecordExternal);
-    cudaEventRecord(ctx->pbe[0][4], fs);
+  int batched_launches = 0;
+  if (!bls.empty()) {
+    cudaStream_t f0 = ctx->pbs[0][0];
+    cudaStreamWaitEvent(f0, fork, 0);
+    cudaMemsetAsync(ctx->fused_work, 0, 4 * sizeof(unsigned long long), f0);
+    if (ctx->profile) cudaEventRecordWithFlags(ctx->fkev[0], f0, cudaEventRecordExternal);
+    cudaEventRecord(ctx->pbe[0][3], f0);
+    for (size_t k = 0; k < bls.size(); ++k) {
+      const BatchedLaunch& L = bls[k];
+      cudaStream_t fs = ctx->pbs[k][0];
+      if (k > 0) cudaStreamWaitEvent(fs, ctx->pbe[0][3], 0);
+      batched_launches += newt_launch_pile_batched(L.t.dG, L.t.dseg, L.t.ng, L.queue, L.t.worlds, n_steps,
+                                                   ctx->fused_work, L.cost, &L.plan, fs);
+      if (k > 0) {
+        cudaEventRecord(ctx->pbe[k][4], fs);
+        cudaStreamWaitEvent(f0, ctx->pbe[k][4], 0);
+      }
+    }
+    if (ctx->profile) cudaEventRecordWithFlags(ctx->fkev[1], f0, cudaEventRecordExternal);
+    cudaEventRecord(ctx->pbe[0][4], f0);
     cudaStreamWaitEvent(ctx->stream, ctx->pbe[0][4], 0);
   }
   for (int b = 0; b < nbr; ++b) {
@@ -386,27 +412,22 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
     cudaEventRecord(ctx->pbe[b][4], bs[0]);
     cudaStreamWaitEvent(ctx->stream, ctx->pbe[b][4], 0);
   }
-  // The trees start once the persistent pile launch is under way: its blocks
-  // stay for the whole call, so one that found its SM set to the trees' large
-  // shared memory would keep the small L1 that goes with it (the uneven
-  // workload lost 5%).
   for (size_t k = 0; k < tls.size(); ++k) {
     const TreeLaunch& L = tls[k];
-    cudaStreamWaitEvent(ctx->side[k], fused && ft.ng > 0 ? pfork : fork, 0);
+    cudaStreamWaitEvent(ctx->side[k], fork, 0);
     newt_launch_tree_lanes(L.dg, L.dq, L.items, L.L, L.serial, n_steps, ctx->tune_tree_grid_pct, ctx->side[k]);
     cudaEventRecord(join[k], ctx->side[k]);
   }
-  const int pile_launches = (int)(ctx->launches - before) + fused_launches;
+  const int pile_launches = (int)(ctx->launches - before) + batched_launches;
   ctx->launches = l0;
   ctx->graph_kev_steps = ctx->profile && nbr > 0 && pile_worlds > 0 ? n_steps : 0;
   ctx->graph_kev_branches = std::max(nbr, 1);
-  ctx->graph_fused = fused && ft.ng > 0;
+  ctx->graph_fused = !bls.empty();
   ctx->graph_tc_steps = tc_timed;
   for (size_t k = 0; k < tls.size(); ++k) cudaStreamWaitEvent(ctx->stream, join[k], 0);
   if (!tcs.empty()) cudaStreamWaitEvent(ctx->stream, tjoin, 0);
   cudaError_t ce = cudaStreamEndCapture(ctx->stream, &graph);
   cudaEventDestroy(fork);
-  cudaEventDestroy(pfork);
   for (size_t k = 0; k < tls.size(); ++k) cudaEventDestroy(join[k]);
   cudaEventDestroy(tjoin);
   if (ce != cudaSuccess) { ctx->err = cudaGetErrorString(ce); return NEWT_E_CUDA; }
@@ -475,10 +496,8 @@ int autotune_batched(newt_gpu_ctx* ctx, int n_steps, int horizon, int32_t* choic
       CKS(cudaMemcpyAsync(live[i].first, snap[k][i], live[i].second, cudaMemcpyDeviceToDevice, ctx->stream));
     return NEWT_OK;
   };
-  // piles: the persistent launch in each gang shape (warps per block,
-  // blocks per SM, whether the gang also meets between assembly and sweeps,
-  // one or two worlds per warp), or the
-  // island-class pipeline with 1, 2 or 3 world-range branches; trees: full
+  // piles: the batched launches in each shape (lanes per world in the
+  // sweeps, warps per block in the contact stage), or the island-class pipeline with 1, 2 or 3 world-range branches; trees: full
   // or half persistent grid
   struct Cand { int fused, shape, branches, grid_pct; };
   const Cand cands[] = {{1, 0, 0, 100},  {1, 1, 0, 100}, {1, 2, 0, 100}, {1, 3, 0, 100}, {1, 4, 0, 100},
