@@ -4,7 +4,9 @@
 //
 //   tree_aba_kernel        thread per world (tree_kernels.cu): a_free, the
 //                          ABA with the implicit damping fold, into qacc
-//   tc_k_solve             warp per world (this file): forward kinematics,
+//   tc_k_small, tc_k_solve warp per world (trees of up to 24 DoF with facet
+//                          and normal rows, tc_small.cuh; the others, this
+//                          file): forward kinematics,
 //                          link-plane contacts, link COM Jacobians and the
 //                          mass matrix, its Cholesky factors, the Jacobian
 //                          row of every cone facet, A = J M^-1 J^T, the
@@ -73,7 +75,6 @@ using dense::warp_llt_solve_mixed;
 using dense::warp_matvec;
 using dense::warp_sum;
 using dense::warp_sumd;
-constexpr int TC_WARPS = 1;  // warps (worlds) per block
 constexpr int CREC = TC_CREC;  // floats per contact record
 // contact record fields
 // K_LINK: the link of the row's tree side with sign K_SIGN; K_LINK2: for an
@@ -222,9 +223,9 @@ NEWT_HD TcSmem tc_smem(int L, int nv, int maxc, int rpc) {
   m.vl = m.ldr > up4(nv) ? m.ldr : up4(nv);
   m.nrs = m.ldr < NRS ? m.ldr : NRS;
   int f = 0;
-  m.vec = f; f += N_VEC * m.vl;
   m.rmap = f; f += 2 * m.ldr;
   m.pose = f; f += up4(7 * L);
+  m.vec = f; f += N_VEC * m.vl;
   m.lm = f; f += up4(nv * nv);
   m.ldf = f; f += up4(nv * nv);
   m.tw = f; f += 2 * up4(L);  // translation, then rotation inverse weights per link
@@ -333,101 +334,97 @@ NEWT_D void chain_columns(const TreeGroupDev& g, int w, const float* pose, int l
 
 }  // namespace
 
-// ---------------------------------------------------------------------------
-// K_B: one warp per world
-// ---------------------------------------------------------------------------
-// REFINE: the instance for trees above REFINE_NV DoF (FP64 sum of M and the
-// refinement step); the smaller trees' instance compiles without those paths.
-template <bool REFINE>
-__global__ void __launch_bounds__(32 * TC_WARPS) tc_k_solve(TcGroupDev G) {
-  extern __shared__ __align__(16) float tcs[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int w = blockIdx.x * TC_WARPS + warp;
-  const TreeGroupDev& g = G.t;
-  if (w >= g.n || !g.live[w]) return;  // uniform per warp
-  const int cap = g.cap, L = g.L, nv = g.nv;
-  const TcLay lay = tc_layout(L, nv, G.ng, G.maxc, G.rpc);
-  const TcSmem sm = tc_smem(L, nv, G.maxc, G.rpc);
-  const int ld = lay.ld, vl = sm.vl;
-  float* wf = G.scr + (size_t)w * G.sstride;
-  float* sv = tcs + (size_t)warp * sm.words;
-  float* vx = sv + V_X * vl; float* vd = sv + V_D * vl; float* vg = sv + V_G * vl; float* vb = sv + V_B * vl;
-  float* vreg = sv + V_REG * vl; float* vdiag = sv + V_DIAG * vl; float* vu = sv + V_U * vl;
-  float* vv = sv + V_V * vl; float* vp = sv + V_P * vl; float* vs = sv + V_S * vl;
-  int* rcon = reinterpret_cast<int*>(sv + sm.rmap);
-  int* rfac = rcon + sm.ldr;
-  const float dt = g.dtg[w];
-  const bool rk4 = g.integ && g.integ[w] == NEWT_INTEGRATOR_RK4;
-  uint32_t status = 0;
-  const float* gm = G.geom;
-  auto gv = [&](int gi, int f) { return gm[(size_t)(GREC * gi + f) * cap + w]; };
+namespace {
 
-  // ---- forward kinematics (tree.rs:771-858) ----
-  // Each lane loads one link's joint parameters; the chain is then walked in
-  // link order by every lane (parameters arrive by shuffle), lane 0 storing
-  // the poses.
-  float* pose = sv + sm.pose;
+// ---------------------------------------------------------------------------
+// stages
+// ---------------------------------------------------------------------------
+// Forward kinematics (tree.rs:771-858), a lane per link, the links of one
+// depth at a time: link poses to `pose` and, where `arms` is not null, each
+// link's joint axis and anchor lever (relative to its origin) and its
+// origin's step from its parent's, world frame, nine floats per link.
+// `topo`: parent, joint type and first DoF of each link, packed (tc_topo).
+NEWT_HD int tc_topo(int parent, int jt, int vo) { return (parent + 1) | jt << 8 | vo << 16; }
+NEWT_D int topo_parent(int t) { return (t & 255) - 1; }
+NEWT_D void tc_kinematics(const TreeGroupDev& g, int w, float* pose, int* topo, float* arms, int lane) {
+  const int cap = g.cap, L = g.L;
   for (int base = 0; base < L; base += 32) {
-    const int li = base + lane;
-    float pj[3] = {0.f, 0.f, 0.f}, pc[3] = {0.f, 0.f, 0.f}, pa[3] = {0.f, 0.f, 0.f}, pq = 0.f;
-    if (li < L) {
-      for (int k = 0; k < 3; ++k) {
-        pj[k] = g.jp[(3 * li + k) * cap + w];
-        pc[k] = g.jc[(3 * li + k) * cap + w];
-        pa[k] = g.axis[(3 * li + k) * cap + w];
-      }
-      const int jt = g.topo[4 * li + 1], qo = g.topo[4 * li + 2];
-      if (jt == JH || jt == JS) pq = g.q[qo * cap + w];
-    }
-    const int nl = L - base < 32 ? L - base : 32;
-    for (int k = 0; k < nl; ++k) {
-      const int i = base + k;
-      const V3 jp = v3(__shfl_sync(FULL, pj[0], k), __shfl_sync(FULL, pj[1], k), __shfl_sync(FULL, pj[2], k));
-      const V3 jc = v3(__shfl_sync(FULL, pc[0], k), __shfl_sync(FULL, pc[1], k), __shfl_sync(FULL, pc[2], k));
-      const V3 ax = v3(__shfl_sync(FULL, pa[0], k), __shfl_sync(FULL, pa[1], k), __shfl_sync(FULL, pa[2], k));
-      const float qa = __shfl_sync(FULL, pq, k);
-      const int parent = g.topo[4 * i], jt = g.topo[4 * i + 1], qo = g.topo[4 * i + 2];
-      V3 p;
-      Q4 o;
+    const int i = base + lane;
+    V3 jp = v3(0.f, 0.f, 0.f), jc = jp, ax = jp, p = jp;
+    Q4 o = Q4{0.f, 0.f, 0.f, 1.f};
+    float qa = 0.f;
+    int jt = -1, depth = -1;
+    if (i < L) {
+      const int4 t = *reinterpret_cast<const int4*>(g.topo + 4 * i);
+      jt = t.y;
+      jp = v3(g.jp[(3 * i) * cap + w], g.jp[(3 * i + 1) * cap + w], g.jp[(3 * i + 2) * cap + w]);
+      jc = v3(g.jc[(3 * i) * cap + w], g.jc[(3 * i + 1) * cap + w], g.jc[(3 * i + 2) * cap + w]);
+      ax = v3(g.axis[(3 * i) * cap + w], g.axis[(3 * i + 1) * cap + w], g.axis[(3 * i + 2) * cap + w]);
+      if (jt == JH || jt == JS) qa = g.q[t.z * cap + w];
       if (i == 0) {
         if (jt == JF) {
-          p = v3(g.q[qo * cap + w], g.q[(qo + 1) * cap + w], g.q[(qo + 2) * cap + w]);
-          o = Q4{g.q[(qo + 3) * cap + w], g.q[(qo + 4) * cap + w], g.q[(qo + 5) * cap + w], g.q[(qo + 6) * cap + w]};
+          p = v3(g.q[t.z * cap + w], g.q[(t.z + 1) * cap + w], g.q[(t.z + 2) * cap + w]);
+          o = Q4{g.q[(t.z + 3) * cap + w], g.q[(t.z + 4) * cap + w], g.q[(t.z + 5) * cap + w], g.q[(t.z + 6) * cap + w]};
         } else {
           o = Q4{g.rootq[w], g.rootq[cap + w], g.rootq[2 * cap + w], g.rootq[3 * cap + w]};
           p = jp - qrot(o, jc);
         }
-      } else {
-        __syncwarp();
+        stv3(pose, p);
+        pose[3] = o.x; pose[4] = o.y; pose[5] = o.z; pose[6] = o.w;
+      }
+      topo[i] = tc_topo(t.x, jt, t.w);
+    }
+    __syncwarp();
+    for (int k = i; k >= 0 && k < L; k = topo_parent(topo[k])) ++depth;
+    const int deepest = __reduce_max_sync(FULL, depth);
+    const Q4 qj = q_axis_angle(ax, qa);
+    const int parent = i < L ? topo_parent(topo[i]) : 0;
+    for (int d = 1; d <= deepest; ++d) {
+      if (depth == d) {
         const float* pp = pose + 7 * parent;
         const Q4 po = Q4{pp[3], pp[4], pp[5], pp[6]};
-        const V3 jpw = ldv3(pp) + qrot(po, jp);
-        if (jt == JH) {
-          o = qmul(po, q_axis_angle(ax, qa));
-          p = jpw - qrot(o, jc);
-        } else if (jt == JS) {
-          o = po;
-          p = jpw + qrot(po, ax * qa) - qrot(o, jc);
+        const V3 a = qrot(po, jp);
+        const V3 jpw = ldv3(pp) + a;
+        o = jt == JH ? qmul(po, qj) : po;
+        const V3 cw = qrot(o, jc);
+        V3 step = a - cw;
+        if (jt == JS) {
+          const V3 sl = qrot(po, ax * qa);
+          p = jpw + sl - cw;
+          step = step + sl;
         } else {
-          o = po;
-          p = jpw - qrot(o, jc);
+          p = jpw - cw;
+        }
+        float* q = pose + 7 * i;
+        stv3(q, p);
+        q[3] = o.x; q[4] = o.y; q[5] = o.z; q[6] = o.w;
+        if (arms) {
+          stv3(arms + 9 * i, qrot(po, ax));
+          stv3(arms + 9 * i + 3, cw);
+          stv3(arms + 9 * i + 6, step);
         }
       }
       __syncwarp();
-      if (lane == 0) {
-        float* d = pose + 7 * i;
-        stv3(d, p);
-        d[3] = o.x; d[4] = o.y; d[5] = o.z; d[6] = o.w;
-      }
     }
   }
-  __syncwarp();
+}
 
+// Contacts and their rows: the link-plane pairs' contacts (and in-tree
+// pairs') to the world's scratch, the rows' contact and kind to rcon and
+// rfac.  Returns the rows; the re-solve of the contact sensors takes the
+// last step's contacts.
+NEWT_D int tc_contacts(const TcGroupDev& G, int w, const float* pose, int* rcon, int* rfac, bool resolve, int lane,
+                       int* ncon_out, uint32_t* status) {
+  const TreeGroupDev& g = G.t;
+  const int cap = g.cap;
+  const TcLay lay = tc_layout(g.L, g.nv, G.ng, G.maxc, G.rpc);
+  float* wf = G.scr + (size_t)w * G.sstride;
+  const float* gm = G.geom;
+  auto gv = [&](int gi, int f) { return gm[(size_t)(GREC * gi + f) * cap + w]; };
   // ---- contacts in newt's pair order (link-plane pairs, and in-tree pairs
   //      when the tree collides with itself): lane per pair, a warp scan
   //      places each pair's contacts ----
   float* con = wf + lay.con;
-  const bool resolve = G.sens != nullptr;  // the contact sensors' re-solve: the last step's contacts, no detection
   int ncon = resolve ? min(max(__float_as_int(wf[lay.misc]), 0), G.maxc) : 0;
   bool overflow = false;
   auto link_geom_pose = [&](int gi) {
@@ -520,7 +517,7 @@ __global__ void __launch_bounds__(32 * TC_WARPS) tc_k_solve(TcGroupDev G) {
     }
     ncon = ncon + total < G.maxc ? ncon + total : G.maxc;
   }
-  if (__any_sync(FULL, overflow)) status |= NEWT_WS_CONTACT_OVERFLOW;
+  if (__any_sync(FULL, overflow)) *status |= NEWT_WS_CONTACT_OVERFLOW;
   __syncwarp();
   // rows of the active contacts, in contact order (solver.rs:2881-2890):
   // lane per contact, a warp scan assigns the row ranges; the pyramidal
@@ -554,7 +551,33 @@ __global__ void __launch_bounds__(32 * TC_WARPS) tc_k_solve(TcGroupDev G) {
     wf[lay.misc + 1] = __int_as_float(nrows);
     wf[lay.misc + 2] = __int_as_float(0);
   }
-  const int nr = nrows;
+  *ncon_out = ncon;
+  return nrows;
+}
+
+// The solve of a world's rows, every size: link Jacobians, M and its
+// factors, the rows, Newton or PGS, and the accelerations.
+// REFINE: the instance for trees above REFINE_NV DoF (FP64 sum of M and the
+// refinement step); the smaller trees' instance compiles without those paths.
+template <bool REFINE>
+NEWT_D void tc_rows_solve(const TcGroupDev& G, int w, float* sv, int nr, int ncon, uint32_t status, int lane) {
+  const TreeGroupDev& g = G.t;
+  const int cap = g.cap, L = g.L, nv = g.nv;
+  const TcLay lay = tc_layout(L, nv, G.ng, G.maxc, G.rpc);
+  const TcSmem sm = tc_smem(L, nv, G.maxc, G.rpc);
+  const int ld = lay.ld, vl = sm.vl;
+  float* wf = G.scr + (size_t)w * G.sstride;
+  float* vec = sv + sm.vec;
+  float* vx = vec + V_X * vl; float* vd = vec + V_D * vl; float* vg = vec + V_G * vl; float* vb = vec + V_B * vl;
+  float* vreg = vec + V_REG * vl; float* vdiag = vec + V_DIAG * vl; float* vu = vec + V_U * vl;
+  float* vv = vec + V_V * vl; float* vp = vec + V_P * vl; float* vs = vec + V_S * vl;
+  float* pose = sv + sm.pose;
+  int* rcon = reinterpret_cast<int*>(sv + sm.rmap);
+  int* rfac = rcon + sm.ldr;
+  float* con = wf + lay.con;
+  const float dt = g.dtg[w];
+  const bool rk4 = g.integ && g.integ[w] == NEWT_INTEGRATOR_RK4;
+  const bool resolve = G.sens != nullptr;  // the contact sensors' re-solve: the last step's contacts, no detection
   // the re-solve's sensor inputs (solver.rs:3334-3364): per link the rows'
   // forces f / dt times their wrench axes (dir x sign, (p - c_link) x
   // dir x sign), in row order; per contact the facets' impulses summed (a
@@ -996,6 +1019,28 @@ __global__ void __launch_bounds__(32 * TC_WARPS) tc_k_solve(TcGroupDev G) {
   }
 }
 
+}  // namespace
+
+// ---------------------------------------------------------------------------
+// One warp per world, every size and cone
+// ---------------------------------------------------------------------------
+template <bool REFINE>
+__global__ void __launch_bounds__(32) tc_k_solve(TcGroupDev G) {
+  extern __shared__ __align__(16) float tcs[];
+  const int lane = threadIdx.x, w = blockIdx.x;
+  if (w >= G.t.n || !G.t.live[w]) return;  // uniform
+  const TcSmem sm = tc_smem(G.t.L, G.t.nv, G.maxc, G.rpc);
+  float* pose = tcs + sm.pose;
+  int* rcon = reinterpret_cast<int*>(tcs + sm.rmap);
+  uint32_t status = 0;
+  int ncon = 0;
+  tc_kinematics(G.t, w, pose, reinterpret_cast<int*>(tcs + sm.vec), nullptr, lane);
+  const int nr = tc_contacts(G, w, pose, rcon, rcon + sm.ldr, G.sens != nullptr, lane, &ncon, &status);
+  tc_rows_solve<REFINE>(G, w, tcs, nr, ncon, status, lane);
+}
+
+#include "tc_small.cuh"
+
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
@@ -1003,28 +1048,50 @@ extern "C" size_t newt_tc_ws_bytes(int L, int nv, int ng, int maxc, int rpc) {
   return (size_t)tc_layout(L, nv, ng, maxc, rpc).words * sizeof(float);
 }
 extern "C" size_t newt_tc_smem_bytes(int L, int nv, int maxc, int rpc) {
-  return (size_t)TC_WARPS * tc_smem(L, nv, maxc, rpc).words * sizeof(float);
+  return (size_t)tc_smem(L, nv, maxc, rpc).words * sizeof(float);
+}
+// The launch of a group: tc_k_small for trees of up to REFINE_NV DoF whose
+// rows are facets or normals, else tc_k_solve.  Blocks of tc_k_small hold
+// TCS_WARPS worlds, fewer where their shared memory would not let two blocks
+// share an SM.
+struct TcPlan { bool small; int warps; size_t bytes; };
+static TcPlan tc_plan(int L, int nv, int maxc, int rpc, bool general, bool resolve) {
+  TcPlan p{nv <= REFINE_NV && !general && !resolve, 1, newt_tc_smem_bytes(L, nv, maxc, rpc)};
+  if (p.small) {
+    const size_t per = (size_t)tcs_smem(L, nv, maxc, rpc).words * sizeof(float);
+    p.warps = TCS_WARPS;
+    while (p.warps > 1 && p.warps * per > (227 * 1024 - 2048) / 2) p.warps /= 2;
+    p.bytes = p.warps * per;
+  }
+  return p;
 }
 // Kernel attribute for the dynamic shared memory (outside stream capture).
 // The limit only grows: every tree-contact group of a step is prepared before
 // any of them launches, so a later, smaller group must not lower the limit an
 // earlier, larger one launches with.
-extern "C" cudaError_t newt_tc_init(int L, int nv, int maxc, int rpc) {
-  const int bytes = (int)newt_tc_smem_bytes(L, nv, maxc, rpc);
-  const bool refine = nv > REFINE_NV;
+static cudaError_t tc_limit(const void* kernel, size_t bytes) {
   cudaFuncAttributes fa;
-  cudaError_t e = refine ? cudaFuncGetAttributes(&fa, tc_k_solve<true>) : cudaFuncGetAttributes(&fa, tc_k_solve<false>);
-  if (e != cudaSuccess) return e;
-  if (bytes <= fa.maxDynamicSharedSizeBytes) return cudaSuccess;
-  return refine ? cudaFuncSetAttribute(tc_k_solve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)
-                : cudaFuncSetAttribute(tc_k_solve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+  if (e != cudaSuccess || (int)bytes <= fa.maxDynamicSharedSizeBytes) return e;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+static cudaError_t newt_tc_init(int L, int nv, int maxc, int rpc, bool general) {
+  const TcPlan p = tc_plan(L, nv, maxc, rpc, general, false);
+  if (p.small) {
+    const cudaError_t e = tc_limit((const void*)tc_k_small, p.bytes);
+    if (e != cudaSuccess) return e;
+  }
+  // the contact sensors' re-solve of any group runs tc_k_solve
+  return tc_limit(nv > REFINE_NV ? (const void*)tc_k_solve<true> : (const void*)tc_k_solve<false>,
+                  newt_tc_smem_bytes(L, nv, maxc, rpc));
 }
 extern "C" void newt_launch_tc_solve(const TcGroupDev& G, cudaStream_t st) {
-  const int grid = (G.t.n + TC_WARPS - 1) / TC_WARPS;
-  if (grid == 0) return;
-  const size_t bytes = newt_tc_smem_bytes(G.t.L, G.t.nv, G.maxc, G.rpc);
-  if (G.t.nv > REFINE_NV) tc_k_solve<true><<<grid, 32 * TC_WARPS, bytes, st>>>(G);
-  else tc_k_solve<false><<<grid, 32 * TC_WARPS, bytes, st>>>(G);
+  const int n = G.t.n;
+  if (n == 0) return;
+  const TcPlan p = tc_plan(G.t.L, G.t.nv, G.maxc, G.rpc, G.general != 0, G.sens != nullptr);
+  if (p.small) tc_k_small<<<(n + p.warps - 1) / p.warps, 32 * p.warps, p.bytes, st>>>(G);
+  else if (G.t.nv > REFINE_NV) tc_k_solve<true><<<n, 32, p.bytes, st>>>(G);
+  else tc_k_solve<false><<<n, 32, p.bytes, st>>>(G);
 }
 extern "C" void newt_tc_offsets(int L, int nv, int ng, int maxc, int rpc, int* con, int* imp, int* misc) {
   const TcLay t = tc_layout(L, nv, ng, maxc, rpc);
@@ -1059,7 +1126,7 @@ extern "C" int newt_tc_prepare(newt_gpu_ctx* ctx, HostGroup* g, int n_steps) {
     ctx->graph_dirty = true;
   }
   g->scr_stride = (long)(per / sizeof(float));
-  CKT(newt_tc_init(g->size, g->nv, g->maxc, g->tc_rpc));
+  CKT(newt_tc_init(g->size, g->nv, g->maxc, g->tc_rpc, g->tc_general));
   if (ctx->profile) {
     while (ctx->tcev.size() < (size_t)6 * n_steps) {
       cudaEvent_t e;
