@@ -291,8 +291,9 @@ extern "C" void pile_k_collide_launch(const PileGroupDev* dG, const int* dwseg, 
                                       int total_slots, int* lists, cudaStream_t st);
 extern "C" void pile_k_integrate_launch(const PileGroupDev* dG, const int* dwseg, int ng, int total_worlds,
                                         int write_diag, cudaStream_t st);
-extern "C" void newt_launch_pile_newton_solve(const PileGroupDev* dG, const int* dwseg, int ng, int total_worlds,
-                                              cudaStream_t st);
+extern "C" int newt_launch_pile_newton_solve(const PileGroupDev* dG, const int* dwseg, int ng, int total_worlds,
+                                             int* lists, int slots, int* counters, cudaStream_t st);
+extern "C" int* newt_pile_newton_counters(int* lists, int slots);
 
 // The general-row solve alone (the contact sensors' re-solve).
 extern "C" void newt_launch_pile_general_solve(const PileGroupDev* dG, const int* dwseg, int ng, int total_worlds,
@@ -310,7 +311,9 @@ extern "C" int newt_launch_pile_solo_step(const PileGroupDev* dG, const int* dws
   if (total_worlds <= 0) return 0;
   int n = 2;
   pile_k_collide_launch(dG, dwseg, ng, total_worlds, total_slots, lists, st);
-  if (kinds & (1 << PS_NEWTON)) { newt_launch_pile_newton_solve(dG, dwseg, ng, total_worlds, st); ++n; }
+  if (kinds & (1 << PS_NEWTON))
+    n += newt_launch_pile_newton_solve(dG, dwseg, ng, total_worlds, lists, total_slots,
+                                       newt_pile_newton_counters(lists, total_slots), st);
   if (kinds & (1 << PS_GENERAL)) { newt_launch_pile_general_solve(dG, dwseg, ng, total_worlds, st); ++n; }
   pile_k_integrate_launch(dG, dwseg, ng, total_worlds, write_diag, st);
   return n;

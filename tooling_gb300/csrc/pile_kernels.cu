@@ -960,7 +960,7 @@ static void launch_class(int cl, const PileGroupDev* dG, const int* dwseg, int n
   }
 }
 
-static_assert(N_COUNTERS <= 32, "counters live in the last 32 ints of the lists");
+static_assert(N_COUNTERS + 3 <= 32, "counters live in the last 32 ints of the lists");
 static_assert(N_ICLASS + 2 == NEWT_PILE_KERNELS && N_ICLASS == NEWT_PILE_ISLAND_CLASSES,
               "kernel table of the profiling surface");
 
@@ -985,7 +985,7 @@ extern "C" int newt_launch_pile_step(const PileGroupDev* dG, const int* dwseg, i
   auto mark = [&](int k, int end, cudaStream_t s) {
     if (kev) cudaEventRecordWithFlags(kev[2 * k + end], s, cudaEventRecordExternal);
   };
-  cudaMemsetAsync(il.counts, 0, N_COUNTERS * sizeof(int), st);
+  cudaMemsetAsync(il.counts, 0, (N_COUNTERS + 3) * sizeof(int), st);
   const int wpb = 4;
   mark(0, 0, st);
   pile_k_collide<<<(total_worlds + wpb - 1) / wpb, 32 * wpb, 0, st>>>(dG, dwseg, ng, total_worlds, il);
@@ -1013,10 +1013,13 @@ extern "C" int newt_launch_pile_step(const PileGroupDev* dG, const int* dwseg, i
   return N_ICLASS + 2;
 }
 
-extern "C" void newt_launch_pile_newton_solve(const PileGroupDev* dG, const int* dwseg, int ng, int total_worlds,
-                                              cudaStream_t st);
+extern "C" int newt_launch_pile_newton_solve(const PileGroupDev* dG, const int* dwseg, int ng, int total_worlds,
+                                             int* lists, int slots, int* counters, cudaStream_t st);
 extern "C" void newt_launch_pile_general_solve(const PileGroupDev* dG, const int* dwseg, int ng, int total_worlds,
                                                cudaStream_t st);
+
+// The Newton solve's counters in the lists (zeroed with the island counters).
+extern "C" int* newt_pile_newton_counters(int* lists, int slots) { return lists + (size_t)N_ICLASS * slots + N_COUNTERS; }
 
 // The contact re-solve of every world of a table at its current state
 // (pile_k_reassemble, then the island-class PGS solvers, the dense Newton
@@ -1031,12 +1034,12 @@ extern "C" int newt_launch_pile_resolve(const PileGroupDev* dG, const int* dwseg
   il.cap = total_slots;
   il.stats = 0;
   il.counts = lists + (size_t)N_ICLASS * total_slots;
-  cudaMemsetAsync(il.counts, 0, N_COUNTERS * sizeof(int), st);
+  cudaMemsetAsync(il.counts, 0, (N_COUNTERS + 3) * sizeof(int), st);
   const int wpb = 4;
   pile_k_reassemble<<<(total_worlds + wpb - 1) / wpb, 32 * wpb, 0, st>>>(dG, dwseg, ng, total_worlds, il);
   if (solve == PS_NEWTON) {
-    newt_launch_pile_newton_solve(dG, dwseg, ng, total_worlds, st);
-    return 2;
+    return 1 + newt_launch_pile_newton_solve(dG, dwseg, ng, total_worlds, lists, total_slots,
+                                             newt_pile_newton_counters(lists, total_slots), st);
   }
   if (solve == PS_GENERAL) {
     newt_launch_pile_general_solve(dG, dwseg, ng, total_worlds, st);
@@ -1126,7 +1129,7 @@ extern "C" void pile_k_collide_launch(const PileGroupDev* dG, const int* dwseg, 
   il.cap = total_slots;
   il.stats = 0;
   il.counts = lists + (size_t)N_ICLASS * total_slots;
-  cudaMemsetAsync(il.counts, 0, N_COUNTERS * sizeof(int), st);
+  cudaMemsetAsync(il.counts, 0, (N_COUNTERS + 3) * sizeof(int), st);
   const int wpb = 4;
   pile_k_collide<<<(total_worlds + wpb - 1) / wpb, 32 * wpb, 0, st>>>(dG, dwseg, ng, total_worlds, il);
 }
@@ -1167,7 +1170,7 @@ extern "C" int newt_launch_pile_step_serial(const PileGroupDev* dG, const int* d
   il.cap = total_slots;
   il.stats = write_diag;
   il.counts = lists + (size_t)N_ICLASS * total_slots;
-  cudaMemsetAsync(il.counts, 0, N_COUNTERS * sizeof(int), st);
+  cudaMemsetAsync(il.counts, 0, (N_COUNTERS + 3) * sizeof(int), st);
   const int wpb = 4;
   pile_k_collide<<<(total_worlds + wpb - 1) / wpb, 32 * wpb, 0, st>>>(dG, dwseg, ng, total_worlds, il);
   const int grid = std::min((total_slots + 127) / 128, cap128);

@@ -40,6 +40,7 @@ extern "C" int newt_launch_pile_batched(const PileGroupDev* dG, const int* dwseg
                                         const PileBatchedPlan* p, cudaStream_t st);
 extern "C" int newt_tc_prepare(newt_gpu_ctx* ctx, HostGroup* g, int n_steps);
 extern "C" size_t newt_pile_newton_bytes(int maxc);
+extern "C" cudaError_t newt_pile_newton_prepare();
 extern "C" int newt_launch_pile_solo_step(const PileGroupDev* dG, const int* dwseg, int ng, int total_worlds,
                                           int total_slots, int* lists, int write_diag, int kinds, cudaStream_t st);
 extern "C" int newt_tc_launch(newt_gpu_ctx* ctx, HostGroup* g, int n_steps, cudaStream_t st, bool capturing);
@@ -66,7 +67,10 @@ static int ensure_pile_scratch(newt_gpu_ctx* ctx, HostGroup* g) {
   int rs = ensure_pile_streams(ctx);
   if (rs != NEWT_OK) return rs;
   size_t per = newt_pile_ws_bytes(g->size, g->np, g->maxc);
-  if (g->pile_newton) per += newt_pile_newton_bytes(g->maxc);  // H, its factors, the solver vectors
+  if (g->pile_newton) {
+    per += newt_pile_newton_bytes(g->maxc);  // H, its factors, the solver vectors
+    CKS(newt_pile_newton_prepare());
+  }
   size_t need = per * (size_t)g->cap;
   if (g->plain_scratch_bytes < need) {
     if (g->plain_scratch) cudaFree(g->plain_scratch);

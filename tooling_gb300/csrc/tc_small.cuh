@@ -168,36 +168,6 @@ NEWT_D bool chol_one(float* m, int n, int ld, int lane, float* mn, float* mx) {
   return ok;
 }
 
-// Sums of N (a power of two) doubles over the warp: the lanes halve the values
-// they carry at each exchange, so N sums take 2 N - 2 + 5 - log2 N additions
-// at most instead of 5 N (an FP64 instruction occupies its pipe for sixteen
-// cycles).
-template <int N>
-NEWT_D void warp_sums(double (&v)[N], int lane) {
-  int width = N, bit = 16;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    if (width > 1) {
-      const int half = width / 2;
-      const bool up = lane & o;
-#pragma unroll
-      for (int k = 0; k < N / 2; ++k)
-        if (k < half) {
-          const double send = up ? v[k] : v[k + half], keep = up ? v[k + half] : v[k];
-          v[k] = keep + __shfl_xor_sync(FULL, send, o);
-        }
-      width = half;
-      bit = o;
-    } else {
-      v[0] += __shfl_xor_sync(FULL, v[0], o);
-    }
-  }
-  // value k's sum lies where the lane's top bits spell k
-  const double mine = v[0];
-#pragma unroll
-  for (int k = 0; k < N; ++k) v[k] = __shfl_sync(FULL, mine, k * bit);
-}
-
 // a / b by Newton steps on the reciprocal from its FP32 value (an FP64 divide
 // keeps the FP64 pipe busy several times as long).
 NEWT_D double quot_d(double a, double b) {
@@ -297,13 +267,13 @@ NEWT_D int small_newton(float* H, int nr, float b, float* xs, int iters, int lan
     double Pu = 0.0, Pv = 0.0, Sv, bP = 0.0, bS;
     if (it == 0) {  // x = 0: p = 0
       double t[2] = {(double)s * (double)v, (double)b * (double)s};
-      warp_sums(t, lane);
+      dense::warp_sums(t, lane);
       Sv = t[0];
       bS = t[1];
     } else {
       double t[8] = {(double)p * (double)u, (double)p * (double)v, (double)s * (double)v, (double)b * (double)p,
                      (double)b * (double)s, (double)x * (double)hx, (double)x * (double)b, 0.0};
-      warp_sums(t, lane);
+      dense::warp_sums(t, lane);
       Pu = t[0]; Pv = t[1]; Sv = t[2]; bP = t[3]; bS = t[4];
       cur = 0.5 * t[5] + t[6];
     }
