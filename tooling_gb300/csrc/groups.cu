@@ -427,11 +427,6 @@ int HostGroup::flush_model(newt_gpu_ctx* ctx) {
 // ---------------------------------------------------------------------------
 // state staging (MuJoCo layout in, newt layout on the device)
 // ---------------------------------------------------------------------------
-void HostGroup::stage_qfrc(int w, const HostModel& m, const float* qfrc) {
-  if (soa()) for (int k = 0; k < nv; ++k) F(r_qfrc + k, w) = qfrc[k];
-  (void)m;
-}
-
 void HostGroup::read_qacc(int w, const HostModel& m, float* qacc) const {
   if (soa()) for (int k = 0; k < nv; ++k) qacc[k] = Fc(r_qacc + k, w);
   else for (int k = 0; k < m.nv; ++k) qacc[k] = 0.f;

@@ -442,62 +442,36 @@ static int group_worlds(newt_gpu_ctx* ctx, const int32_t* slots, int32_t n, std:
   return NEWT_OK;
 }
 
-enum RowSet { ROWS_QFRC, ROWS_QACC };
-
-static std::vector<RowMove> moves_for(newt_gpu_ctx* ctx, std::vector<std::vector<int>>& by_group, RowSet set) {
+static std::vector<RowMove> qacc_moves(newt_gpu_ctx* ctx, std::vector<std::vector<int>>& by_group) {
   std::vector<RowMove> mv;
   for (size_t gi = 0; gi < by_group.size(); ++gi) {
     if (by_group[gi].empty()) continue;
     HostGroup* g = ctx->groups[gi].get();
-    size_t lo = 0, cnt = 0;
-    if (!g->soa()) continue;  // free-body piles carry no generalised force or acceleration rows
-    lo = set == ROWS_QFRC ? g->r_qfrc : g->r_qacc;
-    cnt = g->nv;
-    mv.push_back(RowMove{g, std::move(by_group[gi]), lo, cnt});
+    if (!g->soa()) continue;  // free-body piles carry no acceleration rows
+    mv.push_back(RowMove{g, std::move(by_group[gi]), (size_t)g->r_qacc, (size_t)g->nv});
   }
   return mv;
 }
 
-// State goes in and out in MuJoCo layout, one copy each way, converted on the
-// device (world_io.cu); only the named worlds' rows change.  The host
-// mirror's state rows are not kept: every reader gathers from the device.
+// State and forces go in and out in MuJoCo layout, converted on the device
+// (world_io.cu); only the named worlds' rows change.  The host mirror's rows
+// of them are not kept: every reader gathers from the device.
 int newt_gpu_set_state(newt_gpu_ctx* ctx, const int32_t* slots, int32_t n, const float* qpos, const float* qvel) {
   if (!ctx || (n > 0 && (!slots || !qpos || !qvel))) return NEWT_E_INVALID;
   cudaSetDevice(ctx->device);
-  std::vector<std::vector<int>> by_group;
-  int rc = group_worlds(ctx, slots, n, by_group);
-  if (rc != NEWT_OK) return rc;
-  std::vector<char> seen(ctx->slots.size(), 0);
-  for (int i = 0; i < n; ++i) {
-    if (seen[slots[i]]) return fail(ctx, NEWT_E_INVALID, "slot named twice");
-    seen[slots[i]] = 1;
-  }
   return io_state_in(ctx, slots, n, qpos, qvel);
 }
 
 int newt_gpu_get_state(newt_gpu_ctx* ctx, const int32_t* slots, int32_t n, float* qpos, float* qvel) {
   if (!ctx || (n > 0 && (!slots || !qpos || !qvel))) return NEWT_E_INVALID;
   cudaSetDevice(ctx->device);
-  std::vector<std::vector<int>> by_group;
-  int rc = group_worlds(ctx, slots, n, by_group);
-  if (rc != NEWT_OK) return rc;
   return io_state_out(ctx, slots, n, qpos, qvel);
 }
 
 int newt_gpu_set_qfrc(newt_gpu_ctx* ctx, const int32_t* slots, int32_t n, const float* qfrc) {
   if (!ctx || (n > 0 && (!slots || !qfrc))) return NEWT_E_INVALID;
   cudaSetDevice(ctx->device);
-  std::vector<std::vector<int>> by_group;
-  int rc = group_worlds(ctx, slots, n, by_group);
-  if (rc != NEWT_OK) return rc;
-  long vo = 0;
-  for (int i = 0; i < n; ++i) {
-    const SlotRef& r = ctx->slots[slots[i]];
-    const HostModel& m = ctx->models[r.model];
-    ctx->groups[r.group]->stage_qfrc(r.index, m, qfrc + vo);
-    vo += m.nv;
-  }
-  return io_scatter(ctx, moves_for(ctx, by_group, ROWS_QFRC));
+  return io_qfrc_in(ctx, slots, n, qfrc);
 }
 
 int newt_gpu_step(newt_gpu_ctx* ctx, int32_t n_steps, int32_t mode) {
@@ -544,7 +518,7 @@ int newt_gpu_get_qacc(newt_gpu_ctx* ctx, const int32_t* slots, int32_t n, float*
   std::vector<std::vector<int>> by_group;
   int rc = group_worlds(ctx, slots, n, by_group);
   if (rc != NEWT_OK) return rc;
-  rc = io_gather(ctx, moves_for(ctx, by_group, ROWS_QACC));
+  rc = io_gather(ctx, qacc_moves(ctx, by_group));
   if (rc != NEWT_OK) return rc;
   long vo = 0;
   for (int i = 0; i < n; ++i) {

@@ -120,9 +120,8 @@ struct HostGroup {
   int* live_flag(int idx);      // the world's device live flag
   void write_model(newt_gpu_ctx* ctx, int idx, const HostModel& m);
   int flush_model(newt_gpu_ctx* ctx);
-  // generalised force / acceleration rows of one world in the host mirror,
-  // moved per world by io_scatter / io_gather (state: io_state_in/out)
-  void stage_qfrc(int idx, const HostModel& m, const float* qfrc);
+  // acceleration rows of one world in the host mirror, moved per world by
+  // io_gather (state and forces: io_state_in/out, io_qfrc_in)
   void read_qacc(int idx, const HostModel& m, float* qacc) const;
   int fetch_status(newt_gpu_ctx* ctx);
   int clear_status(newt_gpu_ctx* ctx);
@@ -239,6 +238,7 @@ int io_clear_flags(newt_gpu_ctx* ctx, const std::vector<int*>& flags);  // *flag
 // (world_io.cu)
 int io_state_in(newt_gpu_ctx* ctx, const int32_t* slots, int n, const float* qpos, const float* qvel);
 int io_state_out(newt_gpu_ctx* ctx, const int32_t* slots, int n, float* qpos, float* qvel);
+int io_qfrc_in(newt_gpu_ctx* ctx, const int32_t* slots, int n, const float* qfrc);
 int io_hold_flags(newt_gpu_ctx* ctx, const std::vector<int*>& flags);   // the same, queued without a wait
 void ctrl_release_slot(newt_gpu_ctx* ctx, int slot);                     // ends the slot's control stream
 

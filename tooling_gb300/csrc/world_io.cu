@@ -222,28 +222,50 @@ int io_gather(newt_gpu_ctx* ctx, const std::vector<RowMove>& all) {
 }
 
 // ---------------------------------------------------------------------------
-// state in MuJoCo layout, converted on the device
+// state and forces in MuJoCo layout, converted on the device
 // ---------------------------------------------------------------------------
-// newt_gpu_set_state / newt_gpu_get_state move the caller's MuJoCo-layout
-// arrays in one copy each way and convert them here, a warp per world:
-// quaternions reordered (wxyz <-> xyzw) and, on the way in, normalised; a
-// free root's linear velocity rotated between world and body frame (newt's
+// newt_gpu_set_state / get_state / set_qfrc convert between the caller's
+// MuJoCo-layout arrays and the groups' rows in one launch: quaternions
+// reordered (wxyz <-> xyzw) and, on the way in, normalised; a free root's
+// linear velocity rotated between world and body frame (newt's
 // apply_mujoco_qpos/qvel, world.rs:519-623, and its inverse).  A free root's
 // and a hinge's MuJoCo offsets equal newt's (7 and 1 coordinates, 6 and 1
 // rates), so a link's `topo` offsets index both layouts.
+//
+// What bounds a call: latency for few worlds (a copy for the plan, one per
+// array, the launch, the wait), the host's loops over the slots and the link
+// for many.  So
+//   * the worlds are taken as runs of consecutive indices in a group, a few
+//     of which describe most calls and travel as kernel parameters (up to
+//     128; a table in the staging past that);
+//   * page-locked arrays are read and written by the kernel itself, others
+//     through the page-locked staging;
+//   * a block moves up to 32 worlds of a run by way of shared memory, so that
+//     both the caller's array (worlds one after another) and a tree group's
+//     rows (worlds side by side) are touched in whole lines.
+// Measured (GB300, us for set_state and get_state from page-locked arrays; one
+// plan entry per world and a copy per array before -> now): 16384 quadrupeds
+// 212 and 206 -> 81 and 81 (set_qfrc from an ordinary array, which went by way
+// of a host transpose, 423 -> 127), 8192 piles of 16 153 and 153 -> 81 and 81,
+// 6000 mixed worlds 128 and 130 -> 63 and 61, one pendulum 24 and 22 -> 19 and
+// 18.
 namespace {
 
-struct StateGroup {
+struct StateRun {
   float* F;
-  int soa, cap, size;  // tree SoA (row * cap + w) or pile world-major (w * frows + row); bodies or links
-  long frows;
-  int pos, quat, vel, omg;  // pile rows
-  int rq, rqd;              // tree rows
-  const int* topo;          // tree: parent, joint, q offset, v offset per link
+  const int* topo;                // tree: parent, joint, q offset, v offset per link
+  long frows, q0, v0;             // the run's first coordinate and rate in the caller's arrays
+  int soa, cap, size, nq, nv;     // tree SoA (row * cap + w) or pile world-major (w * frows + row); bodies or links
+  int pos, quat, vel, omg;        // pile rows
+  int rq, rqd, rf;                // tree rows: coordinates, rates, applied forces
+  int w0, n, tile, blk;           // first index, worlds, worlds per block, first block
 };
-struct StateWorld { int g, w, qoff, voff; };
+template <int N>
+struct StateRuns { int n; StateRun r[N]; };
+enum StateMove { STATE_IN, STATE_OUT, QFRC_IN };
+constexpr int TILE_FLOATS = 10240;  // a block's share of the arrays (40 KB of shared memory)
 
-NEWT_D float& frow(const StateGroup& g, int row, int w) {
+NEWT_D float& frow(const StateRun& g, int row, int w) {
   return g.soa ? g.F[(size_t)row * g.cap + w] : g.F[(size_t)w * g.frows + row];
 }
 NEWT_D Q4 qnorm_or_identity(Q4 q) {  // the host's q_norm: a zero quaternion becomes the identity
@@ -251,181 +273,307 @@ NEWT_D Q4 qnorm_or_identity(Q4 q) {  // the host's q_norm: a zero quaternion bec
   return n == 0.f ? Q4{0.f, 0.f, 0.f, 1.f} : Q4{q.x / n, q.y / n, q.z / n, q.w / n};
 }
 
-__global__ void state_in(const StateGroup* __restrict__ G, const StateWorld* __restrict__ W, int n,
-                         const float* __restrict__ qpos, const float* __restrict__ qvel) {
-  const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (t >= n) return;
-  const StateWorld sw = W[t];
-  const StateGroup g = G[sw.g];
-  const float* qp = qpos + sw.qoff;
-  const float* qv = qvel + sw.voff;
-  for (int i = lane; i < g.size; i += 32) {
-    if (!g.soa) {  // free body i
-      const float* p = qp + 7 * i;
-      const float* v = qv + 6 * i;
-      const Q4 q = qnorm_or_identity(Q4{p[4], p[5], p[6], p[3]});
-      for (int k = 0; k < 3; ++k) {
-        frow(g, g.pos + 3 * i + k, sw.w) = p[k];
-        frow(g, g.vel + 3 * i + k, sw.w) = v[k];
-        frow(g, g.omg + 3 * i + k, sw.w) = v[3 + k];
-      }
-      frow(g, g.quat + 4 * i, sw.w) = q.x; frow(g, g.quat + 4 * i + 1, sw.w) = q.y;
-      frow(g, g.quat + 4 * i + 2, sw.w) = q.z; frow(g, g.quat + 4 * i + 3, sw.w) = q.w;
-      continue;
+// Body or link i of world w: its coordinates at qp and rates at qv to the rows.
+NEWT_D void state_in(const StateRun& g, int i, int w, const float* qp, const float* qv) {
+  if (!g.soa) {  // free body i
+    const float* p = qp + 7 * i;
+    const float* v = qv + 6 * i;
+    const Q4 q = qnorm_or_identity(Q4{p[4], p[5], p[6], p[3]});
+    for (int k = 0; k < 3; ++k) {
+      frow(g, g.pos + 3 * i + k, w) = p[k];
+      frow(g, g.vel + 3 * i + k, w) = v[k];
+      frow(g, g.omg + 3 * i + k, w) = v[3 + k];
     }
-    const int jt = g.topo[4 * i + 1], qo = g.topo[4 * i + 2], vo = g.topo[4 * i + 3];
-    if (jt == NEWT_JOINT_FREE) {  // pos, quat xyzw; omega_body, v_body
-      const Q4 q = qnorm_or_identity(Q4{qp[qo + 4], qp[qo + 5], qp[qo + 6], qp[qo + 3]});
-      const V3 vb = qrot_inv(q, v3(qv[vo], qv[vo + 1], qv[vo + 2]));
-      for (int k = 0; k < 3; ++k) frow(g, g.rq + qo + k, sw.w) = qp[qo + k];
-      frow(g, g.rq + qo + 3, sw.w) = q.x; frow(g, g.rq + qo + 4, sw.w) = q.y;
-      frow(g, g.rq + qo + 5, sw.w) = q.z; frow(g, g.rq + qo + 6, sw.w) = q.w;
-      for (int k = 0; k < 3; ++k) frow(g, g.rqd + vo + k, sw.w) = qv[vo + 3 + k];
-      frow(g, g.rqd + vo + 3, sw.w) = vb.x; frow(g, g.rqd + vo + 4, sw.w) = vb.y; frow(g, g.rqd + vo + 5, sw.w) = vb.z;
-    } else if (jt == NEWT_JOINT_HINGE || jt == NEWT_JOINT_SLIDE) {
-      frow(g, g.rq + qo, sw.w) = qp[qo];
-      frow(g, g.rqd + vo, sw.w) = qv[vo];
+    frow(g, g.quat + 4 * i, w) = q.x; frow(g, g.quat + 4 * i + 1, w) = q.y;
+    frow(g, g.quat + 4 * i + 2, w) = q.z; frow(g, g.quat + 4 * i + 3, w) = q.w;
+    return;
+  }
+  const int jt = g.topo[4 * i + 1], qo = g.topo[4 * i + 2], vo = g.topo[4 * i + 3];
+  if (jt == NEWT_JOINT_FREE) {  // pos, quat xyzw; omega_body, v_body
+    const Q4 q = qnorm_or_identity(Q4{qp[qo + 4], qp[qo + 5], qp[qo + 6], qp[qo + 3]});
+    const V3 vb = qrot_inv(q, v3(qv[vo], qv[vo + 1], qv[vo + 2]));
+    for (int k = 0; k < 3; ++k) frow(g, g.rq + qo + k, w) = qp[qo + k];
+    frow(g, g.rq + qo + 3, w) = q.x; frow(g, g.rq + qo + 4, w) = q.y;
+    frow(g, g.rq + qo + 5, w) = q.z; frow(g, g.rq + qo + 6, w) = q.w;
+    for (int k = 0; k < 3; ++k) frow(g, g.rqd + vo + k, w) = qv[vo + 3 + k];
+    frow(g, g.rqd + vo + 3, w) = vb.x; frow(g, g.rqd + vo + 4, w) = vb.y; frow(g, g.rqd + vo + 5, w) = vb.z;
+  } else if (jt == NEWT_JOINT_HINGE || jt == NEWT_JOINT_SLIDE) {
+    frow(g, g.rq + qo, w) = qp[qo];
+    frow(g, g.rqd + vo, w) = qv[vo];
+  }
+}
+NEWT_D void state_out(const StateRun& g, int i, int w, float* qp, float* qv) {
+  if (!g.soa) {
+    float* p = qp + 7 * i;
+    float* v = qv + 6 * i;
+    for (int k = 0; k < 3; ++k) {
+      p[k] = frow(g, g.pos + 3 * i + k, w);
+      v[k] = frow(g, g.vel + 3 * i + k, w);
+      v[3 + k] = frow(g, g.omg + 3 * i + k, w);
     }
+    p[3] = frow(g, g.quat + 4 * i + 3, w); p[4] = frow(g, g.quat + 4 * i, w);
+    p[5] = frow(g, g.quat + 4 * i + 1, w); p[6] = frow(g, g.quat + 4 * i + 2, w);
+    return;
+  }
+  const int jt = g.topo[4 * i + 1], qo = g.topo[4 * i + 2], vo = g.topo[4 * i + 3];
+  if (jt == NEWT_JOINT_FREE) {
+    const Q4 q{frow(g, g.rq + qo + 3, w), frow(g, g.rq + qo + 4, w), frow(g, g.rq + qo + 5, w),
+               frow(g, g.rq + qo + 6, w)};
+    for (int k = 0; k < 3; ++k) qp[qo + k] = frow(g, g.rq + qo + k, w);
+    qp[qo + 3] = q.w; qp[qo + 4] = q.x; qp[qo + 5] = q.y; qp[qo + 6] = q.z;
+    const V3 vw = qrot(q, v3(frow(g, g.rqd + vo + 3, w), frow(g, g.rqd + vo + 4, w), frow(g, g.rqd + vo + 5, w)));
+    qv[vo] = vw.x; qv[vo + 1] = vw.y; qv[vo + 2] = vw.z;
+    for (int k = 0; k < 3; ++k) qv[vo + 3 + k] = frow(g, g.rqd + vo + k, w);
+  } else if (jt == NEWT_JOINT_HINGE || jt == NEWT_JOINT_SLIDE) {
+    qp[qo] = frow(g, g.rq + qo, w);
+    qv[vo] = frow(g, g.rqd + vo, w);
   }
 }
 
-__global__ void state_out(const StateGroup* __restrict__ G, const StateWorld* __restrict__ W, int n,
-                          float* __restrict__ qpos, float* __restrict__ qvel) {
-  const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (t >= n) return;
-  const StateWorld sw = W[t];
-  const StateGroup g = G[sw.g];
-  float* qp = qpos + sw.qoff;
-  float* qv = qvel + sw.voff;
-  for (int i = lane; i < g.size; i += 32) {
-    if (!g.soa) {
-      float* p = qp + 7 * i;
-      float* v = qv + 6 * i;
-      for (int k = 0; k < 3; ++k) {
-        p[k] = frow(g, g.pos + 3 * i + k, sw.w);
-        v[k] = frow(g, g.vel + 3 * i + k, sw.w);
-        v[3 + k] = frow(g, g.omg + 3 * i + k, sw.w);
-      }
-      p[3] = frow(g, g.quat + 4 * i + 3, sw.w); p[4] = frow(g, g.quat + 4 * i, sw.w);
-      p[5] = frow(g, g.quat + 4 * i + 1, sw.w); p[6] = frow(g, g.quat + 4 * i + 2, sw.w);
-      continue;
+template <int MOVE>
+NEWT_D void move_tile(const StateRun* runs, int n, float* qpos, float* qvel) {
+  extern __shared__ float tile_s[];
+  int lo = 0, hi = n - 1;  // the run this block's first block count falls in
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (runs[mid].blk <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
+  }
+  const StateRun g = runs[lo];
+  const int base = ((int)blockIdx.x - g.blk) * g.tile, T = min(g.tile, g.n - base), w0 = g.w0 + base;
+  const int nq = MOVE == QFRC_IN ? 0 : g.nq, nv = g.nv, tid = threadIdx.x, nt = blockDim.x;
+  float* sq = tile_s;
+  float* sv = tile_s + g.tile * nq;
+  float* q = qpos + g.q0 + (long)base * nq;
+  float* v = qvel + g.v0 + (long)base * nv;
+  if (MOVE != STATE_OUT) {
+    for (int e = tid; e < T * nq; e += nt) sq[e] = q[e];
+    for (int e = tid; e < T * nv; e += nt) sv[e] = v[e];
+    __syncthreads();
+  }
+  if (MOVE == QFRC_IN) {
+    if (g.soa)  // free bodies carry no generalised force
+      for (int e = tid; e < 32 * nv; e += nt)
+        if ((e & 31) < T) frow(g, g.rf + (e >> 5), w0 + (e & 31)) = sv[(e & 31) * nv + (e >> 5)];
+    return;
+  }
+  if (g.soa) {  // worlds side by side (a tile of at most 32)
+    for (int e = tid; e < 32 * g.size; e += nt) {
+      const int j = e & 31, i = e >> 5;
+      if (j >= T) continue;
+      if (MOVE == STATE_IN) state_in(g, i, w0 + j, sq + j * nq, sv + j * nv);
+      else state_out(g, i, w0 + j, sq + j * nq, sv + j * nv);
     }
-    const int jt = g.topo[4 * i + 1], qo = g.topo[4 * i + 2], vo = g.topo[4 * i + 3];
-    if (jt == NEWT_JOINT_FREE) {
-      const Q4 q{frow(g, g.rq + qo + 3, sw.w), frow(g, g.rq + qo + 4, sw.w), frow(g, g.rq + qo + 5, sw.w),
-                 frow(g, g.rq + qo + 6, sw.w)};
-      for (int k = 0; k < 3; ++k) qp[qo + k] = frow(g, g.rq + qo + k, sw.w);
-      qp[qo + 3] = q.w; qp[qo + 4] = q.x; qp[qo + 5] = q.y; qp[qo + 6] = q.z;
-      const V3 vw = qrot(q, v3(frow(g, g.rqd + vo + 3, sw.w), frow(g, g.rqd + vo + 4, sw.w),
-                               frow(g, g.rqd + vo + 5, sw.w)));
-      qv[vo] = vw.x; qv[vo + 1] = vw.y; qv[vo + 2] = vw.z;
-      for (int k = 0; k < 3; ++k) qv[vo + 3 + k] = frow(g, g.rqd + vo + k, sw.w);
-    } else if (jt == NEWT_JOINT_HINGE || jt == NEWT_JOINT_SLIDE) {
-      qp[qo] = frow(g, g.rq + qo, sw.w);
-      qv[vo] = frow(g, g.rqd + vo, sw.w);
+  } else {
+    for (int e = tid; e < T * g.size; e += nt) {
+      const int j = e / g.size, i = e % g.size;
+      if (MOVE == STATE_IN) state_in(g, i, w0 + j, sq + j * nq, sv + j * nv);
+      else state_out(g, i, w0 + j, sq + j * nq, sv + j * nv);
     }
   }
-}
-
-bool host_pinned(const void* p) {
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
-  return a.type == cudaMemoryTypeHost;
-}
-
-// The call's worlds: per distinct group a StateGroup, per world its entry,
-// in the staging's head; returns the offsets of qpos and qvel in the staging.
-struct StatePlan { std::vector<StateGroup> groups; std::vector<StateWorld> worlds; long nq = 0, nv = 0; };
-StatePlan plan_state(newt_gpu_ctx* ctx, const int32_t* slots, int n) {
-  StatePlan P;
-  std::vector<int> gslot(ctx->groups.size(), -1);
-  for (int i = 0; i < n; ++i) {
-    const SlotRef& r = ctx->slots[slots[i]];
-    const HostModel& m = ctx->models[r.model];
-    if (gslot[r.group] < 0) {
-      const HostGroup& hg = *ctx->groups[r.group];
-      StateGroup g{};
-      g.F = hg.dF;
-      g.soa = hg.soa() ? 1 : 0;
-      g.cap = hg.cap;
-      g.size = hg.size;
-      g.frows = (long)hg.frows;
-      g.pos = hg.lay.pos; g.quat = hg.lay.quat; g.vel = hg.lay.vel; g.omg = hg.lay.omg;
-      g.rq = hg.r_q; g.rqd = hg.r_qd;
-      g.topo = hg.dtopo;
-      gslot[r.group] = (int)P.groups.size();
-      P.groups.push_back(g);
-    }
-    P.worlds.push_back(StateWorld{gslot[r.group], r.index, (int)P.nq, (int)P.nv});
-    P.nq += m.nq;
-    P.nv += m.nv;
+  if (MOVE == STATE_OUT) {
+    __syncthreads();
+    for (int e = tid; e < T * nq; e += nt) q[e] = sq[e];
+    for (int e = tid; e < T * nv; e += nt) v[e] = sv[e];
   }
-  return P;
+}
+template <int MOVE, int N>
+__global__ void __launch_bounds__(256) state_move(const __grid_constant__ StateRuns<N> R, float* qpos, float* qvel) {
+  move_tile<MOVE>(R.r, R.n, qpos, qvel);
+}
+template <int MOVE>
+__global__ void __launch_bounds__(256) state_move_table(const StateRun* R, int n, float* qpos, float* qvel) {
+  move_tile<MOVE>(R, n, qpos, qvel);
+}
+
+// The device's address of n floats of page-locked host memory, or null.
+float* device_view(const void* p, size_t n) {
+  if (n == 0 || ((uintptr_t)p & 3)) return nullptr;
+  const char* last = (const char*)p + n * sizeof(float) - 1;
+  cudaPointerAttributes a, b;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaPointerGetAttributes(&b, last) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer || !b.devicePointer ||
+      (const char*)b.devicePointer - (const char*)a.devicePointer != last - (const char*)p)
+    return nullptr;
+  return (float*)a.devicePointer;
 }
 
 size_t up256(size_t b) { return (b + 255) & ~(size_t)255; }
 
+// The call's worlds as runs.  Slots are named in ascending order when none
+// can be named twice.
+struct StatePlan {
+  std::vector<StateRun> runs;
+  long nq = 0, nv = 0;
+  bool ascending = true;
+};
+int plan_state(newt_gpu_ctx* ctx, const int32_t* slots, int n, StatePlan& P) {
+  const int n_slots = (int)ctx->slots.size();
+  const SlotRef* refs = ctx->slots.data();
+  int group = -1, next = -1, prev = -1, nq = 0, nv = 0;
+  for (int i = 0; i < n; ++i) {
+    const int s = slots[i];
+    if (s < 0 || s >= n_slots || !refs[s].live) {
+      ctx->err = "bad slot";
+      return NEWT_E_INVALID;
+    }
+    P.ascending = P.ascending && s > prev;
+    prev = s;
+    if (refs[s].group != group || refs[s].index != next) {
+      group = refs[s].group;
+      const HostGroup& hg = *ctx->groups[group];
+      const HostModel& m = ctx->models[refs[s].model];  // a group's models have one layout
+      nq = m.nq;
+      nv = m.nv;
+      StateRun g{};
+      g.F = hg.dF;
+      g.topo = hg.dtopo;
+      g.frows = (long)hg.frows;
+      g.q0 = P.nq;
+      g.v0 = P.nv;
+      g.soa = hg.soa() ? 1 : 0;
+      g.cap = hg.cap;
+      g.size = hg.size;
+      g.nq = nq;
+      g.nv = nv;
+      g.pos = hg.lay.pos; g.quat = hg.lay.quat; g.vel = hg.lay.vel; g.omg = hg.lay.omg;
+      g.rq = hg.r_q; g.rqd = hg.r_qd; g.rf = hg.r_qfrc;
+      g.w0 = refs[s].index;
+      P.runs.push_back(g);
+      next = g.w0;
+    }
+    ++P.runs.back().n;
+    ++next;
+    P.nq += nq;
+    P.nv += nv;
+  }
+  return NEWT_OK;
+}
+
+template <int MOVE, int N>
+void launch_runs(const StateRun* runs, int n, int blocks, size_t smem, float* q, float* v, cudaStream_t st) {
+  StateRuns<N> R;
+  R.n = n;
+  std::copy(runs, runs + n, R.r);
+  state_move<MOVE, N><<<blocks, 256, smem, st>>>(R, q, v);
+}
+
+// Moves the planned runs [first, first + count) between the rows and the
+// arrays at device addresses q and v; `table`: room for the runs in the
+// staging (host and device), used past 128.
+template <int MOVE>
+int move_runs(newt_gpu_ctx* ctx, StatePlan& P, size_t first, size_t count, float* q, float* v, size_t table) {
+  int blocks = 0;
+  size_t smem = 0;
+  StateRun* runs = P.runs.data() + first;
+  for (size_t k = 0; k < count; ++k) {
+    StateRun& g = runs[k];
+    const int per = std::max(1, (MOVE == QFRC_IN ? 0 : g.nq) + g.nv);
+    g.tile = std::min(32, std::max(1, TILE_FLOATS / per));
+    g.blk = blocks;
+    blocks += (g.n + g.tile - 1) / g.tile;
+    smem = std::max(smem, (size_t)g.tile * per * sizeof(float));
+  }
+  if (blocks == 0) return NEWT_OK;
+  if (count <= 2) {
+    launch_runs<MOVE, 2>(runs, (int)count, blocks, smem, q, v, ctx->stream);
+  } else if (count <= 24) {
+    launch_runs<MOVE, 24>(runs, (int)count, blocks, smem, q, v, ctx->stream);
+  } else if (count <= 128) {
+    launch_runs<MOVE, 128>(runs, (int)count, blocks, smem, q, v, ctx->stream);
+  } else {
+    StateRun* h = (StateRun*)((char*)ctx->io_h + table);
+    StateRun* d = (StateRun*)((char*)ctx->io_d + table);
+    std::copy(runs, runs + count, h);
+    CKW(cudaMemcpyAsync(d, h, count * sizeof(StateRun), cudaMemcpyHostToDevice, ctx->stream));
+    state_move_table<MOVE><<<blocks, 256, smem, ctx->stream>>>(d, (int)count, q, v);
+  }
+  ctx->launches++;
+  CKW(cudaGetLastError());
+  return NEWT_OK;
+}
+
+// A slot named twice?
+bool repeats(newt_gpu_ctx* ctx, const int32_t* slots, int n) {
+  std::vector<char> seen(ctx->slots.size(), 0);
+  for (int i = 0; i < n; ++i) {
+    if (seen[slots[i]]) return true;
+    seen[slots[i]] = 1;
+  }
+  return false;
+}
+
+// The arrays as the device reaches them: page-locked ones as they are, others
+// by the staging, past the run table.
+struct Views { float *q = nullptr, *v = nullptr; bool q_staged = false, v_staged = false; size_t qo = 0, vo = 0; };
+int view_arrays(newt_gpu_ctx* ctx, const StatePlan& P, const void* qpos, const void* qvel, Views& w) {
+  const size_t table = P.runs.size() > 128 ? up256(P.runs.size() * sizeof(StateRun)) : 0;
+  const size_t nq = qpos ? (size_t)P.nq : 0, nv = (size_t)P.nv;
+  w.q = device_view(qpos, nq);
+  w.v = device_view(qvel, nv);
+  w.q_staged = nq > 0 && !w.q;
+  w.v_staged = nv > 0 && !w.v;
+  w.qo = table;
+  w.vo = table + (w.q_staged ? up256(nq * sizeof(float)) : 0);
+  const size_t bytes = w.vo + (w.v_staged ? nv * sizeof(float) : 0);
+  if (bytes > 0) {
+    const int rc = ensure_staging(ctx, 0, bytes / sizeof(float) + 1);
+    if (rc != NEWT_OK) return rc;
+  }
+  if (w.q_staged) w.q = device_view((char*)ctx->io_h + w.qo, nq);
+  if (w.v_staged) w.v = device_view((char*)ctx->io_h + w.vo, nv);
+  return NEWT_OK;
+}
+
 }  // namespace
 
 int io_state_in(newt_gpu_ctx* ctx, const int32_t* slots, int n, const float* qpos, const float* qvel) {
-  if (n <= 0) return NEWT_OK;
-  const StatePlan P = plan_state(ctx, slots, n);
-  const size_t gb = up256(P.groups.size() * sizeof(StateGroup)), wb = up256(P.worlds.size() * sizeof(StateWorld));
-  const size_t qb = up256(P.nq * sizeof(float)), vb = P.nv * sizeof(float);
-  int rc = ensure_staging(ctx, 0, (gb + wb + qb + vb) / sizeof(float) + 1);
+  StatePlan P;
+  int rc = plan_state(ctx, slots, n, P);
   if (rc != NEWT_OK) return rc;
-  char* h = (char*)ctx->io_h;
-  char* d = (char*)ctx->io_d;
-  std::memcpy(h, P.groups.data(), P.groups.size() * sizeof(StateGroup));
-  std::memcpy(h + gb, P.worlds.data(), P.worlds.size() * sizeof(StateWorld));
-  CKW(cudaMemcpyAsync(d, h, gb + wb, cudaMemcpyHostToDevice, ctx->stream));
-  // page-locked caller arrays go by DMA as they are; others through the staging
-  const bool pinned = host_pinned(qpos) && host_pinned(qvel);
-  if (!pinned) {
-    std::memcpy(h + gb + wb, qpos, P.nq * sizeof(float));
-    std::memcpy(h + gb + wb + qb, qvel, vb);
+  if (!P.ascending && repeats(ctx, slots, n)) {
+    ctx->err = "slot named twice";
+    return NEWT_E_INVALID;
   }
-  CKW(cudaMemcpyAsync(d + gb + wb, pinned ? (const void*)qpos : (const void*)(h + gb + wb), P.nq * sizeof(float),
-                      cudaMemcpyHostToDevice, ctx->stream));
-  CKW(cudaMemcpyAsync(d + gb + wb + qb, pinned ? (const void*)qvel : (const void*)(h + gb + wb + qb), vb,
-                      cudaMemcpyHostToDevice, ctx->stream));
-  const long threads = 32L * n;
-  state_in<<<(int)((threads + 255) / 256), 256, 0, ctx->stream>>>((const StateGroup*)d, (const StateWorld*)(d + gb), n,
-                                                                   (const float*)(d + gb + wb),
-                                                                   (const float*)(d + gb + wb + qb));
-  ctx->launches++;
-  CKW(cudaGetLastError());
+  Views w;
+  if ((rc = view_arrays(ctx, P, qpos, qvel, w)) != NEWT_OK) return rc;
+  if (w.q_staged) std::memcpy((char*)ctx->io_h + w.qo, qpos, P.nq * sizeof(float));
+  if (w.v_staged) std::memcpy((char*)ctx->io_h + w.vo, qvel, P.nv * sizeof(float));
+  if ((rc = move_runs<STATE_IN>(ctx, P, 0, P.runs.size(), w.q, w.v, 0)) != NEWT_OK) return rc;
   CKW(cudaStreamSynchronize(ctx->stream));  // the caller's arrays and the staging are free again
   return NEWT_OK;
 }
 
 int io_state_out(newt_gpu_ctx* ctx, const int32_t* slots, int n, float* qpos, float* qvel) {
-  if (n <= 0) return NEWT_OK;
-  const StatePlan P = plan_state(ctx, slots, n);
-  const size_t gb = up256(P.groups.size() * sizeof(StateGroup)), wb = up256(P.worlds.size() * sizeof(StateWorld));
-  const size_t qb = up256(P.nq * sizeof(float)), vb = P.nv * sizeof(float);
-  int rc = ensure_staging(ctx, 0, (gb + wb + qb + vb) / sizeof(float) + 1);
+  StatePlan P;
+  int rc = plan_state(ctx, slots, n, P);
   if (rc != NEWT_OK) return rc;
-  char* h = (char*)ctx->io_h;
-  char* d = (char*)ctx->io_d;
-  std::memcpy(h, P.groups.data(), P.groups.size() * sizeof(StateGroup));
-  std::memcpy(h + gb, P.worlds.data(), P.worlds.size() * sizeof(StateWorld));
-  CKW(cudaMemcpyAsync(d, h, gb + wb, cudaMemcpyHostToDevice, ctx->stream));
-  const long threads = 32L * n;
-  state_out<<<(int)((threads + 255) / 256), 256, 0, ctx->stream>>>((const StateGroup*)d, (const StateWorld*)(d + gb),
-                                                                    n, (float*)(d + gb + wb), (float*)(d + gb + wb + qb));
-  ctx->launches++;
-  CKW(cudaGetLastError());
-  const bool pinned = host_pinned(qpos) && host_pinned(qvel);
-  CKW(cudaMemcpyAsync(pinned ? (void*)qpos : (void*)(h + gb + wb), d + gb + wb, P.nq * sizeof(float),
-                      cudaMemcpyDeviceToHost, ctx->stream));
-  CKW(cudaMemcpyAsync(pinned ? (void*)qvel : (void*)(h + gb + wb + qb), d + gb + wb + qb, vb, cudaMemcpyDeviceToHost,
-                      ctx->stream));
+  Views w;
+  if ((rc = view_arrays(ctx, P, qpos, qvel, w)) != NEWT_OK) return rc;
+  if ((rc = move_runs<STATE_OUT>(ctx, P, 0, P.runs.size(), w.q, w.v, 0)) != NEWT_OK) return rc;
   CKW(cudaStreamSynchronize(ctx->stream));
-  if (!pinned) {
-    std::memcpy(qpos, h + gb + wb, P.nq * sizeof(float));
-    std::memcpy(qvel, h + gb + wb + qb, vb);
+  if (w.q_staged) std::memcpy(qpos, (char*)ctx->io_h + w.qo, P.nq * sizeof(float));
+  if (w.v_staged) std::memcpy(qvel, (char*)ctx->io_h + w.vo, P.nv * sizeof(float));
+  return NEWT_OK;
+}
+
+int io_qfrc_in(newt_gpu_ctx* ctx, const int32_t* slots, int n, const float* qfrc) {
+  StatePlan P;
+  int rc = plan_state(ctx, slots, n, P);
+  if (rc != NEWT_OK) return rc;
+  Views w;
+  if ((rc = view_arrays(ctx, P, nullptr, qfrc, w)) != NEWT_OK) return rc;
+  if (w.v_staged) std::memcpy((char*)ctx->io_h + w.vo, qfrc, P.nv * sizeof(float));
+  if (P.ascending || !repeats(ctx, slots, n)) {
+    rc = move_runs<QFRC_IN>(ctx, P, 0, P.runs.size(), nullptr, w.v, 0);
+  } else {  // a slot named twice keeps the last forces: the runs in order
+    for (size_t k = 0; k < P.runs.size() && rc == NEWT_OK; ++k)
+      rc = move_runs<QFRC_IN>(ctx, P, k, 1, nullptr, w.v, 0);
   }
+  if (rc != NEWT_OK) return rc;
+  CKW(cudaStreamSynchronize(ctx->stream));
   return NEWT_OK;
 }
 
