@@ -56,3 +56,9 @@ def test_spread_worlds_match_fp64(n):
 def test_stacks_match_fp64(n, rk4):
     rng = np.random.default_rng([7, n])
     _check([stack(rng, n, general=w % 2 == 1) for w in range(4)], rk4=rk4)
+
+
+def test_more_worlds_than_one_wave_match_fp64():
+    """Past three worlds an SM the smallest take their own launch."""
+    rng = np.random.default_rng(9)
+    _check([spread(rng, (1, 2, 6, 9)[w % 4], general=w % 2 == 1, high=w % 16 == 15) for w in range(480)])

@@ -64,7 +64,7 @@ NEWT_D float4 ldg4f(const float* p) { return *reinterpret_cast<const float4*>(p)
 // the worlds of more rows than any holds.
 constexpr int NB_SMALL = 32, NB_MID = 128, NB_BIG = 224;
 struct NewtonLists { int* items; int* counts; int stride; };
-NEWT_D int newton_class(int nr) { return nr <= NB_SMALL ? -1 : nr <= NB_MID ? 0 : nr <= NB_BIG ? 1 : 2; }
+NEWT_D int newton_class(int nr, int small) { return nr <= small ? -1 : nr <= NB_MID ? 0 : nr <= NB_BIG ? 1 : 2; }
 // Active contacts of a world (islands are packed one after another).
 NEWT_D int active_contacts(const WsLay& L, const int* wi) {
   const int nisl = wi[L.misc + 3];
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(32) pile_k_newton_warp(const PileGroupDev* G, 
 // Three instances: 32 rows (a warp, twelve to an SM), 128 rows (whose shared
 // matrix lets three blocks share an SM) and 224 (the most one SM holds).
 // Measured (GB300, us an env-step, one warp per world -> by rows): 250 worlds
-// of 10 boxes (24 to 108 rows) 1047 -> 130 (the solve 1000 -> about 60), 500 of
+// of 10 boxes (24 to 108 rows) 1047 -> 130 (the solve 1000 -> 80), 500 of
 // 16 boxes 2315 -> 340, 4000 of 5 boxes 761 -> 411, 20000 of 2 capsules
 // 743 -> 510 (with 128 rows alone 1280: its blocks are three to an SM).
 
@@ -635,10 +635,10 @@ NEWT_D void newton_block(const PileGroupDev& g, int w, float* nbs) {
     atomicOr(reinterpret_cast<unsigned*>(g.I + (size_t)w * g.lay.istride + g.lay.status), status);
 }
 
-// Every world of the table: those of up to NB_SMALL rows are solved here, the
-// larger ones listed.
+// Every world of the table: those of up to `small` rows (NB_SMALL or none) are
+// solved here, the larger ones listed.
 __global__ void __launch_bounds__(NB_SMALL, 12) pile_k_newton_small(const PileGroupDev* G, const int* wseg, int ng,
-                                                                    int total, NewtonLists lists) {
+                                                                    int total, int small, NewtonLists lists) {
   extern __shared__ __align__(16) float nbs[];
   const int t = blockIdx.x;
   const int gi = find_seg(wseg, ng, t);
@@ -649,7 +649,7 @@ __global__ void __launch_bounds__(NB_SMALL, 12) pile_k_newton_small(const PileGr
   const WsLay L = ws_layout(g.nb, g.np, g.maxc);
   const int nact = active_contacts(L, reinterpret_cast<const int*>(g.scr + (size_t)w * g.sstride + L.nf));
   if (nact == 0) return;  // the velocity changes stay zero
-  const int c = newton_class(4 * nact);
+  const int c = newton_class(4 * nact, small);
   if (c >= 0) {
     if (threadIdx.x == 0) lists.items[c * lists.stride + atomicAdd(lists.counts + c, 1)] = t;
     return;
@@ -699,7 +699,11 @@ extern "C" int newt_launch_pile_newton_solve(const PileGroupDev* dG, const int* 
   const NewtonLists nl{lists, counters, slots};
   auto grid = [&](int per) { return total_worlds < per * sms ? total_worlds : per * sms; };
   auto bytes = [](int rows) { return nb_smem(rows).words * sizeof(float); };
-  pile_k_newton_small<<<total_worlds, NB_SMALL, bytes(NB_SMALL), st>>>(dG, dwseg, ng, total_worlds, nl);
+  // Worlds that the second instance takes in one wave anyway wait for nothing
+  // there: 250 worlds of 10 boxes took 38 us here for the smallest, then 78 us
+  // for the rest; all together they take the 78.
+  const int small = total_worlds <= 3 * sms ? 0 : NB_SMALL;
+  pile_k_newton_small<<<total_worlds, NB_SMALL, bytes(NB_SMALL), st>>>(dG, dwseg, ng, total_worlds, small, nl);
   pile_k_newton_block<NB_MID, 3><<<grid(3), NB_MID, bytes(NB_MID), st>>>(dG, dwseg, ng, nl);
   pile_k_newton_block<NB_BIG, 1><<<grid(1), NB_BIG, bytes(NB_BIG), st>>>(dG, dwseg, ng, nl);
   pile_k_newton_warp<<<grid(16), 32, 0, st>>>(dG, dwseg, ng, nl);
