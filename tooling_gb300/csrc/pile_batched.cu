@@ -52,10 +52,9 @@
 // products, and one shuffle adds the sides.
 //
 // Measured (GB300, us an env-step, one warp per world for the whole horizon
-// before -> now): ten worlds of 16 bodies 206 -> 103, 8192 of 16 bodies
-// 1100 -> 577, 700 of 53 bodies 790 -> 346, 1500 of 12 capsules (RK4)
-// 196 -> 110.  At 8192 worlds the contact stage takes 177 us and the sweeps
-// 460 us under the profiler.
+// before -> now): ten worlds of 16 bodies 206 -> 92, 8192 of 16 bodies
+// 1100 -> 553, 700 of 53 bodies 790 -> 306, 1500 of 12 capsules (RK4)
+// 196 -> 103.
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
@@ -221,20 +220,30 @@ NEWT_D void pair_step(float fi, float fj, float ri, float rj, float h11, float h
 
 constexpr int ACC = 12;  // floats per body of the accumulators (six used): 16-byte aligned, spread over the banks
 
+// What a contact's update reads of its row and does not change.
+struct RowRegs { float4 q0, q1, q2, q3, q4, b, id, a0, a1, pa, pb; };
+NEWT_D RowRegs row_load(const float4* x, int stride, int side) {
+  const float4* sx = x + side * (5 * stride);
+  const float4* cx = x + 10 * stride;
+  return RowRegs{sx[0], sx[stride], sx[2 * stride], sx[3 * stride], sx[4 * stride], cx[stride], cx[2 * stride],
+                 cx[3 * stride], cx[4 * stride], cx[5 * stride], cx[6 * stride]};
+}
+
 // One contact's update (newt/src/solver.rs:1085-1200, 1448-1518) on two
-// neighbouring lanes, this one on side `side`; x: the row's float4s, `stride`
-// apart; A: its body's accumulator (u linear, angular), `write`: unless the
+// neighbouring lanes, this one on side `side`; R: the row's constants, fp: its
+// impulses; A: its body's accumulator (u linear, angular), `write`: unless the
 // side is static.  The other lanes of `pair` take part in the shuffles.
 // SINGLE: a pair whose determinant is not positive (a bit of `single`) takes
-// two half-line steps.
-template <bool SINGLE>
-NEWT_D void row_update(float4* x, int stride, float* A, bool write, int single, int side, unsigned pair) {
-  const float4* sx = x + side * (5 * stride);
-  const float4 q0 = sx[0], q1 = sx[stride], q2 = sx[2 * stride], q3 = sx[3 * stride], q4 = sx[4 * stride];
+// two half-line steps.  ahead: called once the accumulator's loads are out.
+template <bool SINGLE, class F>
+NEWT_D void row_update(const RowRegs& R, float4* fp, float* A, bool write, int single, int side, unsigned pair, F ahead) {
   const float4 u01 = *reinterpret_cast<const float4*>(A);
   const float2 u2 = *reinterpret_cast<const float2*>(A + 4);
-  const f32x2 n0 = lo2(q0), n1 = hi2(q0), n2 = lo2(q1), s0 = hi2(q1), s1 = lo2(q2), s2 = hi2(q2), t0 = lo2(q3),
-              t1 = hi2(q3), t2 = lo2(q4);
+  const float4 f = *fp;
+  ahead();
+  const float4 b = R.b, id = R.id, a0 = R.a0, a1 = R.a1, pa = R.pa, pb = R.pb;
+  const f32x2 n0 = lo2(R.q0), n1 = hi2(R.q0), n2 = lo2(R.q1), s0 = hi2(R.q1), s1 = lo2(R.q2), s2 = hi2(R.q2),
+              t0 = lo2(R.q3), t1 = hi2(R.q3), t2 = lo2(R.q4);
   f32x2 v0 = lo2(u01), v1 = hi2(u01), v2 = pack2(u2.x, u2.y);
   float dn = sum2(fma2(n2, v2, fma2(n1, v1, mul2(n0, v0))));
   float d1 = sum2(fma2(s2, v2, fma2(s1, v1, mul2(s0, v0))));
@@ -242,9 +251,6 @@ NEWT_D void row_update(float4* x, int stride, float* A, bool write, int single, 
   dn += __shfl_xor_sync(pair, dn, 1);
   d1 += __shfl_xor_sync(pair, d1, 1);
   d2 += __shfl_xor_sync(pair, d2, 1);
-  const float4* cx = x + 10 * stride;
-  const float4 f = cx[0], b = cx[stride], id = cx[2 * stride], a0 = cx[3 * stride], a1 = cx[4 * stride],
-               pa = cx[5 * stride], pb = cx[6 * stride];
   // residuals with the row's own regulariser
   float e0 = (fmaf(a1.w, f.x, b.x) + dn) + d1, e1 = (fmaf(a1.w, f.y, b.y) + dn) - d1;
   float e2 = (fmaf(a1.w, f.z, b.z) + dn) + d2, e3 = (fmaf(a1.w, f.w, b.w) + dn) - d2;
@@ -280,13 +286,13 @@ NEWT_D void row_update(float4* x, int stride, float* A, bool write, int single, 
     *reinterpret_cast<ulonglong2*>(A) = make_ulonglong2(v0, v1);
     *reinterpret_cast<f32x2*>(A + 4) = v2;
   }
-  if (!side) x[ROW_F4 * stride] = make_float4(r0, r1, r2, r3);
+  if (!side) *fp = make_float4(r0, r1, r2, r3);
 }
 
 // The same out of line, for rows in either memory and any pairs.
 __device__ __noinline__ void row_update_far(float4* x, int stride, float* A, bool write, int single, int side,
                                             unsigned pair) {
-  row_update<true>(x, stride, A, write, single, side, pair);
+  row_update<true>(row_load(x, stride, side), x + ROW_F4 * stride, A, write, single, side, pair, [] {});
 }
 
 }  // namespace
@@ -580,7 +586,7 @@ NEWT_HD size_t sweep_smem(int S, int nbm, int space) {
 }
 
 template <int S>
-__global__ void __launch_bounds__(32, 16) pile_k_sweep(Worlds W, int nbm, int space, int first, int last,
+__global__ void __launch_bounds__(32, 12) pile_k_sweep(Worlds W, int nbm, int space, int first, int last,
                                                        unsigned long long* work, unsigned* cost) {
   extern __shared__ __align__(16) float4 ssm[];
   constexpr int N = 32 / S;
@@ -652,24 +658,45 @@ __global__ void __launch_bounds__(32, 16) pile_k_sweep(Worlds W, int nbm, int sp
                    xi[X.ci + s] >> 16, side, pair);
   };
   if (fits && __all_sync(FULL, plain)) {
-    // the next round's offsets are read a round ahead
+    // The next round's constants are read while this one's update runs, and
+    // its offsets a round before that: only the accumulators and the impulses,
+    // which the round before may have changed, are waited for.  (Us an
+    // env-step without -> with: ten worlds of 16 bodies 104 -> 92, 8192 of 16
+    // 577 -> 553, 700 of 53 344 -> 306; at 128 registers, where this spills,
+    // 94, 572 and 319.)
     const int2 *at = sched, *end = sched + 32 * nrm;
-    int2 n = nrm > 0 ? *at : make_int2(0, STATIC);
-    for (int k = itm * nrm; k > 0; --k) {
-      const int2 c = n;
+    auto next = [&]() {
+      const int2 c = *at;
       at += 32;
       if (at == end) at = sched;
-      n = *at;
-      row_update<false>(at_bytes(zero, c.x), 1, at_bytes(acc, c.y & ~STATIC), c.y >= 0, 0, side, FULL);
+      return c;
+    };
+    auto load = [&](int2 c) { return row_load(at_bytes(zero, c.x), 1, side); };
+    auto update = [&](const RowRegs& R, int2 c, auto ahead) {
+      row_update<false>(R, at_bytes(zero, c.x) + ROW_F4, at_bytes(acc, c.y & ~STATIC), c.y >= 0, 0, side, FULL, ahead);
       __syncwarp();
+    };
+    int k = itm * nrm;
+    if (k > 0) {
+      int2 c0 = next(), c1 = next();
+      RowRegs R0 = load(c0), R1;
+      for (; k > 1; k -= 2) {
+        int2 c2;
+        update(R0, c0, [&] { R1 = load(c1); c2 = next(); });
+        c0 = c2;
+        update(R1, c1, [&] { R0 = load(c0); c2 = next(); });
+        c1 = c2;
+      }
+      if (k > 0) update(R0, c0, [] {});
     }
   } else if (fits) {  // the same, then the round's rows that go out of line
     for (int it = 0; it < itm; ++it)
       for (int r = 0; r < nrm; ++r) {
         const int2 c = sched[32 * r];
         const bool on = it < iters, far = on && (c.y & FAR), near = on && !far;
-        row_update<false>(at_bytes(zero, near ? c.x : 0), 1, at_bytes(acc, near ? c.y & ~STATIC : 4 * ACC * nbm),
-                          near && c.y >= 0, 0, side, FULL);
+        float4* x = at_bytes(zero, near ? c.x : 0);
+        row_update<false>(row_load(x, 1, side), x + ROW_F4, at_bytes(acc, near ? c.y & ~STATIC : 4 * ACC * nbm),
+                          near && c.y >= 0, 0, side, FULL, [] {});
         if (__any_sync(FULL, far)) {
           if (far) far_update(c.x, c.y);
           __syncwarp();
