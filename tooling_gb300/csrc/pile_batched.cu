@@ -52,9 +52,9 @@
 // products, and one shuffle adds the sides.
 //
 // Measured (GB300, us an env-step, one warp per world for the whole horizon
-// before -> now): ten worlds of 16 bodies 206 -> 92, 8192 of 16 bodies
-// 1100 -> 553, 700 of 53 bodies 790 -> 306, 1500 of 12 capsules (RK4)
-// 196 -> 103.
+// before -> now): ten worlds of 16 bodies 206 -> 88, 8192 of 16 bodies
+// 1100 -> 505, 700 of 53 bodies 790 -> 289, 1500 of 12 capsules (RK4)
+// 196 -> 97.
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
@@ -330,8 +330,8 @@ namespace {
 
 // Per-warp shared memory of pile_k_contacts, in words: the world record's
 // model and state as they lie there (PileLayout's floats up to the contacts,
-// its ints up to the contact pairs), per body R C_b, the AABBs, the
-// broadphase's buffers, then the first `ccap` contacts.  The pair list's
+// its ints up to the contact pairs), per body R C_b, the AABBs, the pair list,
+// then the first `ccap` contacts.  The pair list's
 // place holds the active contacts' lists once the narrowphase is done.
 struct HotLay {
   WsLay L;  // offsets from the floats and from the ints, as collide() takes them
@@ -344,7 +344,6 @@ NEWT_HD HotLay hot_layout(const PileLayout& P, int nb, int np, int maxc) {
   L.nb = nb; L.np = np; L.ng = nb + np; L.maxc = maxc;
   const int all = L.ng * (L.ng - 1) / 2;
   L.pcap = all < 2 * maxc ? all : 2 * maxc;
-  L.words = (L.ng + 31) / 32;
   L.pos = P.pos; L.quat = P.quat; L.vel = P.vel; L.omg = P.omg; L.mass = P.mass; L.iinvb = P.iinv; L.size = P.size;
   L.gpos = P.gpos; L.gquat = P.gquat; L.plane = P.plane; L.fric = P.fric; L.margin = P.margin; L.soft = P.soft;
   L.dtg = P.dtg;
@@ -354,7 +353,7 @@ NEWT_HD HotLay hot_layout(const PileLayout& P, int nb, int np, int maxc) {
   h.ints = f;
   L.shape = P.shape; L.gent = P.gent;
   int i = (P.cpair + 3) / 4 * 4;
-  L.misc = i; i += 4; L.perm = i; i += 64; L.bits = i; i += L.ng * L.words;
+  L.misc = i; i += 4;
   const int lists = 2 * L.pcap > 3 * maxc + 2 ? 2 * L.pcap : 3 * maxc + 2;
   L.pairs = i; i += lists;
   f += i;
