@@ -409,76 +409,89 @@ NEWT_D void tc_kinematics(const TreeGroupDev& g, int w, float* pose, int* topo, 
   }
 }
 
+// A candidate pair and its geoms' model rows: l the link's geom (side a of an
+// in-tree pair), p the plane (side b).  All of a pair's loads are out at once,
+// well before the narrowphase wants them.
+struct PairGeoms {
+  int a = -1, b = 0, gl = 0, gp = 0;
+  float l[GREC], p[GREC];
+};
+NEWT_D PairGeoms tc_pair(const TcGroupDev& G, int w, int pi) {
+  PairGeoms q;
+  if (pi >= G.npairs) return q;
+  const int cap = G.t.cap;
+  q.a = G.pairs[2 * pi];
+  q.b = G.pairs[2 * pi + 1];
+  const bool swap = G.gtopo[2 * q.a + 1] < 0;
+  q.gl = swap ? q.b : q.a;
+  q.gp = swap ? q.a : q.b;
+  const float* gl = G.geom + (size_t)GREC * q.gl * cap + w;
+  const float* gp = G.geom + (size_t)GREC * q.gp * cap + w;
+#pragma unroll
+  for (int f = 0; f < GREC; ++f) {
+    q.l[f] = gl[(size_t)f * cap];
+    q.p[f] = gp[(size_t)f * cap];
+  }
+  return q;
+}
+
 // Contacts and their rows: the link-plane pairs' contacts (and in-tree
 // pairs') to the world's scratch, the rows' contact and kind to rcon and
 // rfac.  Returns the rows; the re-solve of the contact sensors takes the
-// last step's contacts.
-NEWT_D int tc_contacts(const TcGroupDev& G, int w, const float* pose, int* rcon, int* rfac, bool resolve, int lane,
-                       int* ncon_out, uint32_t* status) {
+// last step's contacts.  first: the lane's pair of the first 32.
+NEWT_D int tc_contacts(const TcGroupDev& G, int w, const float* pose, const PairGeoms& first, int* rcon, int* rfac,
+                       bool resolve, int lane, int* ncon_out, uint32_t* status) {
   const TreeGroupDev& g = G.t;
-  const int cap = g.cap;
   const TcLay lay = tc_layout(g.L, g.nv, G.ng, G.maxc, G.rpc);
   float* wf = G.scr + (size_t)w * G.sstride;
-  const float* gm = G.geom;
-  auto gv = [&](int gi, int f) { return gm[(size_t)(GREC * gi + f) * cap + w]; };
   // ---- contacts in newt's pair order (link-plane pairs, and in-tree pairs
   //      when the tree collides with itself): lane per pair, a warp scan
   //      places each pair's contacts ----
   float* con = wf + lay.con;
   int ncon = resolve ? min(max(__float_as_int(wf[lay.misc]), 0), G.maxc) : 0;
   bool overflow = false;
-  auto link_geom_pose = [&](int gi) {
-    const float* lp = pose + 7 * G.gtopo[2 * gi + 1];
+  auto link_geom_pose = [&](int link, const float* m) {
+    const float* lp = pose + 7 * link;
     const Q4 lo = Q4{lp[3], lp[4], lp[5], lp[6]};
     GPose gp;
-    gp.p = ldv3(lp) + qrot(lo, v3(gv(gi, G_POS), gv(gi, G_POS + 1), gv(gi, G_POS + 2)));
-    gp.q = qmul(lo, Q4{gv(gi, G_QUAT), gv(gi, G_QUAT + 1), gv(gi, G_QUAT + 2), gv(gi, G_QUAT + 3)});
+    gp.p = ldv3(lp) + qrot(lo, ldv3(m + G_POS));
+    gp.q = qmul(lo, Q4{m[G_QUAT], m[G_QUAT + 1], m[G_QUAT + 2], m[G_QUAT + 3]});
     return gp;
   };
   for (int base = 0; base < (resolve ? 0 : G.npairs); base += 32) {
-    const int pi = base + lane;
+    PairGeoms q = first;
+    if (base > 0) q = tc_pair(G, w, base + lane);
     CRes cr[4];
-    int nc = 0, a = 0, b = 0, link = 0, link2 = -1;
-    bool a_static = false, flip = false;
-    if (pi < G.npairs && G.gtopo[2 * G.pairs[2 * pi] + 1] >= 0 && G.gtopo[2 * G.pairs[2 * pi + 1] + 1] >= 0) {
-      // in-tree pair: side a (+1) and side b (-1) both on the tree
-      a = G.pairs[2 * pi];
-      b = G.pairs[2 * pi + 1];
-      link = G.gtopo[2 * a + 1];
-      link2 = G.gtopo[2 * b + 1];
-      const float margin = fmaxf(gv(a, G_MARGIN), gv(b, G_MARGIN));
+    int nc = 0, link = 0, link2 = -1, shape = 0;
+    const int a = q.a, b = q.b;
+    bool flip = false;
+    if (a >= 0) {
+      link = G.gtopo[2 * q.gl + 1];
+      link2 = G.gtopo[2 * q.gp + 1];  // -1: a plane
+      shape = G.gtopo[2 * q.gl];
+    }
+    const bool a_static = a >= 0 && q.gl != a;
+    const float margin = fmaxf(q.l[G_MARGIN], q.p[G_MARGIN]);
+    if (link2 >= 0) {  // in-tree pair: side a (+1) and side b (-1) both on the tree
       CRes ct[4];  // its own buffer: `cr` stays in registers on the link-plane path
-      nc = np_link_pair(G.gtopo[2 * a], G.gtopo[2 * b], link_geom_pose(a), link_geom_pose(b),
-                        v3(gv(a, G_SIZE), gv(a, G_SIZE + 1), gv(a, G_SIZE + 2)),
-                        v3(gv(b, G_SIZE), gv(b, G_SIZE + 1), gv(b, G_SIZE + 2)), margin, ct, &flip);
+      nc = np_link_pair(shape, G.gtopo[2 * b], link_geom_pose(link, q.l), link_geom_pose(link2, q.p),
+                        ldv3(q.l + G_SIZE), ldv3(q.p + G_SIZE), margin, ct, &flip);
 #pragma unroll
       for (int k = 0; k < 4; ++k)
         if (k < nc) cr[k] = ct[k];
-    } else if (pi < G.npairs) {
-      a = G.pairs[2 * pi];
-      b = G.pairs[2 * pi + 1];
-      a_static = G.gtopo[2 * a + 1] < 0;
-      const int gl = a_static ? b : a, gp = a_static ? a : b;  // link geom, plane
-      link = G.gtopo[2 * gl + 1];
-      const int shape = G.gtopo[2 * gl];
-      const float* lp = pose + 7 * link;
-      const Q4 lo = Q4{lp[3], lp[4], lp[5], lp[6]};
-      GPose gpose, ppose;
-      gpose.p = ldv3(lp) + qrot(lo, v3(gv(gl, G_POS), gv(gl, G_POS + 1), gv(gl, G_POS + 2)));
-      gpose.q = qmul(lo, Q4{gv(gl, G_QUAT), gv(gl, G_QUAT + 1), gv(gl, G_QUAT + 2), gv(gl, G_QUAT + 3)});
-      ppose.p = v3(gv(gp, G_POS), gv(gp, G_POS + 1), gv(gp, G_POS + 2));
-      ppose.q = Q4{gv(gp, G_QUAT), gv(gp, G_QUAT + 1), gv(gp, G_QUAT + 2), gv(gp, G_QUAT + 3)};
-      const float margin = fmaxf(gv(a, G_MARGIN), gv(b, G_MARGIN));
+    } else if (a >= 0) {
+      const GPose gpose = link_geom_pose(link, q.l);
+      const GPose ppose{ldv3(q.p + G_POS), Q4{q.p[G_QUAT], q.p[G_QUAT + 1], q.p[G_QUAT + 2], q.p[G_QUAT + 3]}};
       if (shape == NEWT_SHAPE_SPHERE) {
-        nc = np_sphere_plane(gpose, gv(gl, G_SIZE), margin, ppose, cr);
+        nc = np_sphere_plane(gpose, q.l[G_SIZE], margin, ppose, cr);
       } else if (shape == NEWT_SHAPE_BOX) {
-        nc = np_box_plane(gpose, v3(gv(gl, G_SIZE), gv(gl, G_SIZE + 1), gv(gl, G_SIZE + 2)), margin, ppose, cr);
+        nc = np_box_plane(gpose, ldv3(q.l + G_SIZE), margin, ppose, cr);
       } else if (shape == NEWT_SHAPE_CAPSULE) {
-        nc = np_capsule_plane(gpose, gv(gl, G_SIZE), gv(gl, G_SIZE + 1), margin, ppose, cr);
+        nc = np_capsule_plane(gpose, q.l[G_SIZE], q.l[G_SIZE + 1], margin, ppose, cr);
       } else if (shape == NEWT_SHAPE_CYLINDER) {
-        nc = np_cylinder_plane(gpose, gv(gl, G_SIZE), gv(gl, G_SIZE + 1), margin, ppose, cr);
+        nc = np_cylinder_plane(gpose, q.l[G_SIZE], q.l[G_SIZE + 1], margin, ppose, cr);
       } else if (shape == NEWT_SHAPE_ELLIPSOID) {
-        nc = np_ellipsoid_plane(gpose, v3(gv(gl, G_SIZE), gv(gl, G_SIZE + 1), gv(gl, G_SIZE + 2)), margin, ppose, cr);
+        nc = np_ellipsoid_plane(gpose, ldv3(q.l + G_SIZE), margin, ppose, cr);
       }
     }
     int incl = nc;  // inclusive scan of the per-pair counts
@@ -488,32 +501,35 @@ NEWT_D int tc_contacts(const TcGroupDev& G, int w, const float* pose, int* rcon,
     }
     const int total = __shfl_sync(FULL, incl, 31);
     const int off = ncon + incl - nc;
-    for (int k = 0; k < nc; ++k) {
-      if (off + k >= G.maxc) { overflow = true; break; }
-      float* c = con + CREC * (off + k);
-      // the narrowphase ran as (geom, plane); a pair listed as (plane, geom)
-      // is relabelled with the normal flipped (contact.rs:2509-2587)
-      c[K_GA] = __int_as_float(a);
-      c[K_GB] = __int_as_float(b);
-      c[K_LINK] = __int_as_float(link);
-      c[K_LINK2] = __int_as_float(link2);
-      c[K_SIGN] = a_static ? -1.f : 1.f;
-      stv3(c + K_POS, cr[k].pos);
-      stv3(c + K_N, (a_static || flip) ? -cr[k].n : cr[k].n);
-      c[K_PEN] = cr[k].pen;
-      c[K_GAP] = fmaxf(gv(a, G_GAP), gv(b, G_GAP));
-      c[K_MU] = fminf(gv(a, G_FRIC), gv(b, G_FRIC));
-      // combine_solref (geom.rs:156-185), combine_solimp (solver.rs:242)
-      const float ta = gv(a, G_SR), tb = gv(b, G_SR), da = gv(a, G_SR + 1), db = gv(b, G_SR + 1);
-      const bool dira = ta < 0.f, dirb = tb < 0.f;
-      c[K_SR] = dira != dirb ? (dira ? ta : tb) : fminf(ta, tb);
-      c[K_SR + 1] = dira != dirb ? (dira ? da : db) : fminf(da, db);
-      for (int q = 0; q < 3; ++q) c[K_SI + q] = fminf(gv(a, G_SI + q), gv(b, G_SI + q));
-      c[K_SI + 3] = gv(a, G_SI + 3);
-      c[K_SI + 4] = gv(a, G_SI + 4);
-      c[K_CONDIM] = (float)min(G.gtopo[2 * G.ng + a], G.gtopo[2 * G.ng + b]);
-      c[K_MUT] = fminf(gv(a, G_TF), gv(b, G_TF));  // combine_torsional_friction
-      c[K_MUR] = fminf(gv(a, G_RF), gv(b, G_RF));  // combine_rolling_friction
+    if (nc > 0) {
+      // combine_solref (geom.rs:156-185), combine_solimp (solver.rs:242),
+      // combine_torsional_friction, combine_rolling_friction
+      const float ta = q.l[G_SR], tb = q.p[G_SR], da = q.l[G_SR + 1], db = q.p[G_SR + 1];
+      const bool dira = ta < 0.f, dirb = tb < 0.f, pick = dira != dirb;
+      const float sr0 = pick ? (dira ? ta : tb) : fminf(ta, tb), sr1 = pick ? (dira ? da : db) : fminf(da, db);
+      const float gap = fmaxf(q.l[G_GAP], q.p[G_GAP]), mu = fminf(q.l[G_FRIC], q.p[G_FRIC]);
+      const float condim = (float)min(G.gtopo[2 * G.ng + a], G.gtopo[2 * G.ng + b]);
+      const bool relabel = a_static || flip;
+      static_assert(K_SIGN == 3 && K_POS == 4 && K_N == 7 && K_PEN == 10 && K_GAP == 11 && K_MU == 12 && K_SR == 13 &&
+                        K_SI == 15 && K_CONDIM == 20 && K_ROW == 21 && K_LINK2 == 22 && K_MUR == 24 && CREC == 28,
+                    "the record is written in fours");
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (k >= nc) break;
+        if (off + k >= G.maxc) { overflow = true; break; }
+        float4* c = reinterpret_cast<float4*>(con + CREC * (off + k));
+        // the narrowphase ran as (geom, plane); a pair listed as (plane, geom)
+        // is relabelled with the normal flipped (contact.rs:2509-2587)
+        const V3 p = cr[k].pos, n = relabel ? -cr[k].n : cr[k].n;
+        c[0] = make_float4(__int_as_float(a), __int_as_float(b), __int_as_float(link), a_static ? -1.f : 1.f);
+        c[1] = make_float4(p.x, p.y, p.z, n.x);
+        c[2] = make_float4(n.y, n.z, cr[k].pen, gap);
+        c[3] = make_float4(mu, sr0, sr1, fminf(q.l[G_SI], q.p[G_SI]));
+        c[4] = make_float4(fminf(q.l[G_SI + 1], q.p[G_SI + 1]), fminf(q.l[G_SI + 2], q.p[G_SI + 2]),
+                           a_static ? q.p[G_SI + 3] : q.l[G_SI + 3], a_static ? q.p[G_SI + 4] : q.l[G_SI + 4]);
+        c[5] = make_float4(condim, 0.f, __int_as_float(link2), fminf(q.l[G_TF], q.p[G_TF]));
+        c[6] = make_float4(fminf(q.l[G_RF], q.p[G_RF]), 0.f, 0.f, 0.f);
+      }
     }
     ncon = ncon + total < G.maxc ? ncon + total : G.maxc;
   }
@@ -1035,7 +1051,9 @@ __global__ void __launch_bounds__(32) tc_k_solve(TcGroupDev G) {
   uint32_t status = 0;
   int ncon = 0;
   tc_kinematics(G.t, w, pose, reinterpret_cast<int*>(tcs + sm.vec), nullptr, lane);
-  const int nr = tc_contacts(G, w, pose, rcon, rcon + sm.ldr, G.sens != nullptr, lane, &ncon, &status);
+  const bool resolve = G.sens != nullptr;
+  const PairGeoms first = tc_pair(G, w, resolve ? G.npairs : lane);
+  const int nr = tc_contacts(G, w, pose, first, rcon, rcon + sm.ldr, resolve, lane, &ncon, &status);
   tc_rows_solve<REFINE>(G, w, tcs, nr, ncon, status, lane);
 }
 
@@ -1052,15 +1070,15 @@ extern "C" size_t newt_tc_smem_bytes(int L, int nv, int maxc, int rpc) {
 }
 // The launch of a group: tc_k_small for trees of up to REFINE_NV DoF whose
 // rows are facets or normals, else tc_k_solve.  Blocks of tc_k_small hold
-// TCS_WARPS worlds, fewer where their shared memory would not let two blocks
-// share an SM.
+// TCS_WARPS worlds, fewer where their shared memory would not let TCS_BLOCKS
+// blocks share an SM.
 struct TcPlan { bool small; int warps; size_t bytes; };
 static TcPlan tc_plan(int L, int nv, int maxc, int rpc, bool general, bool resolve) {
   TcPlan p{nv <= REFINE_NV && !general && !resolve, 1, newt_tc_smem_bytes(L, nv, maxc, rpc)};
   if (p.small) {
     const size_t per = (size_t)tcs_smem(L, nv, maxc, rpc).words * sizeof(float);
     p.warps = TCS_WARPS;
-    while (p.warps > 1 && p.warps * per > (227 * 1024 - 2048) / 2) p.warps /= 2;
+    while (p.warps > 1 && p.warps * per > 227 * 1024 / TCS_BLOCKS - 1024) p.warps /= 2;
     p.bytes = p.warps * per;
   }
   return p;

@@ -13,21 +13,25 @@
 //   * M's entries go row by row of its lower triangle, so the base's entries,
 //     which sum every link, share their round;
 //   * the two factors (M + dt B and M) take a half-warp each, two rows a
-//     lane, four columns a load;
+//     lane; every factor and substitution advances four columns at a time,
+//     the 4 x 4 blocks by every lane for itself;
 //   * the rows' forward substitution and the inverse weights' (of the links
 //     that own rows) share one pass, a lane per right-hand side;
 //   * the Newton system stays in a lane's registers, and the sums that steer
 //     its line search are reduced together.
 // Measured on 16384 quadrupeds (13 links, 18 DoF, 0 to 28 rows; GB300, a
 // launch): 1737 us as tc_k_solve, 32000 instructions a world at 14.4 cycles
-// each; 413 us here, 11200 at 10.3 (fetch waits 0.4).  Four, eight or sixteen
-// worlds a block differ by 1 %, 0 and 6 %.
+// each; 379 us here, 10400 at 10.3 (fetch waits 1.1, global memory 2.1, shared
+// memory 1.1, barriers 1.0).  Blocks of four worlds, four to an SM, against
+// eight and two: 917 and 939 us for two env-steps; without the barriers around
+// the Newton stage 932 to 948.
 //
 // Quotients by a factor's pivots are x * r corrected by the remainder
 // x - q d (r the correctly rounded reciprocal of d; P. Markstein, IBM J. Res.
 // Dev. 34(1), 1990).
 
-constexpr int TCS_WARPS = 8;  // worlds (warps) per block
+constexpr int TCS_WARPS = 4;   // worlds (warps) per block
+constexpr int TCS_BLOCKS = 4;  // blocks per SM
 constexpr int TCS_ROWS = 32;  // rows of a world, a lane each
 constexpr int TCS_LDH = 36;   // row stride of H: float4 loads of eight rows meet no bank twice
 
@@ -46,8 +50,8 @@ NEWT_HD TcsSmem tcs_smem(int L, int nv, int maxc, int rpc) {
   m.arms = f; f += up4(9 * L);
   m.wa = f; f += up4(3 * nv);
   m.qd = f; f += 2 * up4(nv);
-  m.lm = f; f += nv * ld;   // M + dt B, then its factor; row-major
-  m.ldm = f; f += nv * ld;  // M
+  m.lm = f; f += up4(nv) * ld;   // M + dt B, then its factor; row-major
+  m.ldm = f; f += up4(nv) * ld;  // M
   m.di = f; f += 2 * 24;    // reciprocals of the pivots
   m.links = f; f += up4(L);
   m.s2 = f; f += up4(3 * L);
@@ -62,7 +66,7 @@ NEWT_HD TcsSmem tcs_smem(int L, int nv, int maxc, int rpc) {
   m.jt = m.h;
   const int jt = nv * 32, hh = TCS_ROWS * TCS_LDH;
   m.x = m.h + (jt > hh ? jt : hh);
-  const int b = m.x + 2 * TCS_ROWS - f;
+  const int b = m.x + 3 * TCS_ROWS - f;
   f += up4(a > b ? a : b);
   m.words = f > o.words ? f : o.words;  // tc_rows_solve's own layout lies in the same words
   return m;
@@ -100,10 +104,73 @@ NEWT_D void arm_columns(const float* pose, const int* topo, const float* arms, c
   }
 }
 
-// Lower Cholesky factors of two n x n row-major matrices, in place (the upper
-// triangles stay), n <= 32: half-warp h factors m[h], lane r of it rows r and
-// r + 16.  The entries' products are subtracted in column order.  di: 1 / pivot,
-// n (<= 24) per matrix.  False when a pivot is not positive.
+// The 4 x 4 diagonal block of a factor, and its reciprocal pivots.
+struct Block4 {
+  float l00, l10, l11, l20, l21, l22, l30, l31, l32, l33, i0, i1, i2, i3;
+  // of the block whose lower entries row q's lane holds in s[0..q]; q's lane is `lane0` + q
+  NEWT_D bool factor(const float (&s)[4], int lane0) {
+    auto at = [&](int u, int q) { return __shfl_sync(FULL, s[u], lane0 + q); };
+    const float d00 = at(0, 0), d10 = at(0, 1), d20 = at(0, 2), d30 = at(0, 3), d11 = at(1, 1), d21 = at(1, 2),
+                d31 = at(1, 3), d22 = at(2, 2), d32 = at(2, 3), d33 = at(3, 3);
+    l00 = sqrtf(d00); i0 = 1.f / l00;
+    l10 = d10 * i0; l20 = d20 * i0; l30 = d30 * i0;
+    const float e11 = fmaf(-l10, l10, d11);
+    l11 = sqrtf(e11); i1 = 1.f / l11;
+    l21 = fmaf(-l20, l10, d21) * i1; l31 = fmaf(-l30, l10, d31) * i1;
+    const float e22 = fmaf(-l21, l21, fmaf(-l20, l20, d22));
+    l22 = sqrtf(e22); i2 = 1.f / l22;
+    l32 = fmaf(-l31, l21, fmaf(-l30, l20, d32)) * i2;
+    const float e33 = fmaf(-l32, l32, fmaf(-l31, l31, fmaf(-l30, l30, d33)));
+    l33 = sqrtf(e33); i3 = 1.f / l33;
+    return d00 > 0.f && e11 > 0.f && e22 > 0.f && e33 > 0.f;
+  }
+  // of the factor m (row-major) at row p, reciprocals at di + p
+  NEWT_D void load(const float* m, int ld, int p, const float* di) {
+    const float4 r1 = f4(m + (p + 1) * ld + p), r2 = f4(m + (p + 2) * ld + p), r3 = f4(m + (p + 3) * ld + p),
+                 i = f4(di + p);
+    l00 = m[p * ld + p];
+    l10 = r1.x; l11 = r1.y;
+    l20 = r2.x; l21 = r2.y; l22 = r2.z;
+    l30 = r3.x; l31 = r3.y; l32 = r3.z; l33 = r3.w;
+    i0 = i.x; i1 = i.y; i2 = i.z; i3 = i.w;
+  }
+  // row q of the block, zeros above the diagonal; its reciprocal pivot
+  NEWT_D float4 row(int q) const {
+    return make_float4(q == 0 ? l00 : q == 1 ? l10 : q == 2 ? l20 : l30, q == 0 ? 0.f : q == 1 ? l11 : q == 2 ? l21 : l31,
+                       q < 2 ? 0.f : q == 2 ? l22 : l32, q < 3 ? 0.f : l33);
+  }
+  NEWT_D float inv(int q) const { return q == 0 ? i0 : q == 1 ? i1 : q == 2 ? i2 : i3; }
+  // a row below the block
+  NEWT_D float4 below(const float (&s)[4]) const {
+    const float y0 = s[0] * i0, y1 = fmaf(-y0, l10, s[1]) * i1, y2 = fmaf(-y1, l21, fmaf(-y0, l20, s[2])) * i2;
+    return make_float4(y0, y1, y2, fmaf(-y2, l32, fmaf(-y1, l31, fmaf(-y0, l30, s[3]))) * i3);
+  }
+  // L y = v and L^T z = v
+  NEWT_D float4 forward(float4 v) const {
+    const float y0 = quot(v.x, l00, i0), y1 = quot(fmaf(-l10, y0, v.y), l11, i1);
+    const float y2 = quot(fmaf(-l21, y1, fmaf(-l20, y0, v.z)), l22, i2);
+    return make_float4(y0, y1, y2, quot(fmaf(-l32, y2, fmaf(-l31, y1, fmaf(-l30, y0, v.w))), l33, i3));
+  }
+  NEWT_D float4 backward(float4 v) const {
+    const float z3 = quot(v.w, l33, i3), z2 = quot(fmaf(-l32, z3, v.z), l22, i2);
+    const float z1 = quot(fmaf(-l21, z2, fmaf(-l31, z3, v.y)), l11, i1);
+    return make_float4(quot(fmaf(-l10, z1, fmaf(-l20, z2, fmaf(-l30, z3, v.x))), l00, i0), z1, z2, z3);
+  }
+};
+NEWT_D float pick(float4 v, int q) { return q == 0 ? v.x : q == 1 ? v.y : q == 2 ? v.z : v.w; }
+NEWT_D float4 shfl4(float v, int lane0) {
+  return make_float4(__shfl_sync(FULL, v, lane0), __shfl_sync(FULL, v, lane0 + 1), __shfl_sync(FULL, v, lane0 + 2),
+                     __shfl_sync(FULL, v, lane0 + 3));
+}
+NEWT_D float minus4(float s, float4 a, float4 b) {  // s - a . b, in order
+  return fmaf(-a.w, b.w, fmaf(-a.z, b.z, fmaf(-a.y, b.y, fmaf(-a.x, b.x, s))));
+}
+
+// Lower Cholesky factors of two n x n row-major matrices (n a multiple of
+// four, <= 24; zeros above the diagonal), in place, four columns at a time:
+// half-warp h factors m[h], lane r of it rows r and r + 16.  The entries'
+// products are subtracted in column order.  di: 1 / pivot, 24 per matrix.
+// False when a pivot is not positive.
 NEWT_D bool chol_pair(float* m0, float* m1, int n, int ld, float* di, int lane) {
   float* m = lane & 16 ? m1 : m0;
   float* d = di + (lane & 16 ? 24 : 0);
@@ -111,56 +178,62 @@ NEWT_D bool chol_pair(float* m0, float* m1, int n, int ld, float* di, int lane) 
   float* r1 = m + (i1 < n ? i1 : n - 1) * ld;
   float* r2 = m + (i2 < n ? i2 : n - 1) * ld;
   bool ok = true;
-  for (int j = 0; j < n; ++j) {
-    const float* rj = m + j * ld;
-    float s1 = r1[j], s2 = r2[j];
-    for (int k = 0; k < j; k += 4) {
-      float4 c = f4(rj + k);
+  for (int p = 0; p < n; p += 4) {
+    const float4 c1 = f4(r1 + p), c2 = f4(r2 + p);
+    float s1[4] = {c1.x, c1.y, c1.z, c1.w}, s2[4] = {c2.x, c2.y, c2.z, c2.w};
+    for (int k = 0; k < p; k += 4) {
       const float4 a = f4(r1 + k), b = f4(r2 + k);
-      if (k + 1 >= j) c.y = 0.f;
-      if (k + 2 >= j) c.z = 0.f;
-      if (k + 3 >= j) c.w = 0.f;
-      s1 = fmaf(-a.x, c.x, s1); s2 = fmaf(-b.x, c.x, s2);
-      s1 = fmaf(-a.y, c.y, s1); s2 = fmaf(-b.y, c.y, s2);
-      s1 = fmaf(-a.z, c.z, s1); s2 = fmaf(-b.z, c.z, s2);
-      s1 = fmaf(-a.w, c.w, s1); s2 = fmaf(-b.w, c.w, s2);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4 c = f4(m + (p + u) * ld + k);
+        s1[u] = minus4(s1[u], a, c);
+        s2[u] = minus4(s2[u], b, c);
+      }
     }
-    const float piv = __shfl_sync(FULL, j < 16 ? s1 : s2, (lane & 16) | (j & 15));
-    ok = ok && piv > 0.f;
-    const float l = sqrtf(piv), inv = 1.f / l;
-    if (i1 >= j && i1 < n) r1[j] = i1 == j ? l : s1 * inv;
-    if (i2 >= j && i2 < n) r2[j] = i2 == j ? l : s2 * inv;
-    if (i1 == 0) d[j] = inv;
+    Block4 B;
+    ok = (p < 16 ? B.factor(s1, (lane & 16) | p) : B.factor(s2, (lane & 16) | (p & 15))) && ok;
+    if (i1 >= p && i1 < n) *reinterpret_cast<float4*>(r1 + p) = i1 < p + 4 ? B.row(i1 - p) : B.below(s1);
+    if (i2 >= p && i2 < n) *reinterpret_cast<float4*>(r2 + p) = i2 < p + 4 ? B.row(i2 - p) : B.below(s2);
+    if (i1 < 4) d[p + i1] = B.inv(i1);
     __syncwarp();
   }
   return __all_sync(FULL, ok);
 }
 
-// The same of one matrix, a lane per row; the pivots' range.
-NEWT_D bool chol_one(float* m, int n, int ld, int lane, float* mn, float* mx) {
-  float* r = m + (lane < n ? lane : n - 1) * ld;
+// The same of one matrix, a lane per row, the entries taken above the
+// diagonal, which stay; the range of the first nr pivots.
+NEWT_D bool chol_one(float* m, int n, int nr, int ld, float* di, int lane, float* mn, float* mx) {
+  const int i = lane < n ? lane : n - 1;
+  float* r = m + i * ld;
   float lo = 1e30f, hi = 0.f;
   bool ok = true;
-  for (int j = 0; j < n; ++j) {
-    const float* rj = m + j * ld;
-    float s = rj[lane < n ? lane : n - 1];  // the upper triangle: column j from row j down
-    for (int k = 0; k < j; k += 4) {
-      float4 c = f4(rj + k);
+  for (int p = 0; p < n; p += 4) {
+    float s[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) s[u] = m[(p + u) * ld + i];
+    for (int k = 0; k < p; k += 4) {
       const float4 a = f4(r + k);
-      if (k + 1 >= j) c.y = 0.f;
-      if (k + 2 >= j) c.z = 0.f;
-      if (k + 3 >= j) c.w = 0.f;
-      s = fmaf(-a.x, c.x, s);
-      s = fmaf(-a.y, c.y, s);
-      s = fmaf(-a.z, c.z, s);
-      s = fmaf(-a.w, c.w, s);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) s[u] = minus4(s[u], a, f4(m + (p + u) * ld + k));
     }
-    const float piv = __shfl_sync(FULL, s, j);
-    ok = ok && piv > 0.f;
-    const float l = sqrtf(piv), inv = 1.f / l;
-    lo = l < lo ? l : lo;
-    hi = l > hi ? l : hi;
-    if (lane >= j && lane < n) r[j] = lane == j ? l : s * inv;
+    Block4 B;
+    ok = B.factor(s, p) && ok;
+    lo = fminf(lo, B.l00);
+    hi = fmaxf(hi, B.l00);
+    if (p + 1 < nr) { lo = fminf(lo, B.l11); hi = fmaxf(hi, B.l11); }
+    if (p + 2 < nr) { lo = fminf(lo, B.l22); hi = fmaxf(hi, B.l22); }
+    if (p + 3 < nr) { lo = fminf(lo, B.l33); hi = fmaxf(hi, B.l33); }
+    __syncwarp();
+    if (lane >= p + 4 && lane < n) {
+      *reinterpret_cast<float4*>(r + p) = B.below(s);
+    } else if (lane >= p && lane < n) {
+      const float4 v = B.row(lane - p);
+      r[p] = v.x;
+      if (lane > p) r[p + 1] = v.y;
+      if (lane > p + 1) r[p + 2] = v.z;
+      if (lane > p + 2) r[p + 3] = v.w;
+      di[lane] = B.inv(lane - p);
+    }
     __syncwarp();
   }
   *mn = lo;
@@ -168,15 +241,13 @@ NEWT_D bool chol_one(float* m, int n, int ld, int lane, float* mn, float* mx) {
   return ok;
 }
 
-// a / b by Newton steps on the reciprocal from its FP32 value (an FP64 divide
-// keeps the FP64 pipe busy several times as long).
-NEWT_D double quot_d(double a, double b) {
+// a / b rounded to FP32: the FP32 quotient corrected by its FP64 remainder (an
+// FP64 divide keeps the FP64 pipe busy several times as long).
+NEWT_D float quot_d(double a, double b) {
   const float bf = (float)b;
-  if (!(bf > 1e-30f && bf < 1e30f)) return a / b;
-  double r = (double)(1.f / bf);
-  r = fma(fma(-b, r, 1.0), r, r);
-  const double q = a * r;
-  return fma(fma(-q, b, a), r, q);
+  if (!(bf > 1e-30f && bf < 1e30f)) return (float)(a / b);
+  const float r = 1.f / bf, q = (float)a * r;
+  return fmaf((float)fma(-(double)q, b, a), r, q);
 }
 
 // Row times a shared vector (zeros from nr up to the next multiple of four).
@@ -197,7 +268,7 @@ NEWT_D float row_dot(const float (&h)[TCS_ROWS], const float* x, int nr) {
 // dense::newton_solve for nr <= 32 rows, a lane per row.  H: full symmetric
 // rows of stride TCS_LDH with zeros up to a multiple of four columns; its
 // lower triangle and diagonal are overwritten by the factor.  b: the lane's
-// bias; xs: two shared vectors of 32.  Returns the iterations, or -1 (nothing
+// bias; xs: two shared vectors of 32, then the factor's 32 reciprocal pivots.  Returns the iterations, or -1 (nothing
 // solved) when the factor is too ill-conditioned for FP32.  The lane's impulse
 // in *x_out, its diagonal entry in *hd_out.
 NEWT_D int small_newton(float* H, int nr, float b, float* xs, int iters, int lane, float* x_out, float* hd_out,
@@ -212,11 +283,15 @@ NEWT_D int small_newton(float* H, int nr, float b, float* xs, int iters, int lan
     h[c] = v.x; h[c + 1] = v.y; h[c + 2] = v.z; h[c + 3] = v.w;
   }
   const float hd = row[in ? lane : nr - 1];
+  const int n = up4(nr);
+  float* di = xs + 2 * TCS_ROWS;
+  __syncwarp();
+  if (lane >= nr && lane < n)  // rows of the identity up to a multiple of four
+    for (int c = lane; c < n; ++c) H[lane * TCS_LDH + c] = c == lane ? 1.f : 0.f;
   __syncwarp();
   float mn, mx;
   *hd_out = hd;
-  if (!chol_one(H, nr, TCS_LDH, lane, &mn, &mx) || (mx / mn) * (mx / mn) > 1.0e6f) return -1;
-  const float ld = in ? row[lane] : 1.f, li = 1.f / ld;
+  if (!chol_one(H, n, nr, TCS_LDH, di, lane, &mn, &mx) || (mx / mn) * (mx / mn) > 1.0e6f) return -1;
   float x = 0.f;
   double cur = 0.0;
   int done = 0;
@@ -234,24 +309,22 @@ NEWT_D int small_newton(float* H, int nr, float b, float* xs, int iters, int lan
     const float grad = in ? hx + b : 0.f;
     // d = -(L L^T)^-1 grad
     float d = -grad;
-    for (int k0 = 0; k0 < nr; k0 += 4) {
-      const float4 l = f4(row + k0);
-      const float lk[4] = {l.x, l.y, l.z, l.w};
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int k = k0 + u;
-        const float q = quot(d, ld, li);
-        const float y = __shfl_sync(FULL, q, k & 31);
-        d = lane > k ? fmaf(-lk[u], y, d) : (lane == k ? q : d);
-      }
+    for (int p = 0; p < n; p += 4) {
+      Block4 B;
+      B.load(H, TCS_LDH, p, di);
+      const float4 y = B.forward(shfl4(d, p));
+      d = lane >= p + 4 ? minus4(d, f4(row + p), y) : lane >= p ? pick(y, lane - p) : d;
     }
     if (!in) d = 0.f;
-    for (int k = nr - 1; k >= 0; --k) {
-      const float l = H[k * TCS_LDH + lane];  // L[k][lane], used below the diagonal
-      const float q = quot(d, ld, li);
-      const float z = __shfl_sync(FULL, q, k);
-      d = lane < k ? fmaf(-l, z, d) : (lane == k ? q : d);
+    for (int p = n - 4; p >= 0; p -= 4) {
+      Block4 B;
+      B.load(H, TCS_LDH, p, di);
+      const float* c = H + p * TCS_LDH + lane;  // below the diagonal: the factor's columns, by rows
+      const float l3 = c[3 * TCS_LDH], l2 = c[2 * TCS_LDH], l1 = c[TCS_LDH], l0 = c[0];
+      const float4 z = B.backward(shfl4(d, p));
+      d = lane < p ? fmaf(-l0, z.x, fmaf(-l1, z.y, fmaf(-l2, z.z, fmaf(-l3, z.w, d)))) : lane < p + 4 ? pick(z, lane - p) : d;
     }
+    if (!in) d = 0.f;
     if (dense::warp_sum(grad * d) >= 0.f) break;
     // ---- exact line search over the projected path (newton.rs:435-556) ----
     const bool fr = x > 0.f || (x == 0.f && d > 0.f);
@@ -284,16 +357,22 @@ NEWT_D int small_newton(float* H, int nr, float b, float* xs, int iters, int lan
       const bool last = !(__uint_as_float(bm) < 2.f);
       const float hi = last ? 1.f : __uint_as_float(bm);
       if (hi - lo > 1.0e-7f) {
-        const double c0 = 0.5 * Pu + bP, c1 = Pv + bS, c2 = Sv;
-        const float opt = c2 > 0.0 ? fminf(fmaxf((float)quot_d(-c1, c2), lo), hi) : 0.5f * (lo + hi);
-        // the candidates lo, hi, opt in order, a lane each
-        const float cand = lane == 0 ? lo : lane == 1 ? hi : opt;
-        const double a = cand;
-        const double cost = c0 + c1 * a + 0.5 * c2 * a * a;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const double ck = __shfl_sync(FULL, cost, k);
-          if (ck < best_c) { best_c = ck; best_a = k == 0 ? lo : k == 1 ? hi : opt; }
+        double c0 = 0.0, c1 = bS;
+        const double c2 = Sv;
+        if (it > 0) {
+          c0 = 0.5 * Pu + bP;
+          c1 += Pv;
+        }
+        auto take = [&](float a) {
+          const double cost = c0 + c1 * (double)a + 0.5 * c2 * (double)a * (double)a;
+          if (cost < best_c) { best_c = cost; best_a = a; }
+        };
+        if (c2 > 0.0) {  // the ends are no lower than the clamped minimiser
+          take(fminf(fmaxf(quot_d(-c1, c2), lo), hi));
+        } else {
+          take(lo);
+          take(hi);
+          take(0.5f * (lo + hi));
         }
       }
       if (last) break;
@@ -352,7 +431,7 @@ __device__ __noinline__ int newton_any(float* H, float hd, int nr, float* Hg, fl
 
 }  // namespace
 
-__global__ void __launch_bounds__(32 * TCS_WARPS, 2) tc_k_small(const __grid_constant__ TcGroupDev G) {
+__global__ void __launch_bounds__(32 * TCS_WARPS, TCS_BLOCKS) tc_k_small(const __grid_constant__ TcGroupDev G) {
   extern __shared__ __align__(16) float tcs[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int w = blockIdx.x * (blockDim.x >> 5) + warp;
@@ -386,7 +465,9 @@ __global__ void __launch_bounds__(32 * TCS_WARPS, 2) tc_k_small(const __grid_con
   bool rk4 = false;
 
   // ---- forward kinematics, joint axes and levers ----
+  PairGeoms first;
   if (live) {
+    first = tc_pair(G, w, lane);
     dt = g.dtg[w];
     rk4 = g.integ && g.integ[w] == NEWT_INTEGRATOR_RK4;
     if (lane < nv) {
@@ -414,7 +495,7 @@ __global__ void __launch_bounds__(32 * TCS_WARPS, 2) tc_k_small(const __grid_con
 
   // ---- contacts and their rows ----
   if (live) {
-    nr = tc_contacts(G, w, pose, rcon, rfac, false, lane, &ncon, &status);
+    nr = tc_contacts(G, w, pose, first, rcon, rfac, false, lane, &ncon, &status);
     __syncwarp();
     if (nr == 0 && lane == 0 && status) atomicOr(g.status + w, status);  // qacc stays a_free
   }
@@ -426,8 +507,11 @@ __global__ void __launch_bounds__(32 * TCS_WARPS, 2) tc_k_small(const __grid_con
     float* JV = sv + sm.jv;
     float* IW = sv + sm.iw;  // 6 per link, then the link masses
     float* MS = IW + 6 * L;
-    for (int k = 4 * lane; k < 2 * nv * ldm; k += 128)
+    for (int k = 4 * lane; k < 2 * nq * ldm; k += 128)
       *reinterpret_cast<float4*>(LM + k) = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncwarp();
+    if (lane < nq - nv)  // the identity up to a multiple of four rows
+      LM[(nv + lane) * (ldm + 1)] = LD[(nv + lane) * (ldm + 1)] = 1.f;
     for (int l = lane; l < L; l += 32) {
       const float* pl = pose + 7 * l;
       float* jv = JV + 3 * nv * l;
@@ -486,7 +570,7 @@ __global__ void __launch_bounds__(32 * TCS_WARPS, 2) tc_k_small(const __grid_con
   }
   __syncthreads();
   if (on) {
-    if (!chol_pair(LM, LD, nv, ldm, di, lane)) {
+    if (!chol_pair(LM, LD, nq, ldm, di, lane)) {
       if (lane == 0) atomicOr(g.status + w, status | NEWT_WS_NOT_PD);
       on = false;
     }
@@ -661,12 +745,14 @@ __global__ void __launch_bounds__(32 * TCS_WARPS, 2) tc_k_small(const __grid_con
       for (int r = 0; r < nr; ++r) jf += wf[lay.j0 + (size_t)lane * lay.ld + r] * xs[r];
       g.cfrc[(size_t)w * g.cstride + lane] = jf / dt;
     }
-    const float dv = LM[kv * ldm + kv], rv = di[kv];
-    for (int k = nv - 1; k >= 0; --k) {
-      const float f = LM[k * ldm + kv];
-      const float q = quot(v, dv, rv);
-      const float z = __shfl_sync(FULL, q, k);
-      v = lane < k ? fmaf(-f, z, v) : (lane == k ? q : v);
+    if (lane >= nv) v = 0.f;
+    for (int p = nq - 4; p >= 0; p -= 4) {
+      Block4 B;
+      B.load(LM, ldm, p, di);
+      const float* c = LM + p * ldm + min(lane, nq - 1);
+      const float l3 = c[3 * ldm], l2 = c[2 * ldm], l1 = c[ldm], l0 = c[0];
+      const float4 z = B.backward(shfl4(v, p));
+      v = lane < p ? fmaf(-l0, z.x, fmaf(-l1, z.y, fmaf(-l2, z.z, fmaf(-l3, z.w, v)))) : lane < p + 4 ? pick(z, lane - p) : v;
     }
     if (lane < nv) g.qacc[lane * cap + w] = qa[lane] + v;
     if (lane == 0) {
