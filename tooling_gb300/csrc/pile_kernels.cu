@@ -1130,7 +1130,7 @@ extern "C" void pile_k_collide_launch(const PileGroupDev* dG, const int* dwseg, 
   il.stats = 0;
   il.counts = lists + (size_t)N_ICLASS * total_slots;
   cudaMemsetAsync(il.counts, 0, (N_COUNTERS + 3) * sizeof(int), st);
-  // few worlds: a block each, spread over more SMs (250 worlds of 10 boxes: 52 us in 63 blocks, 40 in 250)
+  // few worlds: a block each, spread over more SMs (250 worlds of 10 boxes: 52 us in 63 blocks, 43 in 250)
   const int wpb = total_worlds <= 2048 ? 1 : 4;
   pile_k_collide<<<(total_worlds + wpb - 1) / wpb, 32 * wpb, 0, st>>>(dG, dwseg, ng, total_worlds, il);
 }

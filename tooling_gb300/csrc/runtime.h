@@ -209,7 +209,7 @@ struct newt_gpu_ctx {
   // per-world state I/O staging (pinned host + device, same size)
   void* io_h = nullptr;
   void* io_d = nullptr;
-  size_t io_bytes = 0;
+  size_t io_bytes = 0, io_d_bytes = 0;
   // control streams: per world a horizon x nv block of the device arena and
   // a cursor; `ctrl_of_slot` maps a slot to its entry (-1: none)
   struct CtrlEntry { int slot, nv, h, t; size_t off; };

@@ -60,20 +60,27 @@ int grid_for(long total) {
   return (int)std::max<long>(1, std::min<long>(b, 152L * 16));
 }
 
-// staging: [idx ints | floats], both for every segment of the call
-int ensure_staging(newt_gpu_ctx* ctx, size_t n_idx, size_t n_f) {
+// staging: [idx ints | floats], both for every segment of the call; the
+// device's half where a call copies into it
+int ensure_staging(newt_gpu_ctx* ctx, size_t n_idx, size_t n_f, bool device = true) {
   const size_t bytes = ((n_idx * sizeof(int) + 255) & ~(size_t)255) + n_f * sizeof(float);
-  if (bytes <= ctx->io_bytes) return NEWT_OK;
-  size_t want = std::max<size_t>(bytes, 2 * ctx->io_bytes);
-  want = std::max<size_t>(want, 1 << 20);
-  if (ctx->io_h) cudaFreeHost(ctx->io_h);
-  if (ctx->io_d) cudaFree(ctx->io_d);
-  ctx->io_h = nullptr;
-  ctx->io_d = nullptr;
-  ctx->io_bytes = 0;
-  CKW(cudaMallocHost(&ctx->io_h, want));
-  CKW(cudaMalloc(&ctx->io_d, want));
-  ctx->io_bytes = want;
+  auto grown = [&](size_t held) { return std::max<size_t>(std::max<size_t>(bytes, 2 * held), 1 << 20); };
+  if (bytes > ctx->io_bytes) {
+    const size_t want = grown(ctx->io_bytes);
+    if (ctx->io_h) cudaFreeHost(ctx->io_h);
+    ctx->io_h = nullptr;
+    ctx->io_bytes = 0;
+    CKW(cudaMallocHost(&ctx->io_h, want));
+    ctx->io_bytes = want;
+  }
+  if (device && bytes > ctx->io_d_bytes) {
+    const size_t want = grown(ctx->io_d_bytes);
+    if (ctx->io_d) cudaFree(ctx->io_d);
+    ctx->io_d = nullptr;
+    ctx->io_d_bytes = 0;
+    CKW(cudaMalloc(&ctx->io_d, want));
+    ctx->io_d_bytes = want;
+  }
   return NEWT_OK;
 }
 
@@ -519,7 +526,7 @@ int view_arrays(newt_gpu_ctx* ctx, const StatePlan& P, const void* qpos, const v
   w.vo = table + (w.q_staged ? up256(nq * sizeof(float)) : 0);
   const size_t bytes = w.vo + (w.v_staged ? nv * sizeof(float) : 0);
   if (bytes > 0) {
-    const int rc = ensure_staging(ctx, 0, bytes / sizeof(float) + 1);
+    const int rc = ensure_staging(ctx, 0, bytes / sizeof(float) + 1, table > 0);
     if (rc != NEWT_OK) return rc;
   }
   if (w.q_staged) w.q = device_view((char*)ctx->io_h + w.qo, nq);
