@@ -5,9 +5,9 @@ Workload (the metric's headline configuration): 8192 independent worlds, each
 friction, PGS 50 iterations, dt = 2e-3 -- seeded synthetic worlds.
 
 A bench step advances every world by `--substeps` env-steps with one call of
-the C ABI's batched step (one CUDA-graph replay of one world-persistent
-launch: a warp per world runs collide, PGS and integration for every
-env-step of the call, worlds pulled from a queue).  The same line carries the
+the C ABI's batched step (one CUDA-graph replay of two launches per env-step:
+contacts and row constants, then PGS sweeps and integration, worlds from a
+cost-sorted queue).  The same line carries the
 plain form (one launch per stage per env-step) on the same worlds and horizon,
 the one-step error against the FP64 oracle on a sample of the timed region's
 start state, and two compact runs of the other metric configurations: the
@@ -49,11 +49,12 @@ FP32_PEAK_TFLOPS = 152 * 128 * 2 * 2.07e9 / 1e12
 # newt/src/solver.rs:1448-1518 with the residuals of :1980 and the impulse
 # application of :2022)
 PGS_FLOP_PER_CONTACT_SWEEP = 5 * 235
-# DRAM bytes (read + write) per world and env-step of pile_k_fused, from the
-# ncu capture summarised in profiles/pile_k_fused_2048worlds_settled_full.md
-# (2048 settled worlds, one launch of 25 env-steps: 28.8 MB read + 272.5 MB
-# written), scaled by worlds x env-steps
-FUSED_DRAM_BYTES_PER_WORLD_STEP = (28.797696e6 + 272.532224e6) / (2048 * 25)
+# DRAM bytes (read + write) per world and env-step of pile_k_contacts and
+# pile_k_sweep, from the ncu captures summarised in
+# profiles/batched_kernels_sections.md (8192 settled worlds, one env-step:
+# 39.0 MB read + 40.3 MB written, 75.7 MB read + 1.8 MB written), scaled by
+# worlds x env-steps
+BATCHED_DRAM_BYTES_PER_WORLD_STEP = (39.012608e6 + 40.318208e6 + 75.677952e6 + 1.83552e6) / 8192
 
 
 def pinned_like(a):
@@ -202,8 +203,8 @@ def pile_kernel_bytes(kernel: str, n_worlds: int, nb: int, work: dict) -> float:
     return 4.0 * (int(contacts[c]) * (ROW_WORDS + 4) + int(bodies[c]) * 6)
 
 
-def fused_kernel_bytes(n_worlds: int, nb: int, contacts_last_step: float) -> float:
-    """Algorithmic HBM bytes of one pile_k_fused launch: every world record
+def batched_kernel_bytes(n_worlds: int, nb: int, contacts_last_step: float) -> float:
+    """Algorithmic HBM bytes of one call's pile launches: every world record
     read once (per body: position, velocity, angular velocity, size, geom
     offset 3 each; orientation, geom orientation 4 each; inverse and body
     inertia 6 each; mass, shape; per geom friction, margin, filter; plane 7,
@@ -262,7 +263,7 @@ def run_gpu(args, rank, ws, local, dist):
     eng.set_state(slots, batch.qpos, batch.qvel)
     S = args.substeps
     nq_t, nv_t = int(batch.nq.sum()), int(batch.nv.sum())
-    # the persistent launch's timing events ride in the captured graph
+    # the batched launches' timing events ride in the captured graph
     eng.pile_profile(1)
     # warm-up (also captures the CUDA graph), then the launch-choice autotuner
     # (it leaves the worlds' state as it found it)
@@ -339,20 +340,20 @@ def run_gpu(args, rank, ws, local, dist):
     nb = int(batch.n_bodies[0])
     persistent = fwork["worlds"] > 0
     if persistent:
-        # the world-persistent kernel: FP32 work of newt's PGS over the
-        # contacts it solved, per launch, against the FP32 pipe's peak
-        dom, dom_ms = "pile_k_fused", fused_ms / args.steps
+        # the batched launches: FP32 work of newt's PGS over the contacts
+        # they solved, per call, against the FP32 pipe's peak
+        dom, dom_ms = "pile_k_contacts + pile_k_sweep", fused_ms / args.steps
         flops = PGS_FLOP_PER_CONTACT_SWEEP * 50 * fwork["contacts"] / args.steps
         achieved = flops / (dom_ms / 1e3) / 1e12 if dom_ms > 0 else None
         contacts_last = fwork["contacts"] / (args.steps * S)
-        alg = fused_kernel_bytes(W, nb, contacts_last)
+        alg = batched_kernel_bytes(W, nb, contacts_last)
         hbm_ach = alg / (dom_ms / 1e3) / 1e9 if dom_ms > 0 else None
-        traffic = (FUSED_DRAM_BYTES_PER_WORLD_STEP * W * S) if FUSED_DRAM_BYTES_PER_WORLD_STEP else None
+        traffic = BATCHED_DRAM_BYTES_PER_WORLD_STEP * W * S
         roof = {"bound": "fp32", "kernel": dom, "achieved": achieved, "peak": FP32_PEAK_TFLOPS, "unit": "TFLOP/s",
                 "frac": achieved / FP32_PEAK_TFLOPS if achieved else None, "traffic": traffic,
-                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one settled 2048-world "
-                                  "launch (profiles/pile_k_fused_2048worlds_settled_full.md), per world-step, "
-                                  "scaled to this launch's worlds x env-steps",
+                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one env-step of 8192 "
+                                  "settled worlds (profiles/batched_kernels_sections.md), per world-step, "
+                                  "scaled to this call's worlds x env-steps",
                 "peak_source": "derived from datasheet figures (152 SMs x 128 FP32 lanes x 2 x 2.07 GHz); "
                                "MEASURED_PEAKS.json has no FP32 figure",
                 "flop_per_launch": flops, "flop_formula": "5 x 235 FLOP x 50 sweeps per active contact and env-step "
@@ -361,11 +362,11 @@ def run_gpu(args, rank, ws, local, dist):
                 "dependency_rounds_per_world_sweep": fwork["rounds"] / (50.0 * W * S * args.steps),
                 "hbm": {"achieved": hbm_ach, "peak": hbm, "unit": "GB/s", "frac": hbm_ach / hbm if hbm_ach else None,
                         "peak_source": src, "algorithmic_bytes_per_launch": alg},
-                "note": "one launch per bench step (all worlds, all env-steps), timed live by an event pair on its "
-                        "stream inside the graph"}
-        kernels = {"pile_k_fused": {"ms_per_launch": dom_ms, "share": 1.0, "algorithmic_bytes": alg}}
-        mode = ("batched: one world-persistent launch per bench step (a warp per world for all its env-steps, "
-                "worlds from a size-sorted queue), CUDA graph")
+                "note": "two launches per env-step (all worlds), all env-steps of a bench step timed live by an event "
+                        "pair on their stream inside the graph"}
+        kernels = {dom: {"ms_per_launch": dom_ms, "share": 1.0, "algorithmic_bytes": alg}}
+        mode = ("batched: two launches per env-step (contacts; sweeps and integration), worlds from a cost-sorted "
+                "queue, CUDA graph")
     else:
         branches = n_launch / (args.steps * S)
         dom = max(kernel_ms, key=kernel_ms.get)
