@@ -53,7 +53,7 @@
 //
 // Measured (GB300, us an env-step, one warp per world for the whole horizon
 // before -> now): ten worlds of 16 bodies 206 -> 88, 8192 of 16 bodies
-// 1100 -> 505, 700 of 53 bodies 790 -> 289, 1500 of 12 capsules (RK4)
+// 1100 -> 505, 700 of 53 bodies 790 -> 252, 1500 of 12 capsules (RK4)
 // 196 -> 97.
 #include <algorithm>
 #include <cmath>
@@ -805,8 +805,21 @@ extern "C" cudaError_t newt_pile_batched_plan(int shape, int worlds, int sms, in
   // (the rest of the space, the other worlds' rounds).  Rounds: twice the five
   // of 16 bodies, the nine of 53.
   const int n = 32 / p->lanes;
-  const int rows = std::min(n * cm, (int)(nbm * (1.5f * n + sqrtf((float)n))) + 4 + std::max(0, 16 - nbm));
-  p->space = ROW_V4 * (rows + 1) + 16 * (10 + nbm / 4) * (n > 2 ? 3 : 2) / 2;
+  auto space = [&](float spread) {
+    const int rows = std::min(n * cm, (int)(nbm * (1.5f * n + spread * sqrtf((float)n))) + 4 + std::max(0, 16 - nbm));
+    return ROW_V4 * (rows + 1) + 16 * (10 + nbm / 4) * (n > 2 ? 3 : 2) / 2;
+  };
+  p->space = space(1.f);
+  // One world a block: where a deviation less lets the chip hold all blocks at
+  // once it is given up (700 worlds of 53 bodies, five an SM in place of four,
+  // 289 -> 252 us an env-step).  Two worlds a block lose more by rows past the
+  // space (2500 of 16 bodies, nine an SM: 281 -> 311; 8192 of 16 at half a
+  // deviation less 507 -> 561).
+  if (n == 1) {
+    const int per_sm = (worlds + sms - 1) / sms;
+    const long all = (227 * 1024 / per_sm - 1024 - (long)sweep_smem(p->lanes, nbm, 0)) / 16;
+    if (all >= space(0.6f)) p->space = (int)std::min<long>(p->space, all);
+  }
   while (sweep_smem(p->lanes, nbm, p->space) > kMostSmem) p->space /= 2;
   cudaError_t e = cudaFuncSetAttribute(pile_k_contacts, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostSmem);
   with_sweep(p->lanes, [&](auto kern) {
