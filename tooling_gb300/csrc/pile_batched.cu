@@ -791,7 +791,8 @@ extern "C" int newt_pile_batched_words(const PileGroupDev* g) {
 
 // Plans the launches over `worlds` worlds of at most nbm bodies, cm contacts
 // and `stride` shared words, and sets the kernels' shared-memory limits (outside stream capture).
-extern "C" cudaError_t newt_pile_batched_plan(int shape, int worlds, int sms, int nbm, int cm, int stride,
+// `alone`: no other worlds step beside them.
+extern "C" cudaError_t newt_pile_batched_plan(int shape, int worlds, int sms, int nbm, int cm, int stride, bool alone,
                                               PileBatchedPlan* p) {
   const BatchedShape s = kShapes[shape % kNumShapes];
   p->nbm = nbm;
@@ -801,15 +802,21 @@ extern "C" cudaError_t newt_pile_batched_plan(int shape, int worlds, int sms, in
   while (p->warps > 1 && (size_t)p->warps * p->stride * 4 > kMostSmem / 2) p->warps /= 2;
   if (worlds <= 4 * sms) p->warps = 1;  // a block each: none waits at another's phase barriers
   // Rows: a settled pile has 1.5 active contacts per body, its worlds spread
-  // by 0.4; a block of n worlds takes the mean and two and a half deviations
-  // (the rest of the space, the other worlds' rounds).  Rounds: twice the five
-  // of 16 bodies, the nine of 53.
+  // by 0.4, smaller piles by more; a block of n worlds takes the mean and two
+  // and a half deviations (the rest of the space, the other worlds' rounds),
+  // three and a half where several worlds share a block and the chip, since a
+  // row past the space slows every world of its block.  Rounds: twice the five
+  // of 16 bodies, the nine of 53.  Us an env-step at two and a half deviations
+  // of 0.4 whatever the size -> now: 3000 worlds of 8 boxes 263 -> 186, 4000 of
+  // 12 307 -> 241, 5000 of 14 414 -> 305, 4000 of 16 369 -> 276, 3000 of 18
+  // 418 -> 265, 8192 of 16 505 -> 504; beside larger worlds the wider blocks
+  // took their place (6000 mixed worlds 364 -> 394).
   const int n = 32 / p->lanes;
   auto space = [&](float spread) {
     const int rows = std::min(n * cm, (int)(nbm * (1.5f * n + spread * sqrtf((float)n))) + 4 + std::max(0, 16 - nbm));
     return ROW_V4 * (rows + 1) + 16 * (10 + nbm / 4) * (n > 2 ? 3 : 2) / 2;
   };
-  p->space = space(1.f);
+  p->space = space((alone && n > 1 ? 1.4f : 1.f) + 0.2f * std::max(0, 16 - nbm));
   // One world a block: where a deviation less lets the chip hold all blocks at
   // once it is given up (700 worlds of 53 bodies, five an SM in place of four,
   // 289 -> 252 us an env-step).  Two worlds a block lose more by rows past the

@@ -32,7 +32,7 @@ extern "C" int newt_launch_pile_step(const PileGroupDev* dG, const int* dwseg, i
 extern "C" void newt_pile_init();
 struct PileBatchedPlan { int lanes, warps, stride, space, nbm; };  // pile_batched.cu
 extern "C" int newt_pile_batched_class(int nb);
-extern "C" cudaError_t newt_pile_batched_plan(int shape, int worlds, int sms, int nbm, int cm, int stride,
+extern "C" cudaError_t newt_pile_batched_plan(int shape, int worlds, int sms, int nbm, int cm, int stride, bool alone,
                                               PileBatchedPlan* p);
 extern "C" int newt_pile_batched_words(const PileGroupDev* g);
 extern "C" int newt_launch_pile_batched(const PileGroupDev* dG, const int* dwseg, int ng, int* queue, int n,
@@ -317,6 +317,10 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
     if (!ctx->fused_work) CKS(cudaMalloc(&ctx->fused_work, 4 * sizeof(unsigned long long)));
     if (!ctx->fkev[0])
       for (int k = 0; k < 2; ++k) CKS(cudaEventCreate(&ctx->fkev[k]));
+    bool alone = true;  // one size class of piles, no other worlds
+    for (auto& gp : ctx->groups)
+      alone = alone && (gp->n == 0 || (gp->kind == GK_PILE && !gp->pile_solo() &&
+                                       newt_pile_batched_class(gp->size) == newt_pile_batched_class(piles[0]->size)));
     for (int cls : {2, 1, 0}) {
       std::vector<HostGroup*> gs;
       BatchedLaunch L{};
@@ -332,7 +336,7 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
       if (gs.empty()) continue;
       int rc = build_pile_table(ctx, gs, L.t, bufs, 0, 1);
       if (rc != NEWT_OK) return rc;
-      CKS(newt_pile_batched_plan(ctx->tune_fused_shape, L.t.worlds, sm_count(ctx), nbm, cm, stride, &L.plan));
+      CKS(newt_pile_batched_plan(ctx->tune_fused_shape, L.t.worlds, sm_count(ctx), nbm, cm, stride, alone, &L.plan));
       if (L.t.worlds > 8 * sm_count(ctx)) {  // several waves: the costly worlds first
         CKS(cudaMalloc(&L.queue, sizeof(int) * (size_t)L.t.worlds));
         CKS(cudaMalloc(&L.cost, sizeof(unsigned) * (size_t)L.t.worlds));
