@@ -9,10 +9,13 @@
 // and moves by one strided copy.  The packed order follows the device layout so both sides of each
 // launch are coalesced: tree groups keep fields as rows x cap (packed as
 // rows x k), pile groups keep worlds contiguous (packed as k x rows).
+#include <cuda.h>
+
 #include <algorithm>
 #include <cstring>
 
 #include "common.cuh"
+#include "host_range.h"
 #include "runtime.h"
 
 #define CKW(call)                                                               \
@@ -392,19 +395,37 @@ __global__ void __launch_bounds__(256) state_move_table(const StateRun* R, int n
   move_tile<MOVE>(R, n, qpos, qvel);
 }
 
-// The device's address of n floats of page-locked host memory, or null.
+// The device's address of n floats of page-locked host memory, or null: the
+// kernels read and write the caller's array in place only where one
+// page-locked range holds all of it.
+HostRange host_range(const void* p) {
+  using Get = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+  static const Get get = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<Get>(f);
+  }();
+  cudaPointerAttributes a;
+  if (!get || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return HostRange{};
+  }
+  if (a.type != cudaMemoryTypeHost || !a.devicePointer) return HostRange{};
+  CUdeviceptr start = 0;
+  size_t bytes = 0;
+  CUpointer_attribute what[2] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void* out[2] = {&start, &bytes};
+  if (get(2, what, out, (CUdeviceptr)a.devicePointer) != CUDA_SUCCESS) return HostRange{};
+  return HostRange{(uintptr_t)a.devicePointer, (uintptr_t)start, bytes};
+}
 float* device_view(const void* p, size_t n) {
   if (n == 0 || ((uintptr_t)p & 3)) return nullptr;
-  const char* last = (const char*)p + n * sizeof(float) - 1;
-  cudaPointerAttributes a, b;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaPointerGetAttributes(&b, last) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer || !b.devicePointer ||
-      (const char*)b.devicePointer - (const char*)a.devicePointer != last - (const char*)p)
-    return nullptr;
-  return (float*)a.devicePointer;
+  return reinterpret_cast<float*>(device_address(p, n * sizeof(float), host_range));
 }
 
 size_t up256(size_t b) { return (b + 255) & ~(size_t)255; }
