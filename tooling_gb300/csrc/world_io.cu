@@ -247,7 +247,12 @@ int io_gather(newt_gpu_ctx* ctx, const std::vector<RowMove>& all) {
 // for many.  So
 //   * the worlds are taken as runs of consecutive indices in a group, a few
 //     of which describe most calls and travel as kernel parameters (up to
-//     128; a table in the staging past that);
+//     128; a table in the staging past that); worlds named in no order, fewer
+//     than eight a run, go by a list in the staging instead, a warp each (runs
+//     cost a block and 120 bytes apiece: 16384 quadrupeds shuffled, set_state
+//     444 us as runs of one and 189 by the list, 152 and 119 as runs of four,
+//     118 and 115 as runs of eight; 512 chains, runs of eight 24 and 24);
+//   * a call for forces skips free bodies, which carry none;
 //   * page-locked arrays are read and written by the kernel itself, others
 //     through the page-locked staging;
 //   * a block moves up to 32 worlds of a run by way of shared memory, so that
@@ -361,9 +366,8 @@ NEWT_D void move_tile(const StateRun* runs, int n, float* qpos, float* qvel) {
     __syncthreads();
   }
   if (MOVE == QFRC_IN) {
-    if (g.soa)  // free bodies carry no generalised force
-      for (int e = tid; e < 32 * nv; e += nt)
-        if ((e & 31) < T) frow(g, g.rf + (e >> 5), w0 + (e & 31)) = sv[(e & 31) * nv + (e >> 5)];
+    for (int e = tid; e < 32 * nv; e += nt)  // of trees alone
+      if ((e & 31) < T) frow(g, g.rf + (e >> 5), w0 + (e & 31)) = sv[(e & 31) * nv + (e >> 5)];
     return;
   }
   if (g.soa) {  // worlds side by side (a tile of at most 32)
@@ -384,6 +388,40 @@ NEWT_D void move_tile(const StateRun* runs, int n, float* qpos, float* qvel) {
     __syncthreads();
     for (int e = tid; e < T * nq; e += nt) q[e] = sq[e];
     for (int e = tid; e < T * nv; e += nt) v[e] = sv[e];
+  }
+}
+// A world of a call that names them in no order: its group's entry, its index,
+// its first coordinate and rate in the caller's arrays.
+struct StateWorld { int g, w; long q0, v0; };
+constexpr int LIST_WARPS = 8, LIST_RUN = 8;
+// A warp per listed world, by way of `per` floats of shared memory each.
+template <int MOVE>
+__global__ void __launch_bounds__(32 * LIST_WARPS) state_move_list(const StateRun* G, const StateWorld* W, int n, int per,
+                                                                   float* qpos, float* qvel) {
+  extern __shared__ float tile_s[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = blockIdx.x * LIST_WARPS + warp;
+  if (t >= n) return;
+  const StateWorld sw = W[t];
+  const StateRun& g = G[sw.g];
+  const int nq = g.nq, nv = g.nv, w = sw.w;
+  float* q = qpos + sw.q0;
+  float* v = qvel + sw.v0;
+  if (MOVE == QFRC_IN) {
+    for (int k = lane; k < nv; k += 32) frow(g, g.rf + k, w) = v[k];
+    return;
+  }
+  float* sq = tile_s + warp * per;
+  float* sv = sq + nq;
+  if (MOVE == STATE_IN) {
+    for (int k = lane; k < nq; k += 32) sq[k] = q[k];
+    for (int k = lane; k < nv; k += 32) sv[k] = v[k];
+    __syncwarp();
+    for (int i = lane; i < g.size; i += 32) state_in(g, i, w, sq, sv);
+  } else {
+    for (int i = lane; i < g.size; i += 32) state_out(g, i, w, sq, sv);
+    __syncwarp();
+    for (int k = lane; k < nq; k += 32) q[k] = sq[k];
+    for (int k = lane; k < nv; k += 32) v[k] = sv[k];
   }
 }
 template <int MOVE, int N>
@@ -430,17 +468,26 @@ float* device_view(const void* p, size_t n) {
 
 size_t up256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// The call's worlds as runs.  Slots are named in ascending order when none
-// can be named twice.
+// The call's worlds as runs of consecutive indices in a group.  Slots are
+// named in ascending order when none can be named twice.
+struct Run { int group, w0, n, nq, nv; long q0, v0; };
 struct StatePlan {
-  std::vector<StateRun> runs;
+  std::vector<Run> runs;
   long nq = 0, nv = 0;
+  int worlds = 0;
   bool ascending = true;
+  // Worlds in no order (a run for every few of them) move by a list, a warp
+  // each; see state_move_list.
+  bool listed() const { return runs.size() > 128 && runs.size() * LIST_RUN > (size_t)worlds; }
 };
-int plan_state(newt_gpu_ctx* ctx, const int32_t* slots, int n, StatePlan& P) {
+// `forces`: only the worlds that carry generalised forces.  `skip` (nullable):
+// a flag per named slot, those to pass over.
+int plan_state(newt_gpu_ctx* ctx, const int32_t* slots, int n, bool forces, const char* skip, StatePlan& P) {
   const int n_slots = (int)ctx->slots.size();
   const SlotRef* refs = ctx->slots.data();
   int group = -1, next = -1, prev = -1, nq = 0, nv = 0;
+  bool moves = true, open = false;  // the group's worlds move; the last run takes its next one
+  Run run{};
   for (int i = 0; i < n; ++i) {
     const int s = slots[i];
     if (s < 0 || s >= n_slots || !refs[s].live) {
@@ -449,35 +496,56 @@ int plan_state(newt_gpu_ctx* ctx, const int32_t* slots, int n, StatePlan& P) {
     }
     P.ascending = P.ascending && s > prev;
     prev = s;
-    if (refs[s].group != group || refs[s].index != next) {
+    if (refs[s].group != group) {
       group = refs[s].group;
       const HostGroup& hg = *ctx->groups[group];
-      const HostModel& m = ctx->models[refs[s].model];  // a group's models have one layout
-      nq = m.nq;
-      nv = m.nv;
-      StateRun g{};
-      g.F = hg.dF;
-      g.topo = hg.dtopo;
-      g.frows = (long)hg.frows;
-      g.q0 = P.nq;
-      g.v0 = P.nv;
-      g.soa = hg.soa() ? 1 : 0;
-      g.cap = hg.cap;
-      g.size = hg.size;
-      g.nq = nq;
-      g.nv = nv;
-      g.pos = hg.lay.pos; g.quat = hg.lay.quat; g.vel = hg.lay.vel; g.omg = hg.lay.omg;
-      g.rq = hg.r_q; g.rqd = hg.r_qd; g.rf = hg.r_qfrc;
-      g.w0 = refs[s].index;
-      P.runs.push_back(g);
-      next = g.w0;
+      nq = hg.nq;
+      nv = hg.nv;
+      moves = !forces || hg.soa();
+      next = -1;
     }
-    ++P.runs.back().n;
-    ++next;
+    if (!moves || (skip && skip[i])) {
+      next = -1;
+    } else {
+      if (refs[s].index != next) {
+        if (open) {
+          if (P.runs.size() == 128) P.runs.reserve(n);  // they keep coming
+          P.runs.push_back(run);
+        }
+        open = true;
+        run = Run{group, refs[s].index, 0, nq, nv, P.nq, P.nv};
+        next = run.w0;
+      }
+      ++run.n;
+      ++next;
+      ++P.worlds;
+    }
     P.nq += nq;
     P.nv += nv;
   }
+  if (open) P.runs.push_back(run);
   return NEWT_OK;
+}
+
+// What the kernels take of a run.
+StateRun describe(newt_gpu_ctx* ctx, const Run& r) {
+  const HostGroup& hg = *ctx->groups[r.group];
+  StateRun g{};
+  g.F = hg.dF;
+  g.topo = hg.dtopo;
+  g.frows = (long)hg.frows;
+  g.soa = hg.soa() ? 1 : 0;
+  g.cap = hg.cap;
+  g.size = hg.size;
+  g.nq = r.nq;
+  g.nv = r.nv;
+  g.q0 = r.q0;
+  g.v0 = r.v0;
+  g.w0 = r.w0;
+  g.n = r.n;
+  g.pos = hg.lay.pos; g.quat = hg.lay.quat; g.vel = hg.lay.vel; g.omg = hg.lay.omg;
+  g.rq = hg.r_q; g.rqd = hg.r_qd; g.rf = hg.r_qfrc;
+  return g;
 }
 
 template <int MOVE, int N>
@@ -488,35 +556,65 @@ void launch_runs(const StateRun* runs, int n, int blocks, size_t smem, float* q,
   state_move<MOVE, N><<<blocks, 256, smem, st>>>(R, q, v);
 }
 
-// Moves the planned runs [first, first + count) between the rows and the
-// arrays at device addresses q and v; `table`: room for the runs in the
-// staging (host and device), used past 128.
+// Bytes of the staging's head (host and device) that the move takes.
+size_t table_bytes(newt_gpu_ctx* ctx, const StatePlan& P) {
+  if (P.listed()) return up256(ctx->groups.size() * sizeof(StateRun)) + up256(P.worlds * sizeof(StateWorld));
+  return P.runs.size() > 128 ? up256(P.runs.size() * sizeof(StateRun)) : 0;
+}
+
+// Moves the planned worlds between the rows and the arrays at device
+// addresses q and v.
 template <int MOVE>
-int move_runs(newt_gpu_ctx* ctx, StatePlan& P, size_t first, size_t count, float* q, float* v, size_t table) {
-  int blocks = 0;
-  size_t smem = 0;
-  StateRun* runs = P.runs.data() + first;
-  for (size_t k = 0; k < count; ++k) {
-    StateRun& g = runs[k];
-    const int per = std::max(1, (MOVE == QFRC_IN ? 0 : g.nq) + g.nv);
-    g.tile = std::min(32, std::max(1, TILE_FLOATS / per));
-    g.blk = blocks;
-    blocks += (g.n + g.tile - 1) / g.tile;
-    smem = std::max(smem, (size_t)g.tile * per * sizeof(float));
-  }
-  if (blocks == 0) return NEWT_OK;
-  if (count <= 2) {
-    launch_runs<MOVE, 2>(runs, (int)count, blocks, smem, q, v, ctx->stream);
-  } else if (count <= 24) {
-    launch_runs<MOVE, 24>(runs, (int)count, blocks, smem, q, v, ctx->stream);
-  } else if (count <= 128) {
-    launch_runs<MOVE, 128>(runs, (int)count, blocks, smem, q, v, ctx->stream);
+int move_worlds(newt_gpu_ctx* ctx, const StatePlan& P, float* q, float* v) {
+  if (P.worlds == 0) return NEWT_OK;
+  char* h = (char*)ctx->io_h;
+  char* d = (char*)ctx->io_d;
+  if (P.listed()) {
+    const size_t head = up256(ctx->groups.size() * sizeof(StateRun));
+    StateRun* hg = (StateRun*)h;
+    StateWorld* hw = (StateWorld*)(h + head);
+    std::vector<int> entry(ctx->groups.size(), -1);
+    int groups = 0, per = 1;
+    for (const Run& r : P.runs) {
+      if (entry[r.group] < 0) {
+        hg[groups] = describe(ctx, r);
+        per = std::max(per, r.nq + r.nv);
+        entry[r.group] = groups++;
+      }
+      for (int k = 0; k < r.n; ++k) *hw++ = StateWorld{entry[r.group], r.w0 + k, r.q0 + (long)k * r.nq, r.v0 + (long)k * r.nv};
+    }
+    CKW(cudaMemcpyAsync(d, h, groups * sizeof(StateRun), cudaMemcpyHostToDevice, ctx->stream));
+    // the list is read once, where it lies
+    const StateWorld* dw = (const StateWorld*)device_view(h + head, P.worlds * sizeof(StateWorld) / sizeof(float));
+    state_move_list<MOVE><<<(P.worlds + LIST_WARPS - 1) / LIST_WARPS, 32 * LIST_WARPS,
+                            MOVE == QFRC_IN ? 0 : LIST_WARPS * per * sizeof(float), ctx->stream>>>(
+        (const StateRun*)d, dw, P.worlds, per, q, v);
   } else {
-    StateRun* h = (StateRun*)((char*)ctx->io_h + table);
-    StateRun* d = (StateRun*)((char*)ctx->io_d + table);
-    std::copy(runs, runs + count, h);
-    CKW(cudaMemcpyAsync(d, h, count * sizeof(StateRun), cudaMemcpyHostToDevice, ctx->stream));
-    state_move_table<MOVE><<<blocks, 256, smem, ctx->stream>>>(d, (int)count, q, v);
+    std::vector<StateRun> runs;
+    runs.reserve(P.runs.size());
+    int blocks = 0;
+    size_t smem = 0;
+    for (const Run& r : P.runs) {
+      StateRun g = describe(ctx, r);
+      const int per = std::max(1, (MOVE == QFRC_IN ? 0 : g.nq) + g.nv);
+      g.tile = std::min(32, std::max(1, TILE_FLOATS / per));
+      g.blk = blocks;
+      blocks += (g.n + g.tile - 1) / g.tile;
+      smem = std::max(smem, (size_t)g.tile * per * sizeof(float));
+      runs.push_back(g);
+    }
+    const int n = (int)runs.size();
+    if (n <= 2) {
+      launch_runs<MOVE, 2>(runs.data(), n, blocks, smem, q, v, ctx->stream);
+    } else if (n <= 24) {
+      launch_runs<MOVE, 24>(runs.data(), n, blocks, smem, q, v, ctx->stream);
+    } else if (n <= 128) {
+      launch_runs<MOVE, 128>(runs.data(), n, blocks, smem, q, v, ctx->stream);
+    } else {
+      std::copy(runs.begin(), runs.end(), (StateRun*)h);
+      CKW(cudaMemcpyAsync(d, h, n * sizeof(StateRun), cudaMemcpyHostToDevice, ctx->stream));
+      state_move_table<MOVE><<<blocks, 256, smem, ctx->stream>>>((const StateRun*)d, n, q, v);
+    }
   }
   ctx->launches++;
   CKW(cudaGetLastError());
@@ -537,7 +635,7 @@ bool repeats(newt_gpu_ctx* ctx, const int32_t* slots, int n) {
 // by the staging, past the run table.
 struct Views { float *q = nullptr, *v = nullptr; bool q_staged = false, v_staged = false; size_t qo = 0, vo = 0; };
 int view_arrays(newt_gpu_ctx* ctx, const StatePlan& P, const void* qpos, const void* qvel, Views& w) {
-  const size_t table = P.runs.size() > 128 ? up256(P.runs.size() * sizeof(StateRun)) : 0;
+  const size_t table = table_bytes(ctx, P);
   const size_t nq = qpos ? (size_t)P.nq : 0, nv = (size_t)P.nv;
   w.q = device_view(qpos, nq);
   w.v = device_view(qvel, nv);
@@ -559,7 +657,7 @@ int view_arrays(newt_gpu_ctx* ctx, const StatePlan& P, const void* qpos, const v
 
 int io_state_in(newt_gpu_ctx* ctx, const int32_t* slots, int n, const float* qpos, const float* qvel) {
   StatePlan P;
-  int rc = plan_state(ctx, slots, n, P);
+  int rc = plan_state(ctx, slots, n, false, nullptr, P);
   if (rc != NEWT_OK) return rc;
   if (!P.ascending && repeats(ctx, slots, n)) {
     ctx->err = "slot named twice";
@@ -569,18 +667,18 @@ int io_state_in(newt_gpu_ctx* ctx, const int32_t* slots, int n, const float* qpo
   if ((rc = view_arrays(ctx, P, qpos, qvel, w)) != NEWT_OK) return rc;
   if (w.q_staged) std::memcpy((char*)ctx->io_h + w.qo, qpos, P.nq * sizeof(float));
   if (w.v_staged) std::memcpy((char*)ctx->io_h + w.vo, qvel, P.nv * sizeof(float));
-  if ((rc = move_runs<STATE_IN>(ctx, P, 0, P.runs.size(), w.q, w.v, 0)) != NEWT_OK) return rc;
+  if ((rc = move_worlds<STATE_IN>(ctx, P, w.q, w.v)) != NEWT_OK) return rc;
   CKW(cudaStreamSynchronize(ctx->stream));  // the caller's arrays and the staging are free again
   return NEWT_OK;
 }
 
 int io_state_out(newt_gpu_ctx* ctx, const int32_t* slots, int n, float* qpos, float* qvel) {
   StatePlan P;
-  int rc = plan_state(ctx, slots, n, P);
+  int rc = plan_state(ctx, slots, n, false, nullptr, P);
   if (rc != NEWT_OK) return rc;
   Views w;
   if ((rc = view_arrays(ctx, P, qpos, qvel, w)) != NEWT_OK) return rc;
-  if ((rc = move_runs<STATE_OUT>(ctx, P, 0, P.runs.size(), w.q, w.v, 0)) != NEWT_OK) return rc;
+  if ((rc = move_worlds<STATE_OUT>(ctx, P, w.q, w.v)) != NEWT_OK) return rc;
   CKW(cudaStreamSynchronize(ctx->stream));
   if (w.q_staged) std::memcpy(qpos, (char*)ctx->io_h + w.qo, P.nq * sizeof(float));
   if (w.v_staged) std::memcpy(qvel, (char*)ctx->io_h + w.vo, P.nv * sizeof(float));
@@ -589,18 +687,31 @@ int io_state_out(newt_gpu_ctx* ctx, const int32_t* slots, int n, float* qpos, fl
 
 int io_qfrc_in(newt_gpu_ctx* ctx, const int32_t* slots, int n, const float* qfrc) {
   StatePlan P;
-  int rc = plan_state(ctx, slots, n, P);
+  int rc = plan_state(ctx, slots, n, true, nullptr, P);
   if (rc != NEWT_OK) return rc;
-  Views w;
-  if ((rc = view_arrays(ctx, P, nullptr, qfrc, w)) != NEWT_OK) return rc;
-  if (w.v_staged) std::memcpy((char*)ctx->io_h + w.vo, qfrc, P.nv * sizeof(float));
-  if (P.ascending || !repeats(ctx, slots, n)) {
-    rc = move_runs<QFRC_IN>(ctx, P, 0, P.runs.size(), nullptr, w.v, 0);
-  } else {  // a slot named twice keeps the last forces: the runs in order
-    for (size_t k = 0; k < P.runs.size() && rc == NEWT_OK; ++k)
-      rc = move_runs<QFRC_IN>(ctx, P, k, 1, nullptr, w.v, 0);
+  if (!P.ascending && repeats(ctx, slots, n)) {  // a slot named twice keeps the last forces
+    std::vector<char> seen(ctx->slots.size(), 0), skip(n, 0);
+    for (int i = n - 1; i >= 0; --i) {
+      skip[i] = seen[slots[i]];
+      seen[slots[i]] = 1;
+    }
+    P = StatePlan{};
+    if ((rc = plan_state(ctx, slots, n, true, skip.data(), P)) != NEWT_OK) return rc;
   }
-  if (rc != NEWT_OK) return rc;
+  if (P.worlds > 0) {  // free bodies alone carry no generalised force
+    Views w;
+    if ((rc = view_arrays(ctx, P, nullptr, qfrc, w)) != NEWT_OK) return rc;
+    if (w.v_staged) {
+      float* h = (float*)((char*)ctx->io_h + w.vo);
+      for (size_t k = 0; k < P.runs.size();) {  // what is moved, in runs that follow one another
+        const long a = P.runs[k].v0;
+        long b = a;
+        for (; k < P.runs.size() && P.runs[k].v0 == b; ++k) b += (long)P.runs[k].n * P.runs[k].nv;
+        std::memcpy(h + a, qfrc + a, (size_t)(b - a) * sizeof(float));
+      }
+    }
+    if ((rc = move_worlds<QFRC_IN>(ctx, P, nullptr, w.v)) != NEWT_OK) return rc;
+  }
   CKW(cudaStreamSynchronize(ctx->stream));
   return NEWT_OK;
 }
