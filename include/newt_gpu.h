@@ -196,7 +196,7 @@ NEWT_API int newt_gpu_set_qfrc(newt_gpu_ctx* ctx, const int32_t* slots, int32_t 
  *   over a cost-sorted queue; pile worlds of every size run two launches per
  *   env-step and size class (contacts, then sweeps and integration, over a
  *   queue sorted by the previous call's cost, most costly first), each class
- *   on a branch of the graph; tree-contact worlds run their three kernels per env-step on a
+ *   on a branch of the graph; tree-contact worlds run three or four kernels per env-step on a
  *   branch of the graph.  newt_gpu_autotune may instead pick the
  *   island-class pipeline for piles (collide, island-class solvers on forked
  *   streams, integrate, per env-step).  Pile worlds under the Newton solver

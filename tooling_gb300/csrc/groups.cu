@@ -535,7 +535,8 @@ void HostGroup::release() {
   if (dgtopo) cudaFree(dgtopo);
   if (dpairs) cudaFree(dpairs);
   if (plain_scratch) cudaFree(plain_scratch);
-  dF = nullptr; dI = nullptr; dtopo = nullptr; dgtopo = nullptr; dpairs = nullptr; plain_scratch = nullptr;
+  if (tc_list) cudaFree(tc_list);
+  dF = nullptr; dI = nullptr; dtopo = nullptr; dgtopo = nullptr; dpairs = nullptr; plain_scratch = nullptr; tc_list = nullptr;
 }
 
 TreeGroupDev HostGroup::tree_dev() const {
@@ -548,7 +549,7 @@ TreeGroupDev HostGroup::tree_dev() const {
   d.solver = dI + (size_t)ri_solver * cap;
   d.live = dI + (size_t)ri_live * cap;
   d.integ = ri_integ >= 0 ? dI + (size_t)ri_integ * cap : nullptr;
-  d.cfrc = nullptr; d.cstride = 0;
+  d.cfrc = nullptr; d.cstride = 0; d.zero = nullptr;
   d.q = row(r_q); d.qd = row(r_qd); d.qfrc = row(r_qfrc); d.qacc = row(r_qacc);
   d.status = (uint32_t*)(dI + (size_t)ri_status * cap);
   return d;
@@ -575,6 +576,7 @@ TcGroupDev HostGroup::tc_dev() const {
   d.iters = dI + (size_t)ri_iters * cap;
   d.scr = (float*)plain_scratch;
   d.sstride = scr_stride;
+  d.list = tc_list;
   d.sens = nullptr;
   d.sens_stride = 0;
   return d;

@@ -37,6 +37,7 @@ struct TreeGroupDev {
   const int* integ;    // 1    NEWT_INTEGRATOR_* (null: Euler for every world)
   float* cfrc;         // tree-contact groups: the contact solve's J^T f / dt (nv per world, stride
   long cstride;        // `cstride` floats, in the solver scratch); null for trees without geoms
+  int* zero;           // tree-contact groups: two counters that the integration sets to zero; null otherwise
   // per-world state (SoA)
   float* q;     // nq  (newt layout: free root p xyz, quat xyzw; hinge angle)
   float* qd;    // nv  (free root: omega_body, v_body; hinge rate)
@@ -71,6 +72,8 @@ struct TcGroupDev {
   const int* iters;  // per world
   float* scr;        // world-major solver scratch
   long sstride;      // floats per world in `scr`
+  int* list;         // how many worlds have more than 32 rows, how many of them are taken (both zero
+                     // between env-steps), then the worlds
   // the contact sensors' re-solve (null in a step): the last step's contacts
   // solved again at the current state; per world (stride `sens_stride`)
   // each link's contact wrench (world force, torque about its COM), then per

@@ -1037,24 +1037,50 @@ NEWT_D void tc_rows_solve(const TcGroupDev& G, int w, float* sv, int nr, int nco
 
 }  // namespace
 
-// ---------------------------------------------------------------------------
-// One warp per world, every size and cone
-// ---------------------------------------------------------------------------
+namespace {
+
+// One world's solve, every size and cone, one warp; `resolve`: on the last
+// step's contacts.
 template <bool REFINE>
-__global__ void __launch_bounds__(32) tc_k_solve(TcGroupDev G) {
-  extern __shared__ __align__(16) float tcs[];
-  const int lane = threadIdx.x, w = blockIdx.x;
-  if (w >= G.t.n || !G.t.live[w]) return;  // uniform
+NEWT_D void tc_world(const TcGroupDev& G, int w, float* sv, bool resolve, int lane) {
   const TcSmem sm = tc_smem(G.t.L, G.t.nv, G.maxc, G.rpc);
-  float* pose = tcs + sm.pose;
-  int* rcon = reinterpret_cast<int*>(tcs + sm.rmap);
+  float* pose = sv + sm.pose;
+  int* rcon = reinterpret_cast<int*>(sv + sm.rmap);
   uint32_t status = 0;
   int ncon = 0;
-  tc_kinematics(G.t, w, pose, reinterpret_cast<int*>(tcs + sm.vec), nullptr, lane);
-  const bool resolve = G.sens != nullptr;
+  tc_kinematics(G.t, w, pose, reinterpret_cast<int*>(sv + sm.vec), nullptr, lane);
   const PairGeoms first = tc_pair(G, w, resolve ? G.npairs : lane);
   const int nr = tc_contacts(G, w, pose, first, rcon, rcon + sm.ldr, resolve, lane, &ncon, &status);
-  tc_rows_solve<REFINE>(G, w, tcs, nr, ncon, status, lane);
+  tc_rows_solve<REFINE>(G, w, sv, nr, ncon, status, lane);
+}
+
+}  // namespace
+
+// A warp per world of the group, 16 to an SM (a pair's geom rows in flight
+// would take 168 registers and 12 warps: 2000 elliptic quadrupeds 661 us an
+// env-step, 403 with the few registers spilled that 128 leave short).
+template <bool REFINE>
+__global__ void __launch_bounds__(32, 16) tc_k_solve(const __grid_constant__ TcGroupDev G) {
+  extern __shared__ __align__(16) float tcs[];
+  const int w = blockIdx.x;
+  if (w >= G.t.n || !G.t.live[w]) return;  // uniform
+  tc_world<REFINE>(G, w, tcs, G.sens != nullptr, threadIdx.x);
+}
+
+// The worlds that tc_k_small lists, a warp each, from the contacts it found;
+// taken one by one, since their rows and so their times differ (16000 worlds
+// of 20 DoF and 36 to 56 rows in fixed strides 9600 us an env-step, taken 6640).
+__global__ void __launch_bounds__(32, 16) tc_k_listed(const __grid_constant__ TcGroupDev G) {
+  extern __shared__ __align__(16) float tcs[];
+  const int n = G.list[0];
+  for (;;) {
+    int k = 0;
+    if (threadIdx.x == 0) k = n > 0 ? atomicAdd(G.list + 1, 1) : n;
+    k = __shfl_sync(FULL, k, 0);
+    if (k >= n) return;
+    tc_world<false>(G, G.list[2 + k], tcs, true, threadIdx.x);
+    __syncwarp();
+  }
 }
 
 #include "tc_small.cuh"
@@ -1071,13 +1097,22 @@ extern "C" size_t newt_tc_smem_bytes(int L, int nv, int maxc, int rpc) {
 // The launch of a group: tc_k_small for trees of up to REFINE_NV DoF whose
 // rows are facets or normals, else tc_k_solve.  Blocks of tc_k_small hold
 // TCS_WARPS worlds, fewer where their shared memory would not let TCS_BLOCKS
-// blocks share an SM.
-struct TcPlan { bool small; int warps; size_t bytes; };
-static TcPlan tc_plan(int L, int nv, int maxc, int rpc, bool general, bool resolve) {
-  TcPlan p{nv <= REFINE_NV && !general && !resolve, 1, newt_tc_smem_bytes(L, nv, maxc, rpc)};
+// blocks share an SM, and its worlds of more than 32 rows go to tc_k_listed: a
+// block that solved one itself kept its other warps waiting and had what L1
+// the large blocks leave (20000 worlds of 20 DoF, 28 to 36 rows, 5840 us an
+// env-step, listed 3521; a warp per world for all of them 4287).  Up to
+// TCS_FEW worlds an SM a world has a block of its own, which solves any rows
+// and leaves L1 all but its blocks' shared memory: a second launch could not
+// start before the slowest small world is done (128 fallen quadrupeds of up to
+// 84 rows: all in blocks of four 1430 us, listed 990, so 740; a warp per world
+// 850.  2000 worlds of 28 to 36 rows: 688 in blocks of their own, listed 558).
+struct TcPlan { bool small, list; int warps; size_t bytes; };
+static TcPlan tc_plan(int L, int nv, int maxc, int rpc, bool general, bool resolve, bool few) {
+  TcPlan p{nv <= REFINE_NV && !general && !resolve, false, 1, newt_tc_smem_bytes(L, nv, maxc, rpc)};
   if (p.small) {
     const size_t per = (size_t)tcs_smem(L, nv, maxc, rpc).words * sizeof(float);
-    p.warps = TCS_WARPS;
+    p.list = !few;
+    p.warps = few ? 1 : TCS_WARPS;
     while (p.warps > 1 && p.warps * per > 227 * 1024 / TCS_BLOCKS - 1024) p.warps /= 2;
     p.bytes = p.warps * per;
   }
@@ -1094,22 +1129,43 @@ static cudaError_t tc_limit(const void* kernel, size_t bytes) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 static cudaError_t newt_tc_init(int L, int nv, int maxc, int rpc, bool general) {
-  const TcPlan p = tc_plan(L, nv, maxc, rpc, general, false);
+  const TcPlan p = tc_plan(L, nv, maxc, rpc, general, false, false);
   if (p.small) {
-    const cudaError_t e = tc_limit((const void*)tc_k_small, p.bytes);
+    cudaError_t e = tc_limit((const void*)tc_k_small, p.bytes);
+    if (e == cudaSuccess) e = tc_limit((const void*)tc_k_listed, newt_tc_smem_bytes(L, nv, maxc, rpc));
     if (e != cudaSuccess) return e;
   }
   // the contact sensors' re-solve of any group runs tc_k_solve
   return tc_limit(nv > REFINE_NV ? (const void*)tc_k_solve<true> : (const void*)tc_k_solve<false>,
                   newt_tc_smem_bytes(L, nv, maxc, rpc));
 }
-extern "C" void newt_launch_tc_solve(const TcGroupDev& G, cudaStream_t st) {
+// Returns the launches.
+static int newt_launch_tc_solve(const TcGroupDev& G, int sms, cudaStream_t st) {
   const int n = G.t.n;
-  if (n == 0) return;
-  const TcPlan p = tc_plan(G.t.L, G.t.nv, G.maxc, G.rpc, G.general != 0, G.sens != nullptr);
-  if (p.small) tc_k_small<<<(n + p.warps - 1) / p.warps, 32 * p.warps, p.bytes, st>>>(G);
-  else if (G.t.nv > REFINE_NV) tc_k_solve<true><<<n, 32, p.bytes, st>>>(G);
+  if (n == 0) return 0;
+  const TcPlan p = tc_plan(G.t.L, G.t.nv, G.maxc, G.rpc, G.general != 0, G.sens != nullptr, n <= TCS_FEW * sms);
+  if (p.small) {
+    TcGroupDev D = G;
+    if (!p.list) D.list = nullptr;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((n + p.warps - 1) / p.warps);
+    c.blockDim = dim3(32 * p.warps);
+    c.dynamicSmemBytes = p.bytes;
+    c.stream = st;
+    cudaLaunchAttribute a{};
+    a.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    a.val.sharedMemCarveout =
+        (unsigned)std::min<size_t>(100, ((n + sms - 1) / sms * (p.bytes + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024));
+    c.attrs = &a;
+    c.numAttrs = p.list ? 0 : 1;
+    cudaLaunchKernelEx(&c, tc_k_small, D);
+    if (!p.list) return 1;
+    tc_k_listed<<<n < 16 * sms ? n : 16 * sms, 32, newt_tc_smem_bytes(G.t.L, G.t.nv, G.maxc, G.rpc), st>>>(G);
+    return 2;
+  }
+  if (G.t.nv > REFINE_NV) tc_k_solve<true><<<n, 32, p.bytes, st>>>(G);
   else tc_k_solve<false><<<n, 32, p.bytes, st>>>(G);
+  return 1;
 }
 extern "C" void newt_tc_offsets(int L, int nv, int ng, int maxc, int rpc, int* con, int* imp, int* misc) {
   const TcLay t = tc_layout(L, nv, ng, maxc, rpc);
@@ -1144,6 +1200,15 @@ extern "C" int newt_tc_prepare(newt_gpu_ctx* ctx, HostGroup* g, int n_steps) {
     ctx->graph_dirty = true;
   }
   g->scr_stride = (long)(per / sizeof(float));
+  if (g->tc_list_cap < g->cap) {
+    if (g->tc_list) cudaFree(g->tc_list);
+    g->tc_list = nullptr;
+    g->tc_list_cap = 0;
+    CKT(cudaMalloc(&g->tc_list, sizeof(int) * (size_t)(g->cap + 2)));
+    CKT(cudaMemset(g->tc_list, 0, 2 * sizeof(int)));
+    g->tc_list_cap = g->cap;
+    ctx->graph_dirty = true;
+  }
   CKT(newt_tc_init(g->size, g->nv, g->maxc, g->tc_rpc, g->tc_general));
   if (ctx->profile) {
     while (ctx->tcev.size() < (size_t)6 * n_steps) {
@@ -1156,7 +1221,7 @@ extern "C" int newt_tc_prepare(newt_gpu_ctx* ctx, HostGroup* g, int n_steps) {
 }
 
 // n_steps env-steps of one prepared tree-contact group on stream `st`:
-// a_free, the contact solve and the integration, three launches per
+// a_free, the contact solve and the integration, three or four launches per
 // env-step.  With profiling on, every kernel is bracketed by timing events
 // (recorded as external event nodes when `capturing`).
 extern "C" int newt_tc_launch(newt_gpu_ctx* ctx, HostGroup* g, int n_steps, cudaStream_t st, bool capturing) {
@@ -1164,6 +1229,7 @@ extern "C" int newt_tc_launch(newt_gpu_ctx* ctx, HostGroup* g, int n_steps, cuda
   TcGroupDev d = g->tc_dev();
   d.t.cfrc = d.scr + tc_layout(g->size, g->nv, g->ng, g->maxc, g->tc_rpc).qfc;
   d.t.cstride = d.sstride;
+  d.t.zero = d.list;
   const bool timed = ctx->profile && ctx->tcev.size() >= (size_t)6 * n_steps;
   auto mark = [&](int s, int k) {
     if (!timed) return;
@@ -1175,12 +1241,12 @@ extern "C" int newt_tc_launch(newt_gpu_ctx* ctx, HostGroup* g, int n_steps, cuda
     newt_launch_tree_aba(d.t, st);
     mark(s, 1);
     mark(s, 2);
-    newt_launch_tc_solve(d, st);
+    const int solves = newt_launch_tc_solve(d, sm_count(ctx), st);
     mark(s, 3);
     mark(s, 4);
     newt_launch_tree_integrate(d.t, st);
     mark(s, 5);
-    ctx->launches += 3;
+    ctx->launches += 2 + solves;
   }
   return timed ? n_steps : 0;
 }
@@ -1205,8 +1271,7 @@ extern "C" int newt_tc_resolve(newt_gpu_ctx* ctx, HostGroup* g, float* sens, lon
   d.sens = sens;
   d.sens_stride = sens_stride;
   newt_launch_tree_aba(d.t, st);
-  newt_launch_tc_solve(d, st);
-  return 2;
+  return 1 + newt_launch_tc_solve(d, sm_count(ctx), st);
 }
 
 // Floats per world of the re-solve's output for a group of `L` links and

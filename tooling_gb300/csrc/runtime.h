@@ -114,6 +114,8 @@ struct HostGroup {
   void* plain_scratch = nullptr;  // pile solver scratch, cap worlds (both step forms)
   size_t plain_scratch_bytes = 0;
   long scr_stride = 0;             // floats per world in plain_scratch
+  int* tc_list = nullptr;          // tree-contact groups: TcGroupDev::list, room for tc_list_cap worlds
+  int tc_list_cap = 0;
 
   int reserve_indices(newt_gpu_ctx* ctx, int k, std::vector<int>& out);
   int* release_index(int idx);  // host side; returns the world's device live flag
@@ -233,6 +235,7 @@ struct RowMove {
 };
 int io_scatter(newt_gpu_ctx* ctx, const std::vector<RowMove>& mv);  // host mirror -> device
 int io_gather(newt_gpu_ctx* ctx, const std::vector<RowMove>& mv);   // device -> host mirror
+int sm_count(newt_gpu_ctx* ctx);  // of the context's device
 int io_clear_flags(newt_gpu_ctx* ctx, const std::vector<int*>& flags);  // *flag = 0 on the device
 // MuJoCo-layout state of the named worlds in and out, converted on the device
 // (world_io.cu)

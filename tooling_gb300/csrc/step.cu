@@ -56,7 +56,7 @@ static int ensure_pile_streams(newt_gpu_ctx* ctx) {
 extern "C" size_t newt_pile_list_bytes(int slots);
 extern "C" int newt_tc_step(newt_gpu_ctx* ctx, HostGroup* g, int n_steps, int fused);
 
-static int sm_count(newt_gpu_ctx* ctx) {
+int sm_count(newt_gpu_ctx* ctx) {
   static int n = 0;
   if (n == 0) { cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, ctx->device); if (n <= 0) n = 1; }
   return n;

@@ -1,7 +1,8 @@
 // The tree-contact solve of trees of up to 24 DoF whose rows are facets or
 // normals (included by newton_kernels.cu): the same stages as tc_rows_solve,
-// a warp per world and a lane per row, for worlds of up to 32 rows; a world
-// with more takes tc_rows_solve itself.
+// a warp per world and a lane per row, for worlds of up to 32 rows; the
+// worlds with more take tc_rows_solve, in a launch of their own (tc_k_listed)
+// or, where a block is one world, here.
 //
 // What bounds it: instruction supply.  One warp per block with the stages in
 // a straight line (tc_k_solve) waits 6.5 of every 14.4 cycles an instruction
@@ -32,6 +33,7 @@
 
 constexpr int TCS_WARPS = 4;   // worlds (warps) per block
 constexpr int TCS_BLOCKS = 4;  // blocks per SM
+constexpr int TCS_FEW = 8;     // worlds per SM up to which each has a block of its own
 constexpr int TCS_ROWS = 32;  // rows of a world, a lane each
 constexpr int TCS_LDH = 36;   // row stride of H: float4 loads of eight rows meet no bank twice
 
@@ -406,7 +408,8 @@ NEWT_D int small_newton(float* H, int nr, float b, float* xs, int iters, int lan
   return done;
 }
 
-// A world of more rows, and the Newton solve with its FP64 factor, out of line.
+// A world of more rows where the launch lists none, and the Newton solve with
+// its FP64 factor, out of line.
 __device__ __noinline__ void rows_solve_any(const TcGroupDev& G, int w, float* sv, int nr, int ncon, uint32_t status,
                                             int lane) {
   tc_rows_solve<false>(G, w, sv, nr, ncon, status, lane);
@@ -497,10 +500,15 @@ __global__ void __launch_bounds__(32 * TCS_WARPS, TCS_BLOCKS) tc_k_small(const _
   if (live) {
     nr = tc_contacts(G, w, pose, first, rcon, rfac, false, lane, &ncon, &status);
     __syncwarp();
-    if (nr == 0 && lane == 0 && status) atomicOr(g.status + w, status);  // qacc stays a_free
+    if (nr > TCS_ROWS && !G.list) {  // a block of one warp
+      rows_solve_any(G, w, sv, nr, ncon, status, lane);
+      return;
+    }
+    if ((nr == 0 || nr > TCS_ROWS) && lane == 0 && status) atomicOr(g.status + w, status);
+    if (nr > TCS_ROWS && lane == 0) G.list[2 + atomicAdd(G.list, 1)] = w;
   }
-  bool on = nr > 0 && nr <= TCS_ROWS;
-  __syncthreads();
+  bool on = nr > 0 && nr <= TCS_ROWS;  // without rows qacc stays a_free
+  if (!__syncthreads_or(on)) return;
 
   // ---- link COM Jacobians, world inertias and masses, lane per link; M ----
   if (on) {
@@ -725,8 +733,6 @@ __global__ void __launch_bounds__(32 * TCS_WARPS, TCS_BLOCKS) tc_k_small(const _
         done = newton_any(H, hd, nr, wf + lay.H, wf + lay.LH, reinterpret_cast<double*>(wf + lay.LHd), lay.ld, bias,
                           iters, __any_sync(FULL, facet && mu == 0.f), lane, &x, &status);
     }
-  } else if (nr > TCS_ROWS) {
-    rows_solve_any(G, w, sv, nr, ncon, status, lane);
   }
   __syncthreads();
 
