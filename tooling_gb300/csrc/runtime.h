@@ -162,7 +162,7 @@ struct newt_gpu_ctx {
   bool graph_dirty = true;
   std::vector<void*> plan_bufs;  // device queues / group tables the graph reads
   int queue_items = 0;
-  cudaStream_t side[4] = {};     // capture branches of the tree launches, one per size bucket
+  cudaStream_t side[5] = {};     // capture branches of the tree launches, one per size bucket
   cudaStream_t pside[3] = {nullptr, nullptr, nullptr};  // pile island-class branches
   cudaEvent_t pev[4] = {nullptr, nullptr, nullptr, nullptr};
   // batched piles: world-range branches, each with its own main stream, three

@@ -24,6 +24,8 @@
 extern "C" void newt_launch_tree_lanes(const TreeGroupDev* dgroups, const int* dqueue, int n_items, int L, int serial,
                                        int n_steps, int pct, cudaStream_t st);
 extern "C" cudaError_t newt_tree_lanes_prepare();
+extern "C" void newt_launch_tree_threads(const TreeGroupDev* dgroups, const int* dqueue, int n_items, int n_steps,
+                                         cudaStream_t st);
 extern "C" int newt_tree_item_worlds();
 extern "C" size_t newt_pile_ws_bytes(int nb, int np, int maxc);
 extern "C" int newt_launch_pile_step(const PileGroupDev* dG, const int* dwseg, int ng, int total_worlds,
@@ -241,18 +243,36 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
   std::vector<void*> bufs;
   // trees: one launch per size bucket over a cost-sorted queue, each on its
   // own branch (the bucket's largest tree sizes the blocks' shared memory)
-  struct TreeLaunch { int L, serial; TreeGroupDev* dg; int* dq; int items; };
+  struct TreeLaunch { int L, serial; TreeGroupDev* dg; int* dq; int items; bool threads; };
   std::vector<TreeLaunch> tls;
-  const int buckets[4] = {8, 16, 32, 65};
+  // The smallest trees: eight lanes gain too little on a world of two or
+  // three joints where there are worlds enough for a thread each.  Us for ten
+  // env-steps, lanes and threads: fixed base, 2 hinges (3 links), 8000 worlds
+  // 45 and 52, 13000 66 and 57, 40000 157 and 94, 100000 347 and 233; floating
+  // under RK4 202 and 249, 340 and 292, 873 and 523, 2025 and 1559; 3 hinges,
+  // fixed under RK4, 16000 320 and 336, 25000 490 and 446, 40000 760 and 597;
+  // 4 hinges, 100000 560 and 589.  The lines lie past the crossings, since the
+  // threads' recursion (about the joints' anchors) ends 4 to 8% further from
+  // 64 bits.
+  long small = 0, tiny = 0;
+  for (auto& gp : ctx->groups)
+    if (gp->kind == GK_TREE && gp->size <= NEWT_TREE_TINY) (gp->size < NEWT_TREE_TINY ? tiny : small) += gp->n;
+  const bool tiny_many = tiny > 80L * sm_count(ctx), small_many = small > 120L * sm_count(ctx);
+  auto by_threads = [&](int size) {
+    return size < NEWT_TREE_TINY ? tiny_many : size == NEWT_TREE_TINY && small_many;
+  };
+  const int buckets[5] = {NEWT_TREE_TINY, 8, 16, 32, 65};
   for (int bucket : buckets) {
     struct It { int cost, g, base, count; };
     std::vector<It> its;
     std::vector<TreeGroupDev> tg;
-    const int chunk = newt_tree_item_worlds();
+    const bool threads = bucket == NEWT_TREE_TINY;
+    const int chunk = threads ? NEWT_TREE_THREADS : newt_tree_item_worlds();
     int most = 0, serial = 1;
     for (auto& gp : ctx->groups) {
       HostGroup* g = gp.get();
-      if (g->n == 0 || g->kind != GK_TREE || newt_tree_bucket(g->size) != bucket) continue;
+      if (g->n == 0 || g->kind != GK_TREE) continue;
+      if ((by_threads(g->size) ? NEWT_TREE_TINY : newt_tree_bucket(g->size)) != bucket) continue;
       for (int i = 1; i < g->size; ++i) serial &= g->topo[4 * i] == i - 1;
       int gi = (int)tg.size();
       tg.push_back(g->tree_dev());
@@ -263,7 +283,7 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
     std::stable_sort(its.begin(), its.end(), [](const It& a, const It& b) { return a.cost > b.cost; });
     std::vector<int> q;
     for (auto& i : its) { q.push_back(i.g); q.push_back(i.base); q.push_back(i.count); }
-    TreeLaunch L{most, serial, nullptr, nullptr, (int)its.size()};
+    TreeLaunch L{most, serial, nullptr, nullptr, (int)its.size(), threads};
     CKS(newt_tree_lanes_prepare());
     CKS(cudaMalloc(&L.dg, tg.size() * sizeof(TreeGroupDev)));
     CKS(cudaMemcpy(L.dg, tg.data(), tg.size() * sizeof(TreeGroupDev), cudaMemcpyHostToDevice));
@@ -361,7 +381,7 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
     }
   if (!tcs.empty() && !ctx->tcstream) CKS(cudaStreamCreateWithFlags(&ctx->tcstream, cudaStreamNonBlocking));
 
-  cudaEvent_t fork = nullptr, join[4] = {}, tjoin = nullptr;
+  cudaEvent_t fork = nullptr, join[5] = {}, tjoin = nullptr;
   CKS(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
   for (size_t k = 0; k < tls.size(); ++k) {
     if (!ctx->side[k]) CKS(cudaStreamCreateWithFlags(&ctx->side[k], cudaStreamNonBlocking));
@@ -423,7 +443,8 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
   for (size_t k = 0; k < tls.size(); ++k) {
     const TreeLaunch& L = tls[k];
     cudaStreamWaitEvent(ctx->side[k], fork, 0);
-    newt_launch_tree_lanes(L.dg, L.dq, L.items, L.L, L.serial, n_steps, ctx->tune_tree_grid_pct, ctx->side[k]);
+    if (L.threads) newt_launch_tree_threads(L.dg, L.dq, L.items, n_steps, ctx->side[k]);
+    else newt_launch_tree_lanes(L.dg, L.dq, L.items, L.L, L.serial, n_steps, ctx->tune_tree_grid_pct, ctx->side[k]);
     cudaEventRecord(join[k], ctx->side[k]);
   }
   const int pile_launches = (int)(ctx->launches - before) + batched_launches;
