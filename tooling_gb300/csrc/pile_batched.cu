@@ -578,14 +578,15 @@ __global__ void __launch_bounds__(256, 2) pile_k_contacts(Worlds W, int cap, int
 // one at each store took a sixth of its time.
 // work (nullable): [0] active contacts summed over every world's env-steps,
 // [1] rounds summed over sweeps, [2] rounds summed over env-steps, [3] worlds
-// stepped.  cost (per flat world index): this call's rounds over its sweeps
-// plus 64 per contact, the sort key of the next call's queue.
+// stepped.  cost (per flat world index): this graph's rounds over its sweeps
+// plus 64 per contact, the sort key of its next replay's queue.  `first`,
+// `tally`: the graph's first and last env-step; `last`: the call's last.
 NEWT_HD size_t sweep_smem(int S, int nbm, int space) {
   return (size_t)(32 / S) * (nbm + 1) * ACC * 4 + (size_t)space * 16;
 }
 
 template <int S>
-__global__ void __launch_bounds__(32, 12) pile_k_sweep(Worlds W, int nbm, int space, int first, int last,
+__global__ void __launch_bounds__(32, 12) pile_k_sweep(Worlds W, int nbm, int space, int first, int tally, int last,
                                                        unsigned long long* work, unsigned* cost) {
   extern __shared__ __align__(16) float4 ssm[];
   constexpr int N = 32 / S;
@@ -742,14 +743,14 @@ __global__ void __launch_bounds__(32, 12) pile_k_sweep(Worlds W, int nbm, int sp
     const int con = nact + (first ? 0 : xi[X.misc + B_CON]), lv = nr + (first ? 0 : xi[X.misc + B_LEV]);
     xi[X.misc + B_CON] = con;
     xi[X.misc + B_LEV] = lv;
-    if (last) {
+    if (tally) {
       const unsigned long long rounds = (unsigned long long)lv * (unsigned long long)max(iters, 0);
       if (cost) cost[flat] = (unsigned)min(rounds + 64ull * (unsigned long long)con, 0xffffffffull);
       if (work) {
         atomicAdd(work + 0, (unsigned long long)con);
         atomicAdd(work + 1, rounds);
         atomicAdd(work + 2, (unsigned long long)lv);
-        atomicAdd(work + 3, 1ull);
+        if (last) atomicAdd(work + 3, 1ull);
       }
     }
   }
@@ -835,11 +836,11 @@ extern "C" cudaError_t newt_pile_batched_plan(int shape, int worlds, int sms, in
   return e;
 }
 
-// One call's launches on `st`: the queue sort by last call's costs (when
+// One graph's launches on `st`: the queue sort by its last replay's costs (when
 // `cost` and `queue` are given), then two per env-step.  Every live world of
-// the table advances `n_steps` env-steps.
+// the table advances `n_steps` env-steps; `end`: the call's last.
 extern "C" int newt_launch_pile_batched(const PileGroupDev* dG, const int* dwseg, int ng, int* queue, int n,
-                                        int n_steps, unsigned long long* work, unsigned* cost,
+                                        int n_steps, int end, unsigned long long* work, unsigned* cost,
                                         const PileBatchedPlan* p, cudaStream_t st) {
   if (n <= 0) return 0;
   int launches = 0;
@@ -850,11 +851,11 @@ extern "C" int newt_launch_pile_batched(const PileGroupDev* dG, const int* dwseg
   const Worlds W{dG, dwseg, ng, queue, n};
   const int per = 32 / p->lanes;
   for (int s = 0; s < n_steps; ++s) {
-    const int last = s == n_steps - 1;
+    const int tally = s == n_steps - 1, last = tally && end;
     pile_k_contacts<<<(n + p->warps - 1) / p->warps, 32 * p->warps, (size_t)p->warps * p->stride * 4, st>>>(
         W, p->lanes / 2, p->stride, last);
     with_sweep(p->lanes, [&](auto kern) {
-      kern<<<(n + per - 1) / per, 32, sweep_smem(p->lanes, p->nbm, p->space), st>>>(W, p->nbm, p->space, s == 0, last, work,
+      kern<<<(n + per - 1) / per, 32, sweep_smem(p->lanes, p->nbm, p->space), st>>>(W, p->nbm, p->space, s == 0, tally, last, work,
                                                                                         cost);
     });
     launches += 2;

@@ -270,8 +270,7 @@ int newt_gpu_destroy(newt_gpu_ctx* ctx) {
   cudaStreamSynchronize(ctx->stream);
   for (auto& g : ctx->groups) g->release();
   if (ctx->l2buf) cudaFree(ctx->l2buf);
-  if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
-  for (void* p : ctx->plan_bufs) cudaFree(p);
+  for (StepGraph& g : ctx->graphs) g.drop();
   for (void* p : ctx->plain_bufs) cudaFree(p);
   for (cudaStream_t s : ctx->side) if (s) cudaStreamDestroy(s);
   for (int k = 0; k < 3; ++k) if (ctx->pside[k]) cudaStreamDestroy(ctx->pside[k]);

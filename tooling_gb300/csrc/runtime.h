@@ -141,6 +141,21 @@ struct HostGroup {
   int Ic(size_t row, size_t w) const { return soa() ? hI[row * cap + w] : hI[w * irows + row]; }
 };
 
+// A captured graph of the batched form: the env-steps of a whole call, or of a
+// long call a piece or the end (step.cu).
+enum GraphPart { GRAPH_WHOLE, GRAPH_PIECE, GRAPH_END };
+struct StepGraph {
+  cudaGraphExec_t exec = nullptr;
+  int steps = -1;
+  GraphPart part = GRAPH_WHOLE;
+  std::vector<void*> bufs;  // device queues and group tables it reads
+  int launches = 0;         // kernels a replay issues
+  std::vector<std::pair<int*, int>> lists;  // island work lists (pointer, slots)
+  int kev_steps = 0, kev_branches = 1, tc_steps = 0;  // env-steps with timing events (profiling)
+  bool fused = false;       // it holds the batched pile launches
+  void drop();
+};
+
 struct newt_gpu_ctx {
   int device = 0;
   int max_worlds = 0;
@@ -157,11 +172,8 @@ struct newt_gpu_ctx {
   unsigned l2flip = 0;
   int64_t launches = 0;
   // batched path
-  cudaGraphExec_t graph_exec = nullptr;
-  int graph_steps = -1;
+  StepGraph graphs[2];      // a whole call's or a long call's end; a long call's pieces
   bool graph_dirty = true;
-  std::vector<void*> plan_bufs;  // device queues / group tables the graph reads
-  int queue_items = 0;
   cudaStream_t side[5] = {};     // capture branches of the tree launches, one per size bucket
   cudaStream_t pside[3] = {nullptr, nullptr, nullptr};  // pile island-class branches
   cudaEvent_t pev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -177,17 +189,13 @@ struct newt_gpu_ctx {
   // default: lanes by the worlds' size and number, eight warps per block in
   // the contact stage, the fastest on 8192 sixteen-body piles)
   int tune_pile_fused = 1, tune_fused_shape = 10;
-  // the persistent launch of the captured graph: its timing events (external
-  // records when profiling), its work counters (device: contacts, rounds,
-  // levels, worlds) and whether the graph holds one; `last_fused` tells the
-  // profiling surface that the last batched call ran it
+  // the batched pile launches: their timing events (external records when
+  // profiling) and work counters (device: contacts, rounds, levels, worlds);
+  // `last_fused` tells the profiling surface that the last batched call ran them
   cudaEvent_t fkev[2] = {nullptr, nullptr};
   unsigned long long* fused_work = nullptr;
-  bool graph_fused = false, last_fused = false;
-  // tree-contact groups' branch of the captured graph, and its env-steps
-  // with timing events (profiling)
-  cudaStream_t tcstream = nullptr;
-  int graph_tc_steps = 0;
+  bool last_fused = false;
+  cudaStream_t tcstream = nullptr;  // tree-contact groups' branch of the captured graph
   cudaStream_t pbs[PILE_BRANCHES][4] = {};
   cudaEvent_t pbe[PILE_BRANCHES][5] = {};
   // plain path: one single-group table per group
@@ -202,8 +210,6 @@ struct newt_gpu_ctx {
   std::vector<cudaEvent_t> kev;  // [branch][env-step][kernel][start, end]
   int kev_steps = 0, kev_branches = 1;
   std::vector<std::pair<int*, int>> last_lists;
-  std::vector<std::pair<int*, int>> graph_lists;  // the captured graph's, copied to last_lists per replay
-  int graph_kev_steps = 0, graph_kev_branches = 1;
   // tree-contact step timing: 3 kernels x (start, end) per env-step of the
   // last tree-contact step call, recorded when `profile` is on
   std::vector<cudaEvent_t> tcev;

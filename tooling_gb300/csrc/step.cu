@@ -38,7 +38,7 @@ extern "C" cudaError_t newt_pile_batched_plan(int shape, int worlds, int sms, in
                                               PileBatchedPlan* p);
 extern "C" int newt_pile_batched_words(const PileGroupDev* g);
 extern "C" int newt_launch_pile_batched(const PileGroupDev* dG, const int* dwseg, int ng, int* queue, int n,
-                                        int n_steps, unsigned long long* work, unsigned* cost,
+                                        int n_steps, int end, unsigned long long* work, unsigned* cost,
                                         const PileBatchedPlan* p, cudaStream_t st);
 extern "C" int newt_tc_prepare(newt_gpu_ctx* ctx, HostGroup* g, int n_steps);
 extern "C" size_t newt_pile_newton_bytes(int maxc);
@@ -239,7 +239,13 @@ int step_plain(newt_gpu_ctx* ctx, int n_steps) {
 // ---------------------------------------------------------------------------
 // batched
 // ---------------------------------------------------------------------------
-static int capture(newt_gpu_ctx* ctx, int n_steps) {
+void StepGraph::drop() {
+  if (exec) cudaGraphExecDestroy(exec);
+  for (void* p : bufs) cudaFree(p);
+  *this = StepGraph{};
+}
+
+static int capture(newt_gpu_ctx* ctx, int n_steps, GraphPart part, StepGraph& out) {
   std::vector<void*> bufs;
   // trees: one launch per size bucket over a cost-sorted queue, each on its
   // own branch (the bucket's largest tree sizes the blocks' shared memory)
@@ -393,9 +399,9 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
     int r = ensure_kernel_events(ctx, n_steps, nbr);
     if (r != NEWT_OK) return r;
   }
-  ctx->graph_lists.clear();
+  std::vector<std::pair<int*, int>> lists;
   for (const PileTable& t : pts)
-    if (t.ng > 0) ctx->graph_lists.push_back({t.lists, t.slots});
+    if (t.ng > 0) lists.push_back({t.lists, t.slots});
   CKS(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
   cudaEventRecord(fork, ctx->stream);
   int tc_timed = 0;
@@ -414,7 +420,7 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
   if (!bls.empty()) {
     cudaStream_t f0 = ctx->pbs[0][0];
     cudaStreamWaitEvent(f0, fork, 0);
-    cudaMemsetAsync(ctx->fused_work, 0, 4 * sizeof(unsigned long long), f0);
+    if (part == GRAPH_WHOLE) cudaMemsetAsync(ctx->fused_work, 0, 4 * sizeof(unsigned long long), f0);
     if (ctx->profile) cudaEventRecordWithFlags(ctx->fkev[0], f0, cudaEventRecordExternal);
     cudaEventRecord(ctx->pbe[0][3], f0);
     for (size_t k = 0; k < bls.size(); ++k) {
@@ -422,7 +428,7 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
       cudaStream_t fs = ctx->pbs[k][0];
       if (k > 0) cudaStreamWaitEvent(fs, ctx->pbe[0][3], 0);
       batched_launches += newt_launch_pile_batched(L.t.dG, L.t.dseg, L.t.ng, L.queue, L.t.worlds, n_steps,
-                                                   ctx->fused_work, L.cost, &L.plan, fs);
+                                                   part != GRAPH_PIECE, ctx->fused_work, L.cost, &L.plan, fs);
       if (k > 0) {
         cudaEventRecord(ctx->pbe[k][4], fs);
         cudaStreamWaitEvent(f0, ctx->pbe[k][4], 0);
@@ -449,10 +455,7 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
   }
   const int pile_launches = (int)(ctx->launches - before) + batched_launches;
   ctx->launches = l0;
-  ctx->graph_kev_steps = ctx->profile && nbr > 0 && pile_worlds > 0 ? n_steps : 0;
-  ctx->graph_kev_branches = std::max(nbr, 1);
-  ctx->graph_fused = !bls.empty();
-  ctx->graph_tc_steps = tc_timed;
+  const int kev_steps = ctx->profile && nbr > 0 && pile_worlds > 0 ? n_steps : 0;
   for (size_t k = 0; k < tls.size(); ++k) cudaStreamWaitEvent(ctx->stream, join[k], 0);
   if (!tcs.empty()) cudaStreamWaitEvent(ctx->stream, tjoin, 0);
   cudaError_t ce = cudaStreamEndCapture(ctx->stream, &graph);
@@ -460,32 +463,63 @@ static int capture(newt_gpu_ctx* ctx, int n_steps) {
   for (size_t k = 0; k < tls.size(); ++k) cudaEventDestroy(join[k]);
   cudaEventDestroy(tjoin);
   if (ce != cudaSuccess) { ctx->err = cudaGetErrorString(ce); return NEWT_E_CUDA; }
-  if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
-  CKS(cudaGraphInstantiate(&ctx->graph_exec, graph, 0));
+  out.drop();
+  CKS(cudaGraphInstantiate(&out.exec, graph, 0));
   cudaGraphDestroy(graph);
-  for (void* p : ctx->plan_bufs) cudaFree(p);
-  ctx->plan_bufs = bufs;
-  ctx->graph_steps = n_steps;
-  ctx->graph_dirty = false;
-  // kernel launches one replay issues
-  ctx->queue_items = (int)tls.size() + pile_launches + tc_launches;
+  out.bufs = bufs;
+  out.steps = n_steps;
+  out.part = part;
+  out.launches = (int)tls.size() + pile_launches + tc_launches;
+  out.lists = lists;
+  out.kev_steps = kev_steps;
+  out.kev_branches = std::max(nbr, 1);
+  out.tc_steps = tc_timed;
+  out.fused = !bls.empty();
   return NEWT_OK;
 }
 
+// Env-steps per graph of a call with worlds that take kernels every env-step:
+// a longer call replays a graph of so many and one of the rest, so that its
+// capture and its graph stay small (one pile: 5 us of the host, 15 KB of its
+// memory and 5 KB of the device's an env-step; 100000 env-steps 0.6 s, 1.5 GB
+// and 461 MB in one graph).  The boundaries cost less than one run differs from
+// the next (5000 env-steps of ten 16-body piles 442 ms in one graph, 440 in 40).
+constexpr int LONG_CALL = 128;
+
 int step_batched(newt_gpu_ctx* ctx, int n_steps) {
-  if (ctx->graph_dirty || ctx->graph_steps != n_steps || !ctx->graph_exec) {
-    int rc = capture(ctx, n_steps);
-    if (rc != NEWT_OK) return rc;
+  bool per_step = false;
+  for (auto& gp : ctx->groups) per_step = per_step || (gp->kind != GK_TREE && gp->n > 0);
+  const int pieces = per_step && !ctx->profile && n_steps > LONG_CALL ? (n_steps - 1) / LONG_CALL : 0;
+  const int end = n_steps - pieces * LONG_CALL;
+  if (ctx->graph_dirty)
+    for (StepGraph& g : ctx->graphs) g.drop();
+  ctx->graph_dirty = false;
+  StepGraph &last = ctx->graphs[0], &piece = ctx->graphs[1];
+  auto ready = [&](StepGraph& g, int steps, GraphPart part) -> int {
+    if (g.exec && g.steps == steps && g.part == part) return NEWT_OK;
+    const int rc = capture(ctx, steps, part, g);
+    if (ctx->graph_dirty) (&g == &last ? piece : last).drop();  // a group's scratch moved on the way
+    ctx->graph_dirty = rc != NEWT_OK;
+    return rc;
+  };
+  int rc = NEWT_OK;
+  if (pieces > 0 && (rc = ready(piece, LONG_CALL, GRAPH_PIECE)) != NEWT_OK) return rc;
+  if ((rc = ready(last, end, pieces > 0 ? GRAPH_END : GRAPH_WHOLE)) != NEWT_OK) return rc;
+  if (pieces > 0 && (rc = ready(piece, LONG_CALL, GRAPH_PIECE)) != NEWT_OK) return rc;
+  if (pieces > 0 && last.fused) CKS(cudaMemsetAsync(ctx->fused_work, 0, 4 * sizeof(unsigned long long), ctx->stream));
+  for (int k = 0; k < pieces && piece.launches > 0; ++k) {
+    CKS(cudaGraphLaunch(piece.exec, ctx->stream));
+    ctx->launches += piece.launches;
   }
-  if (ctx->queue_items > 0) {
-    CKS(cudaGraphLaunch(ctx->graph_exec, ctx->stream));
-    ctx->launches += ctx->queue_items;
+  if (last.launches > 0) {
+    CKS(cudaGraphLaunch(last.exec, ctx->stream));
+    ctx->launches += last.launches;
   }
-  ctx->last_lists = ctx->graph_lists;
-  ctx->kev_steps = ctx->graph_kev_steps;
-  ctx->kev_branches = ctx->graph_kev_branches;
-  ctx->last_fused = ctx->graph_fused;
-  ctx->tcev_steps = ctx->graph_tc_steps;
+  ctx->last_lists = last.lists;
+  ctx->kev_steps = last.kev_steps;
+  ctx->kev_branches = last.kev_branches;
+  ctx->last_fused = last.fused;
+  ctx->tcev_steps = last.tc_steps;
   return NEWT_OK;
 }
 
