@@ -468,14 +468,15 @@ NEWT_API int newt_gpu_serve(newt_gpu_ctx* ctx, newt_serve_request* reqs, int32_t
 NEWT_API int newt_gpu_pile_profile(newt_gpu_ctx* ctx, int32_t enable, float* kernel_ms, int32_t* work,
                                    int32_t* launches);
 
-/* Profiling surface of the world-persistent pile launch (no counterpart in
- * newt).  After waiting for the last newt_gpu_step call: `kernel_ms` (nullable)
- * its device time, when timing is on (newt_gpu_pile_profile's `enable`) and
- * that call was batched with piles in the persistent launch, else 0; `work`
- * (nullable, 4 counters, zero unless that call ran the launch): active
- * contacts summed over every world's env-steps, contact-update rounds (a
- * dependency level's groups of eight contacts) summed over the sweeps,
- * dependency levels summed over env-steps, worlds stepped. */
+/* Profiling surface of the batched pile launches (no counterpart in newt).
+ * After waiting for the last newt_gpu_step call: `kernel_ms` (nullable) their
+ * device time from the first to the last, when timing is on
+ * (newt_gpu_pile_profile's `enable`) and that call was batched with piles in
+ * these launches, else 0; `work` (nullable, 4 counters, zero unless that call
+ * ran them), whatever the launch choice: active contacts summed over every
+ * world's env-steps, contact-update rounds (a dependency level's groups of
+ * eight contacts) summed over the sweeps, dependency levels summed over
+ * env-steps, worlds stepped. */
 NEWT_API int newt_gpu_pile_fused_profile(newt_gpu_ctx* ctx, float* kernel_ms, uint64_t* work);
 
 /* Profiling surface of the tree-contact step (quadruped worlds).  With

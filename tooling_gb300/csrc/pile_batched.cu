@@ -374,7 +374,7 @@ NEWT_D void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // What pile_k_contacts leaves for pile_k_sweep in the world's scratch record:
 // the rows at L.sc (float4 q of row s at q * nact + s, in sweep order), their
 // body words at L.ci, and these ints.
-enum { B_NACT = 0, B_ROUNDS = 1, B_CON = 2, B_LEV = 3 };  // at L.misc; B_CON, B_LEV: totals over the call's env-steps
+enum { B_NACT = 0, B_ROUNDS = 1, B_CON = 2, B_RND = 3 };  // at L.misc; B_CON, B_RND: totals over the graph's env-steps
 
 struct Worlds {
   const PileGroupDev* G;
@@ -399,10 +399,12 @@ NEWT_D const PileGroupDev* world_at(const Worlds& W, int item, int* w, int* flat
 
 // `cap`: contacts per round of the sweeps; `stride`: words of shared memory
 // per warp; `last`: the call's last env-step (the contacts go to the world
-// record).  The warps of a block meet between the phases: the code is long
+// record); `work`: pile_k_sweep's.  (The counters are added here, where the
+// levels are: as totals in pile_k_sweep they cost its loop 5%, by registers.)  The warps of a block meet between the phases: the code is long
 // and runs once per world, and warps that are spread over it wait for
 // instructions more than for anything else.
-__global__ void __launch_bounds__(256, 2) pile_k_contacts(Worlds W, int cap, int stride, int last) {
+__global__ void __launch_bounds__(256, 2) pile_k_contacts(Worlds W, int cap, int stride, int last,
+                                                       unsigned long long* work) {
   extern __shared__ __align__(16) float psm[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   int w = 0, flat;
@@ -510,7 +512,7 @@ __global__ void __launch_bounds__(256, 2) pile_k_contacts(Worlds W, int cap, int
     // sweep order: by level, rounds of at most `cap` contacts; each round's
     // first row goes to the scratch record's schedule
     int* loff = xi + X.scid;
-    int row0 = 0, rounds = 0;
+    int row0 = 0, rounds = 0, levels = 0, eights = 0;
     for (int v = 1; row0 < nact; ++v) {
       int cnt = 0;
 #pragma unroll 1
@@ -525,11 +527,17 @@ __global__ void __launch_bounds__(256, 2) pile_k_contacts(Worlds W, int cap, int
       if (lane < nr) loff[rounds + lane] = row0 + cap * lane;
       row0 += cnt;
       rounds += nr;
+      ++levels;
+      eights += (cnt + 7) / 8;
     }
     if (lane == 0) {
       loff[rounds] = nact;
       xi[X.misc + B_NACT] = nact;
       xi[X.misc + B_ROUNDS] = rounds;
+      if (levels > 0) {
+        atomicAdd(work + 1, (unsigned long long)eights * (unsigned long long)max(si[gp->lay.iters], 0));
+        atomicAdd(work + 2, (unsigned long long)levels);
+      }
     }
     __syncwarp();
   }
@@ -576,11 +584,12 @@ __global__ void __launch_bounds__(256, 2) pile_k_contacts(Worlds W, int cap, int
 // without a contact in a round updates the row of zeros against the static
 // side's zero: the round is straight-line code, where a branch around it and
 // one at each store took a sixth of its time.
-// work (nullable): [0] active contacts summed over every world's env-steps,
-// [1] rounds summed over sweeps, [2] rounds summed over env-steps, [3] worlds
-// stepped.  cost (per flat world index): this graph's rounds over its sweeps
-// plus 64 per contact, the sort key of its next replay's queue.  `first`,
-// `tally`: the graph's first and last env-step; `last`: the call's last.
+// work: [0] active contacts summed over every world's env-steps, [3] worlds
+// stepped; pile_k_contacts adds [1] the levels' groups of eight contacts summed
+// over the sweeps and [2] the levels summed over env-steps.  cost (per flat
+// world index): this graph's rounds over its sweeps plus 64 per contact, the
+// sort key of its next replay's queue.  `first`, `tally`: the graph's first and
+// last env-step; `last`: the call's last.
 NEWT_HD size_t sweep_smem(int S, int nbm, int space) {
   return (size_t)(32 / S) * (nbm + 1) * ACC * 4 + (size_t)space * 16;
 }
@@ -740,18 +749,14 @@ __global__ void __launch_bounds__(32, 12) pile_k_sweep(Worlds W, int nbm, int sp
       o[0] = f.x; o[1] = f.y; o[2] = f.z; o[3] = f.w;
     }
   if (l == 0) {
-    const int con = nact + (first ? 0 : xi[X.misc + B_CON]), lv = nr + (first ? 0 : xi[X.misc + B_LEV]);
+    const int con = nact + (first ? 0 : xi[X.misc + B_CON]), rnd = nr + (first ? 0 : xi[X.misc + B_RND]);
     xi[X.misc + B_CON] = con;
-    xi[X.misc + B_LEV] = lv;
+    xi[X.misc + B_RND] = rnd;
     if (tally) {
-      const unsigned long long rounds = (unsigned long long)lv * (unsigned long long)max(iters, 0);
+      const unsigned long long rounds = (unsigned long long)rnd * (unsigned long long)max(iters, 0);
       if (cost) cost[flat] = (unsigned)min(rounds + 64ull * (unsigned long long)con, 0xffffffffull);
-      if (work) {
-        atomicAdd(work + 0, (unsigned long long)con);
-        atomicAdd(work + 1, rounds);
-        atomicAdd(work + 2, (unsigned long long)lv);
-        if (last) atomicAdd(work + 3, 1ull);
-      }
+      atomicAdd(work + 0, (unsigned long long)con);
+      if (last) atomicAdd(work + 3, 1ull);
     }
   }
 }
@@ -853,7 +858,7 @@ extern "C" int newt_launch_pile_batched(const PileGroupDev* dG, const int* dwseg
   for (int s = 0; s < n_steps; ++s) {
     const int tally = s == n_steps - 1, last = tally && end;
     pile_k_contacts<<<(n + p->warps - 1) / p->warps, 32 * p->warps, (size_t)p->warps * p->stride * 4, st>>>(
-        W, p->lanes / 2, p->stride, last);
+        W, p->lanes / 2, p->stride, last, work);
     with_sweep(p->lanes, [&](auto kern) {
       kern<<<(n + per - 1) / per, 32, sweep_smem(p->lanes, p->nbm, p->space), st>>>(W, p->nbm, p->space, s == 0, tally, last, work,
                                                                                         cost);
