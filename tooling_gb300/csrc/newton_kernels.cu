@@ -62,6 +62,7 @@
 #include "groups.h"
 #include "narrowphase.cuh"
 #include "newton_dense.cuh"
+#include "quotient.cuh"
 #include "runtime.h"
 
 namespace {

@@ -399,9 +399,10 @@ NEWT_D const PileGroupDev* world_at(const Worlds& W, int item, int* w, int* flat
 
 // `cap`: contacts per round of the sweeps; `stride`: words of shared memory
 // per warp; `last`: the call's last env-step (the contacts go to the world
-// record); `work`: pile_k_sweep's.  (The counters are added here, where the
-// levels are: as totals in pile_k_sweep they cost its loop 5%, by registers.)  The warps of a block meet between the phases: the code is long
-// and runs once per world, and warps that are spread over it wait for
+// record); `work`: pile_k_sweep's.  (Its counters of levels are added here,
+// where the levels are: as totals in pile_k_sweep they cost that loop 5%, by
+// its registers.)  The warps of a block meet between the phases: the code is
+// long and runs once per world, and warps that are spread over it wait for
 // instructions more than for anything else.
 __global__ void __launch_bounds__(256, 2) pile_k_contacts(Worlds W, int cap, int stride, int last,
                                                        unsigned long long* work) {

@@ -26,6 +26,7 @@
 #include "../../include/newt_gpu.h"
 #include "newton_dense.cuh"
 #include "pile_solver.cuh"
+#include "quotient.cuh"
 
 using namespace pile;
 
@@ -225,13 +226,6 @@ NEWT_HD NbSmem nb_smem(int rows) {
   n.flag = f; f += 8;
   n.words = (f + 3) / 4 * 4;
   return n;
-}
-
-// x / d with r = 1 / d: the product corrected by the remainder (P. Markstein,
-// IBM J. Res. Dev. 34(1), 1990).
-NEWT_D float nb_quot(float x, float d, float r) {
-  const float q = x * r;
-  return fmaf(fmaf(-q, d, x), r, q);
 }
 
 template <int ROWS>
@@ -435,10 +429,10 @@ NEWT_D void newton_block(const PileGroupDev& g, int w, float* nbs) {
         const float4 v = f4(V + p), i = f4(di + p);
         const float l00 = M[p * ld + p];
         const float4 l1 = f4(M + (p + 1) * ld + p), l2 = f4(M + (p + 2) * ld + p), l3 = f4(M + (p + 3) * ld + p);
-        const float y0 = nb_quot(v.x, l00, i.x);
-        const float y1 = nb_quot(fmaf(-l1.x, y0, v.y), l1.y, i.y);
-        const float y2 = nb_quot(fmaf(-l2.y, y1, fmaf(-l2.x, y0, v.z)), l2.z, i.z);
-        const float y3 = nb_quot(fmaf(-l3.z, y2, fmaf(-l3.y, y1, fmaf(-l3.x, y0, v.w))), l3.w, i.w);
+        const float y0 = quot(v.x, l00, i.x);
+        const float y1 = quot(fmaf(-l1.x, y0, v.y), l1.y, i.y);
+        const float y2 = quot(fmaf(-l2.y, y1, fmaf(-l2.x, y0, v.z)), l2.z, i.z);
+        const float y3 = quot(fmaf(-l3.z, y2, fmaf(-l3.y, y1, fmaf(-l3.x, y0, v.w))), l3.w, i.w);
         if (in && r >= p + 4) {
           const float4 l = f4(row + p);
           d = fmaf(-l.x, y0, d);
@@ -457,10 +451,10 @@ NEWT_D void newton_block(const PileGroupDev& g, int w, float* nbs) {
         const float4 v = f4(V + p), i = f4(di + p);
         const float l00 = M[p * ld + p];
         const float4 l1 = f4(M + (p + 1) * ld + p), l2 = f4(M + (p + 2) * ld + p), l3 = f4(M + (p + 3) * ld + p);
-        const float z3 = nb_quot(v.w, l3.w, i.w);
-        const float z2 = nb_quot(fmaf(-l3.z, z3, v.z), l2.z, i.z);
-        const float z1 = nb_quot(fmaf(-l2.y, z2, fmaf(-l3.y, z3, v.y)), l1.y, i.y);
-        const float z0 = nb_quot(fmaf(-l1.x, z1, fmaf(-l2.x, z2, fmaf(-l3.x, z3, v.x))), l00, i.x);
+        const float z3 = quot(v.w, l3.w, i.w);
+        const float z2 = quot(fmaf(-l3.z, z3, v.z), l2.z, i.z);
+        const float z1 = quot(fmaf(-l2.y, z2, fmaf(-l3.y, z3, v.y)), l1.y, i.y);
+        const float z0 = quot(fmaf(-l1.x, z1, fmaf(-l2.x, z2, fmaf(-l3.x, z3, v.x))), l00, i.x);
         if (r < p) {
           const float* c = M + p * ld + r;
           d = fmaf(-c[3 * ld], z3, d);

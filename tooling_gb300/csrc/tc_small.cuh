@@ -26,10 +26,6 @@
 // memory 1.1, barriers 1.0).  Blocks of four worlds, four to an SM, against
 // eight and two: 917 and 939 us for two env-steps; without the barriers around
 // the Newton stage 932 to 948.
-//
-// Quotients by a factor's pivots are x * r corrected by the remainder
-// x - q d (r the correctly rounded reciprocal of d; P. Markstein, IBM J. Res.
-// Dev. 34(1), 1990).
 
 constexpr int TCS_WARPS = 4;   // worlds (warps) per block
 constexpr int TCS_BLOCKS = 4;  // blocks per SM
@@ -75,11 +71,6 @@ NEWT_HD TcsSmem tcs_smem(int L, int nv, int maxc, int rpc) {
 }
 
 NEWT_D float4 f4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-// x / d with r = 1 / d
-NEWT_D float quot(float x, float d, float r) {
-  const float q = x * r;
-  return fmaf(fmaf(-q, d, x), r, q);
-}
 
 // Columns of the point Jacobian, as chain_columns, from the levers of
 // tc_kinematics and the angular axes `wa` of the DoFs.
@@ -241,15 +232,6 @@ NEWT_D bool chol_one(float* m, int n, int nr, int ld, float* di, int lane, float
   *mn = lo;
   *mx = hi;
   return ok;
-}
-
-// a / b rounded to FP32: the FP32 quotient corrected by its FP64 remainder (an
-// FP64 divide keeps the FP64 pipe busy several times as long).
-NEWT_D float quot_d(double a, double b) {
-  const float bf = (float)b;
-  if (!(bf > 1e-30f && bf < 1e30f)) return (float)(a / b);
-  const float r = 1.f / bf, q = (float)a * r;
-  return fmaf((float)fma(-(double)q, b, a), r, q);
 }
 
 // Row times a shared vector (zeros from nr up to the next multiple of four).
