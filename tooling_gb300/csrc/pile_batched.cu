@@ -218,6 +218,7 @@ NEWT_D void pair_step(float fi, float fj, float ri, float rj, float h11, float h
   *nj = uj >= 0.f ? (ui >= 0.f ? uj : sj) : 0.f;
 }
 
+constexpr int FARS = 10;  // percent of a warp's rows past their place that pile_k_sweep's own loops put up with
 constexpr int ACC = 12;  // floats per body of the accumulators (six used): 16-byte aligned, spread over the banks
 
 // What a contact's update reads of its row and does not change.
@@ -293,6 +294,69 @@ NEWT_D void row_update(const RowRegs& R, float4* fp, float* A, bool write, int s
 __device__ __noinline__ void row_update_far(float4* x, int stride, float* A, bool write, int single, int side,
                                             unsigned pair) {
   row_update<true>(row_load(x, stride, side), x + ROW_F4 * stride, A, write, single, side, pair, [] {});
+}
+
+// The sweeps of a warp whose schedule or more than a few of its rows exceed
+// their place in shared memory: rows from either memory, any pairs, the
+// schedule from the scratch record.  Out of line, so that pile_k_sweep's own
+// loop keeps its registers.  As there, a round's constants are read while the
+// one before it updates, its rows' bodies a round before that and its bounds
+// one more.  Contacts between boxes come in fours on the same two bodies, so
+// stacks and walls have as many rounds: us an env-step with every far row read
+// in its own round, and now (the world-persistent kernel in brackets): 1000
+// walls of 8 boxes 1203, 643 (849), of 16 2135, 1474 (1544), 8192 of 16 9123,
+// 5829 (8382), 1000 stacks of 16 1655, 877 (1187).
+// The lane's world: `fit` of its nact rows lie at `mine`, all at `rec`; nr
+// rounds that start at loff[], body words `words`, `iters` sweeps; nrm and itm:
+// the warp's rounds and sweeps.
+struct MixedWorld {
+  float4 *zero, *mine, *rec;
+  float* acc;
+  const int *loff, *words;
+  int fit, nact, nr, iters, nb;
+};
+__device__ __noinline__ void sweep_mixed(const MixedWorld W, int nrm, int itm, int slot, int side) {
+  float4 *const zero = W.zero, *const mine = W.mine, *const rec = W.rec;
+  float* const acc = W.acc;
+  const int *const loff = W.loff, *const words = W.words;
+  const int fit = W.fit, nact = W.nact, nr = W.nr, iters = W.iters, nb = W.nb;
+  int ra = 0, ia = 0, left = itm * nrm;
+  if (left <= 0) return;
+  struct Bounds { int lo, hi; };
+  auto bounds = [&]() {  // of the next round, none past the end
+    Bounds b{0, 0};
+    if (ia < iters && ra < nr) b = Bounds{loff[ra], loff[ra + 1]};
+    if (++ra == nrm) { ra = 0; ++ia; }
+    return b;
+  };
+  struct Place { int s, word; };  // a row or -1, its bodies
+  auto place = [&](Bounds b) {
+    Place p{b.lo + slot < b.hi ? b.lo + slot : -1, nb | nb << 8};
+    if (p.s >= 0) p.word = words[p.s];
+    return p;
+  };
+  auto row = [&](Place p) { return p.s < 0 ? zero : p.s < fit ? mine + (size_t)p.s * ROW_V4 : rec + p.s; };
+  auto stride = [&](Place p) { return p.s >= fit ? nact : 1; };
+  auto load = [&](Place p) { return row_load(row(p), stride(p), side); };
+  auto update = [&](const RowRegs& R, Place p, auto ahead) {
+    const int b = (side ? p.word >> 8 : p.word) & 0xff;
+    row_update<true>(R, row(p) + ROW_F4 * stride(p), acc + ACC * b, b < nb, p.s < 0 ? 0 : p.word >> 16, side, FULL, ahead);
+    __syncwarp();
+  };
+  Bounds b2 = bounds();
+  Place p0 = place(b2), p1;
+  b2 = bounds();
+  p1 = place(b2);
+  b2 = bounds();
+  RowRegs R0 = load(p0), R1;
+  Place p2;
+  for (; left > 1; left -= 2) {
+    update(R0, p0, [&] { R1 = load(p1); p2 = place(b2); b2 = bounds(); });
+    p0 = p2;
+    update(R1, p1, [&] { R0 = load(p0); p2 = place(b2); b2 = bounds(); });
+    p1 = p2;
+  }
+  if (left > 0) update(R0, p0, [] {});
 }
 
 }  // namespace
@@ -622,18 +686,22 @@ __global__ void __launch_bounds__(32, 12) pile_k_sweep(Worlds W, int nbm, int sp
     iters = g->I[(size_t)w * g->lay.istride + g->lay.iters];
   }
   for (int b = l; b < ACC * (nbm + 1); b += S) acc[b] = 0.f;
-  int base = 0, nrm = nr, itm = iters;  // this world's first row in the pool; the warp's rounds and sweeps
+  int base = 0, rows = 0, nrm = nr, itm = iters;  // this world's first row in the pool; the warp's rows, rounds and sweeps
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     const int o = __shfl_sync(FULL, nact, k * S);
     if (k < sub) base += o;
+    rows += o;
   }
 #pragma unroll
   for (int o = 16; o >= S; o >>= 1) {
     nrm = max(nrm, __shfl_xor_sync(FULL, nrm, o));
     itm = max(itm, __shfl_xor_sync(FULL, itm, o));
   }
-  const bool fits = ROW_V4 + 16 * nrm <= space;  // the schedule does (uniform over the warp)
+  // the schedule and all rows but FARS in a hundred fit (uniform over the warp;
+  // at 25 in a hundred 1000 stacks of 20 took 1046 us an env-step, 987 at 10, at
+  // 50 those of 16 1663 in place of 876)
+  const bool fits = 100 * (space - ROW_V4 - 16 * nrm) >= (100 - FARS) * ROW_V4 * rows;
   int2* sched = reinterpret_cast<int2*>(zero + ROW_V4) + lane;
   const int head = ROW_V4 + (fits ? 16 * nrm : 0), fit = max(0, min(nact, (space - head) / ROW_V4 - base));
   float4* mine = zero + head + (size_t)base * ROW_V4;
@@ -662,11 +730,6 @@ __global__ void __launch_bounds__(32, 12) pile_k_sweep(Worlds W, int nbm, int sp
   copies_done();
   __syncwarp();
   auto at_bytes = [](auto* p, int o) { return reinterpret_cast<decltype(p)>(reinterpret_cast<char*>(p) + o); };
-  auto far_update = [&](int s, int y) {
-    const bool in = s < fit;
-    row_update_far(in ? mine + (size_t)s * ROW_V4 : rec + s, in ? 1 : nact, at_bytes(acc, y & ~(STATIC | FAR)), y >= 0,
-                   xi[X.ci + s] >> 16, side, pair);
-  };
   if (fits && __all_sync(FULL, plain)) {
     // The next round's constants are read while this one's update runs, and
     // its offsets a round before that: only the accumulators and the impulses,
@@ -708,21 +771,17 @@ __global__ void __launch_bounds__(32, 12) pile_k_sweep(Worlds W, int nbm, int sp
         row_update<false>(row_load(x, 1, side), x + ROW_F4, at_bytes(acc, near ? c.y & ~STATIC : 4 * ACC * nbm),
                           near && c.y >= 0, 0, side, FULL, [] {});
         if (__any_sync(FULL, far)) {
-          if (far) far_update(c.x, c.y);
+          if (far) {
+            const bool in = c.x < fit;
+            row_update_far(in ? mine + (size_t)c.x * ROW_V4 : rec + c.x, in ? 1 : nact, at_bytes(acc, c.y & ~(STATIC | FAR)),
+                           c.y >= 0, xi[X.ci + c.x] >> 16, side, pair);
+          }
           __syncwarp();
         }
         __syncwarp();
       }
   } else {
-    for (int it = 0; it < itm; ++it)
-      for (int r = 0; r < nrm; ++r) {
-        const int s = it < iters ? row_of(r) : -1;
-        if (s >= 0) {
-          const int b = body_of(xi[X.ci + s]);
-          far_update(s, 4 * ACC * b | (b < nb ? 0 : STATIC));
-        }
-        __syncwarp();
-      }
+    sweep_mixed(MixedWorld{zero, mine, rec, acc, loff, g ? xi + X.ci : nullptr, fit, nact, nr, iters, nb}, nrm, itm, slot, side);
   }
   if (!g) return;
   const PileLayout& P = g->lay;
