@@ -269,27 +269,32 @@ static int capture(newt_gpu_ctx* ctx, int n_steps, GraphPart part, StepGraph& ou
   };
   const int buckets[5] = {NEWT_TREE_TINY, 8, 16, 32, 65};
   for (int bucket : buckets) {
-    struct It { int cost, g, base, count; };
-    std::vector<It> its;
     std::vector<TreeGroupDev> tg;
     const bool threads = bucket == NEWT_TREE_TINY;
     const int chunk = threads ? NEWT_TREE_THREADS : newt_tree_item_worlds();
     int most = 0, serial = 1;
-    for (auto& gp : ctx->groups) {
-      HostGroup* g = gp.get();
-      if (g->n == 0 || g->kind != GK_TREE) continue;
-      if ((by_threads(g->size) ? NEWT_TREE_TINY : newt_tree_bucket(g->size)) != bucket) continue;
+    std::vector<HostGroup*> gs;
+    for (auto& gp : ctx->groups)
+      if (gp->n > 0 && gp->kind == GK_TREE &&
+          (by_threads(gp->size) ? NEWT_TREE_TINY : newt_tree_bucket(gp->size)) == bucket)
+        gs.push_back(gp.get());
+    if (gs.empty()) continue;
+    std::stable_sort(gs.begin(), gs.end(), [](HostGroup* a, HostGroup* b) { return a->size > b->size; });
+    size_t items = 0;
+    for (HostGroup* g : gs) items += (g->n + chunk - 1) / chunk;
+    std::vector<int> q(3 * items);
+    int* at = q.data();
+    for (HostGroup* g : gs) {
       for (int i = 1; i < g->size; ++i) serial &= g->topo[4 * i] == i - 1;
-      int gi = (int)tg.size();
-      tg.push_back(g->tree_dev());
       most = std::max(most, g->size);
-      for (int b = 0; b < g->n; b += chunk) its.push_back({g->size, gi, b, std::min(chunk, g->n - b)});
+      for (int b = 0; b < g->n; b += chunk, at += 3) {
+        at[0] = (int)tg.size();
+        at[1] = b;
+        at[2] = std::min(chunk, g->n - b);
+      }
+      tg.push_back(g->tree_dev());
     }
-    if (its.empty()) continue;
-    std::stable_sort(its.begin(), its.end(), [](const It& a, const It& b) { return a.cost > b.cost; });
-    std::vector<int> q;
-    for (auto& i : its) { q.push_back(i.g); q.push_back(i.base); q.push_back(i.count); }
-    TreeLaunch L{most, serial, nullptr, nullptr, (int)its.size(), threads};
+    TreeLaunch L{most, serial, nullptr, nullptr, (int)items, threads};
     CKS(newt_tree_lanes_prepare());
     CKS(cudaMalloc(&L.dg, tg.size() * sizeof(TreeGroupDev)));
     CKS(cudaMemcpy(L.dg, tg.data(), tg.size() * sizeof(TreeGroupDev), cudaMemcpyHostToDevice));
