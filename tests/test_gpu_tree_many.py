@@ -1,8 +1,7 @@
-"""Very many of the smallest trees in the batched form (a thread per world past
-80 worlds an SM of two or three links, 120 of four; tree_kernels.cu): the FP64
-oracle's step within the bars of test_gpu_tree_lanes.py on both sides of the
-line, blocks that are not full, held worlds, both integrators and both roots
-in one call, and larger trees beside them."""
+"""Many of the smallest trees in the batched form (tree_lanes.cu): the digits
+of the same worlds alone, the FP64 oracle's step within the bars of
+test_gpu_tree_lanes.py, blocks that are not full, held worlds, both
+integrators and both roots in one call, and larger trees beside them."""
 import numpy as np
 import pytest
 import torch
@@ -22,9 +21,8 @@ def _states(rng, m, n):
     return q.astype(np.float32), v.astype(np.float32), rng.normal(0, 0.5, (n, m.nv)).astype(np.float32)
 
 
-@pytest.mark.parametrize("links,per_sm", [(2, 80), (3, 80), (4, 120)])
-@pytest.mark.parametrize("past", [0, 1, 45])
-def test_many_small_trees_match_fp64(links, per_sm, past):
+@pytest.mark.parametrize("links", [2, 3, 4])
+def test_many_small_trees_match_fp64(links):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
     rng = np.random.default_rng([51, links])
     # four kinds: both roots, both integrators; a third with a slide
@@ -32,7 +30,7 @@ def test_many_small_trees_match_fp64(links, per_sm, past):
     for m in kinds[1:3]:
         m.links[1].joint = M.JOINT_SLIDE
     large = tree(rng, 9, False, False, False, jointmix=False)
-    W = per_sm * sms + past
+    W = 120 * sms + 45  # more than a wave
     eng = A.Engine()
     P = M.PackedModels(kinds + [large])
     ids = eng.upload(P)
@@ -53,8 +51,19 @@ def test_many_small_trees_match_fp64(links, per_sm, past):
     q, v = eng.get_state(slots, nq, nv)
     assert not eng.status(slots).any()
     oq, ov = eng.get_state(beside, large.nq, large.nv)
-    acc = eng.get_qacc(slots[:4], sum(m.nv for m in kinds))
+    acc = eng.get_qacc(slots[:12], 3 * sum(m.nv for m in kinds))
     eng.close()
+    # the first of them alone
+    eng = A.Engine()
+    few = eng.alloc(eng.upload(P)[k[:12]])
+    n, m = 3 * sum(x.nq for x in kinds), 3 * sum(x.nv for x in kinds)
+    eng.set_state(few, pick(0)[:n], pick(1)[:m])
+    eng.set_qfrc(few, pick(2)[:m])
+    eng.hold(few[5:6])  # as among the many
+    eng.step(2)
+    alone = eng.get_state(few, n, m) + (eng.get_qacc(few, m),)
+    eng.close()
+    assert np.array_equal(alone[0], q[:n]) and np.array_equal(alone[1], v[:m]) and np.array_equal(alone[2], acc)
     ref = {}
     for a, m in enumerate(kinds):
         for b in range(3):

@@ -14,10 +14,6 @@
 #define NEWT_MAX_BODIES 64
 #define NEWT_MAX_PLANES 4
 
-#define NEWT_TREE_TINY 4      // links up to which very many trees take a thread each (step.cu)
-#define NEWT_TREE_THREADS 32  // their worlds per queue item: a warp a block (24000 of 3 links: 72.6 us for ten
-                              // env-steps, 77.9 with two)
-
 enum GroupKind { GK_TREE = 0, GK_PILE = 1, GK_TREE_CONTACT = 2 };
 
 // Kinematic tree without contact (config 0 chains, config 3 chains).

@@ -174,7 +174,7 @@ struct newt_gpu_ctx {
   // batched path
   StepGraph graphs[2];      // a whole call's or a long call's end; a long call's pieces
   bool graph_dirty = true;
-  cudaStream_t side[5] = {};     // capture branches of the tree launches, one per size bucket
+  cudaStream_t side[4] = {};     // capture branches of the tree launches, one per size bucket
   cudaStream_t pside[3] = {nullptr, nullptr, nullptr};  // pile island-class branches
   cudaEvent_t pev[4] = {nullptr, nullptr, nullptr, nullptr};
   // batched piles: world-range branches, each with its own main stream, three

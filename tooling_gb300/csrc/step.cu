@@ -24,8 +24,6 @@
 extern "C" void newt_launch_tree_lanes(const TreeGroupDev* dgroups, const int* dqueue, int n_items, int L, int serial,
                                        int n_steps, int pct, cudaStream_t st);
 extern "C" cudaError_t newt_tree_lanes_prepare();
-extern "C" void newt_launch_tree_threads(const TreeGroupDev* dgroups, const int* dqueue, int n_items, int n_steps,
-                                         cudaStream_t st);
 extern "C" int newt_tree_item_worlds();
 extern "C" size_t newt_pile_ws_bytes(int nb, int np, int maxc);
 extern "C" int newt_launch_pile_step(const PileGroupDev* dG, const int* dwseg, int ng, int total_worlds,
@@ -249,35 +247,16 @@ static int capture(newt_gpu_ctx* ctx, int n_steps, GraphPart part, StepGraph& ou
   std::vector<void*> bufs;
   // trees: one launch per size bucket over a cost-sorted queue, each on its
   // own branch (the bucket's largest tree sizes the blocks' shared memory)
-  struct TreeLaunch { int L, serial; TreeGroupDev* dg; int* dq; int items; bool threads; };
+  struct TreeLaunch { int L, serial; TreeGroupDev* dg; int* dq; int items; };
   std::vector<TreeLaunch> tls;
-  // The smallest trees: eight lanes gain too little on a world of two or
-  // three joints where there are worlds enough for a thread each.  Us for ten
-  // env-steps, lanes and threads: fixed base, 2 hinges (3 links), 8000 worlds
-  // 45 and 52, 13000 66 and 57, 40000 157 and 94, 100000 347 and 233; floating
-  // under RK4 202 and 249, 340 and 292, 873 and 523, 2025 and 1559; 3 hinges,
-  // fixed under RK4, 16000 320 and 336, 25000 490 and 446, 40000 760 and 597;
-  // 4 hinges, 100000 560 and 589.  The lines lie past the crossings, since the
-  // threads' recursion (about the joints' anchors) ends 4 to 8% further from
-  // 64 bits.
-  long small = 0, tiny = 0;
-  for (auto& gp : ctx->groups)
-    if (gp->kind == GK_TREE && gp->size <= NEWT_TREE_TINY) (gp->size < NEWT_TREE_TINY ? tiny : small) += gp->n;
-  const bool tiny_many = tiny > 80L * sm_count(ctx), small_many = small > 120L * sm_count(ctx);
-  auto by_threads = [&](int size) {
-    return size < NEWT_TREE_TINY ? tiny_many : size == NEWT_TREE_TINY && small_many;
-  };
-  const int buckets[5] = {NEWT_TREE_TINY, 8, 16, 32, 65};
+  const int buckets[4] = {8, 16, 32, 65};
   for (int bucket : buckets) {
     std::vector<TreeGroupDev> tg;
-    const bool threads = bucket == NEWT_TREE_TINY;
-    const int chunk = threads ? NEWT_TREE_THREADS : newt_tree_item_worlds();
+    const int chunk = newt_tree_item_worlds();
     int most = 0, serial = 1;
     std::vector<HostGroup*> gs;
     for (auto& gp : ctx->groups)
-      if (gp->n > 0 && gp->kind == GK_TREE &&
-          (by_threads(gp->size) ? NEWT_TREE_TINY : newt_tree_bucket(gp->size)) == bucket)
-        gs.push_back(gp.get());
+      if (gp->n > 0 && gp->kind == GK_TREE && newt_tree_bucket(gp->size) == bucket) gs.push_back(gp.get());
     if (gs.empty()) continue;
     std::stable_sort(gs.begin(), gs.end(), [](HostGroup* a, HostGroup* b) { return a->size > b->size; });
     size_t items = 0;
@@ -294,7 +273,7 @@ static int capture(newt_gpu_ctx* ctx, int n_steps, GraphPart part, StepGraph& ou
       }
       tg.push_back(g->tree_dev());
     }
-    TreeLaunch L{most, serial, nullptr, nullptr, (int)items, threads};
+    TreeLaunch L{most, serial, nullptr, nullptr, (int)items};
     CKS(newt_tree_lanes_prepare());
     CKS(cudaMalloc(&L.dg, tg.size() * sizeof(TreeGroupDev)));
     CKS(cudaMemcpy(L.dg, tg.data(), tg.size() * sizeof(TreeGroupDev), cudaMemcpyHostToDevice));
@@ -392,7 +371,7 @@ static int capture(newt_gpu_ctx* ctx, int n_steps, GraphPart part, StepGraph& ou
     }
   if (!tcs.empty() && !ctx->tcstream) CKS(cudaStreamCreateWithFlags(&ctx->tcstream, cudaStreamNonBlocking));
 
-  cudaEvent_t fork = nullptr, join[5] = {}, tjoin = nullptr;
+  cudaEvent_t fork = nullptr, join[4] = {}, tjoin = nullptr;
   CKS(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
   for (size_t k = 0; k < tls.size(); ++k) {
     if (!ctx->side[k]) CKS(cudaStreamCreateWithFlags(&ctx->side[k], cudaStreamNonBlocking));
@@ -454,8 +433,7 @@ static int capture(newt_gpu_ctx* ctx, int n_steps, GraphPart part, StepGraph& ou
   for (size_t k = 0; k < tls.size(); ++k) {
     const TreeLaunch& L = tls[k];
     cudaStreamWaitEvent(ctx->side[k], fork, 0);
-    if (L.threads) newt_launch_tree_threads(L.dg, L.dq, L.items, n_steps, ctx->side[k]);
-    else newt_launch_tree_lanes(L.dg, L.dq, L.items, L.L, L.serial, n_steps, ctx->tune_tree_grid_pct, ctx->side[k]);
+    newt_launch_tree_lanes(L.dg, L.dq, L.items, L.L, L.serial, n_steps, ctx->tune_tree_grid_pct, ctx->side[k]);
     cudaEventRecord(join[k], ctx->side[k]);
   }
   const int pile_launches = (int)(ctx->launches - before) + batched_launches;

@@ -14,7 +14,7 @@
 // The plain form (`tree_aba_kernel`, `tree_integrate_kernel`): one launch per
 // stage per step with state round-tripping through HBM; also the stages
 // around the tree-contact solve.  The batched form of trees without contact
-// is tree_lanes.cu, and for very many of the smallest tree_threads_kernel.
+// is tree_lanes.cu.
 #include "common.cuh"
 #include "groups.h"
 #include "../../include/newt_gpu.h"
@@ -249,36 +249,6 @@ __device__ __forceinline__ bool finite_all(const float* a, int n) {
 
 }  // namespace
 
-// Batched form of the smallest trees, very many of them: a thread per world
-// for the whole horizon, the state kept on chip.  One block per item (group,
-// first world, count) of a queue.
-template <int MAXL>
-__global__ void __launch_bounds__(NEWT_TREE_THREADS) tree_threads_kernel(const TreeGroupDev* __restrict__ groups,
-                                                                         const int* __restrict__ queue, int n_steps) {
-  const TreeGroupDev g = groups[queue[3 * blockIdx.x]];
-  const int w = queue[3 * blockIdx.x + 1] + (int)threadIdx.x;
-  if ((int)threadIdx.x >= queue[3 * blockIdx.x + 2] || w >= g.n || !g.live[w]) return;
-  const int cap = g.cap, nq = g.nq, nv = g.nv;
-  float q[MAXL + 6], qd[MAXL + 5], qf[MAXL + 5], qdd[MAXL + 5];
-  for (int k = 0; k < nq; ++k) q[k] = g.q[k * cap + w];
-  for (int k = 0; k < nv; ++k) { qd[k] = g.qd[k * cap + w]; qf[k] = g.qfrc[k * cap + w]; qdd[k] = 0.f; }
-  LinkScratch scr[MAXL];
-  bool ok = true;
-  const bool rk4 = is_rk4(g, w);
-  for (int s = 0; s < n_steps; ++s) {
-    if (rk4) {
-      ok = tree_rk4<MAXL>(g, w, q, qd, qf, qdd, scr) && ok;
-    } else {
-      ok = tree_aba<MAXL>(g, w, q, qd, qf, qdd, scr, g.dtg[w]) && ok;
-      tree_integrate<MAXL>(g, w, q, qd, qdd);
-    }
-  }
-  const unsigned st = (ok ? 0u : NEWT_WS_NOT_PD) | (finite_all(q, nq) && finite_all(qd, nv) ? 0u : NEWT_WS_NONFINITE);
-  for (int k = 0; k < nq; ++k) g.q[k * cap + w] = q[k];
-  for (int k = 0; k < nv; ++k) { g.qd[k * cap + w] = qd[k]; g.qacc[k * cap + w] = qdd[k]; }
-  if (st) g.status[w] |= st;
-}
-
 // Plain form, stage 1+2: forward dynamics from HBM state into HBM qacc.
 template <int MAXL>
 __global__ void __launch_bounds__(128) tree_aba_kernel(TreeGroupDev g) {
@@ -341,11 +311,6 @@ __global__ void __launch_bounds__(128) tree_integrate_kernel(TreeGroupDev g) {
 
 // Host-side launchers (MAXL buckets 8, 16, 32, 65).
 #define NEWT_TREE_BUCKETS(X) X(8) X(16) X(32) X(65)
-
-extern "C" void newt_launch_tree_threads(const TreeGroupDev* dgroups, const int* dqueue, int n_items, int n_steps,
-                                         cudaStream_t st) {
-  if (n_items > 0) tree_threads_kernel<NEWT_TREE_TINY><<<n_items, NEWT_TREE_THREADS, 0, st>>>(dgroups, dqueue, n_steps);
-}
 
 extern "C" int newt_tree_bucket(int L) { return L <= 8 ? 8 : L <= 16 ? 16 : L <= 32 ? 32 : 65; }
 
