@@ -577,6 +577,7 @@ TcGroupDev HostGroup::tc_dev() const {
   d.scr = (float*)plain_scratch;
   d.sstride = scr_stride;
   d.list = tc_list;
+  d.here = 0;
   d.sens = nullptr;
   d.sens_stride = 0;
   return d;

@@ -37,7 +37,7 @@ struct TreeGroupDev {
   const int* integ;    // 1    NEWT_INTEGRATOR_* (null: Euler for every world)
   float* cfrc;         // tree-contact groups: the contact solve's J^T f / dt (nv per world, stride
   long cstride;        // `cstride` floats, in the solver scratch); null for trees without geoms
-  int* zero;           // tree-contact groups: two counters that the integration sets to zero; null otherwise
+  int* zero;           // tree-contact groups: three counters that the integration sets to zero; null otherwise
   // per-world state (SoA)
   float* q;     // nq  (newt layout: free root p xyz, quat xyzw; hinge angle)
   float* qd;    // nv  (free root: omega_body, v_body; hinge rate)
@@ -72,8 +72,9 @@ struct TcGroupDev {
   const int* iters;  // per world
   float* scr;        // world-major solver scratch
   long sstride;      // floats per world in `scr`
-  int* list;         // how many worlds have more than 32 rows, how many of them are taken (both zero
-                     // between env-steps), then the worlds
+  int* list;         // listed worlds, how many of them are taken, worlds of more than 32 rows (zero between
+                     // env-steps), then the list
+  int here;          // of those worlds, the first so many are solved in their blocks, the others listed
   // the contact sensors' re-solve (null in a step): the last step's contacts
   // solved again at the current state; per world (stride `sens_stride`)
   // each link's contact wrench (world force, torque about its COM), then per
@@ -97,7 +98,7 @@ struct PileLayout {
 };
 
 // How a pile group's contacts are solved: PGS over the pyramidal facet rows
-// (condim 3 everywhere, the island-class and world-persistent kernels), the
+// (condim 3 everywhere, the island-class and batched kernels), the
 // dense Newton solve (pile_newton.cu), or PGS over newt's general rows
 // (elliptic cone, condim 1, 4 or 6: pile_general.cu).
 enum PileSolve { PS_PGS = 0, PS_NEWTON = 1, PS_GENERAL = 2 };

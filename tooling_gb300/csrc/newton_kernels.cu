@@ -5,7 +5,8 @@
 //   tree_aba_kernel        thread per world (tree_kernels.cu): a_free, the
 //                          ABA with the implicit damping fold, into qacc
 //   tc_k_small, tc_k_solve warp per world (trees of up to 24 DoF with facet
-//                          and normal rows, tc_small.cuh; the others, this
+//                          and normal rows, tc_small.cuh, many worlds' of more
+//                          than 32 rows by tc_k_listed; the others, this
 //                          file): forward kinematics,
 //                          link-plane contacts, link COM Jacobians and the
 //                          mass matrix, its Cholesky factors, the Jacobian
@@ -1079,7 +1080,7 @@ __global__ void __launch_bounds__(32, 16) tc_k_listed(const __grid_constant__ Tc
     if (threadIdx.x == 0) k = n > 0 ? atomicAdd(G.list + 1, 1) : n;
     k = __shfl_sync(FULL, k, 0);
     if (k >= n) return;
-    tc_world<false>(G, G.list[2 + k], tcs, true, threadIdx.x);
+    tc_world<false>(G, G.list[3 + k], tcs, true, threadIdx.x);
     __syncwarp();
   }
 }
@@ -1107,6 +1108,10 @@ extern "C" size_t newt_tc_smem_bytes(int L, int nv, int maxc, int rpc) {
 // start before the slowest small world is done (128 fallen quadrupeds of up to
 // 84 rows: all in blocks of four 1430 us, listed 990, so 740; a warp per world
 // 850.  2000 worlds of 28 to 36 rows: 688 in blocks of their own, listed 558).
+// From TCS_MANY worlds an SM on, where later blocks hide a few long solves, one
+// world in sixteen may be solved in its block before the others are listed:
+// 16384 quadrupeds of which a few have fallen 816 us an env-step with all in
+// their blocks, 954 with all listed, 821 so.
 struct TcPlan { bool small, list; int warps; size_t bytes; };
 static TcPlan tc_plan(int L, int nv, int maxc, int rpc, bool general, bool resolve, bool few) {
   TcPlan p{nv <= REFINE_NV && !general && !resolve, false, 1, newt_tc_smem_bytes(L, nv, maxc, rpc)};
@@ -1148,6 +1153,7 @@ static int newt_launch_tc_solve(const TcGroupDev& G, int sms, cudaStream_t st) {
   if (p.small) {
     TcGroupDev D = G;
     if (!p.list) D.list = nullptr;
+    else if (n >= TCS_MANY * sms) D.here = n / 16;
     cudaLaunchConfig_t c{};
     c.gridDim = dim3((n + p.warps - 1) / p.warps);
     c.blockDim = dim3(32 * p.warps);
@@ -1205,8 +1211,8 @@ extern "C" int newt_tc_prepare(newt_gpu_ctx* ctx, HostGroup* g, int n_steps) {
     if (g->tc_list) cudaFree(g->tc_list);
     g->tc_list = nullptr;
     g->tc_list_cap = 0;
-    CKT(cudaMalloc(&g->tc_list, sizeof(int) * (size_t)(g->cap + 2)));
-    CKT(cudaMemset(g->tc_list, 0, 2 * sizeof(int)));
+    CKT(cudaMalloc(&g->tc_list, sizeof(int) * (size_t)(g->cap + 3)));
+    CKT(cudaMemset(g->tc_list, 0, 3 * sizeof(int)));
     g->tc_list_cap = g->cap;
     ctx->graph_dirty = true;
   }

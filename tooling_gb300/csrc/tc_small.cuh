@@ -22,7 +22,7 @@
 //     its line search are reduced together.
 // Measured on 16384 quadrupeds (13 links, 18 DoF, 0 to 28 rows; GB300, a
 // launch): 1737 us as tc_k_solve, 32000 instructions a world at 14.4 cycles
-// each; 379 us here, 10400 at 10.3 (fetch waits 1.1, global memory 2.1, shared
+// each; 376 us here, 10400 at 10.2 (fetch waits 1.0, global memory 1.8, shared
 // memory 1.1, barriers 1.0).  Blocks of four worlds, four to an SM, against
 // eight and two: 917 and 939 us for two env-steps; without the barriers around
 // the Newton stage 932 to 948.
@@ -30,6 +30,7 @@
 constexpr int TCS_WARPS = 4;   // worlds (warps) per block
 constexpr int TCS_BLOCKS = 4;  // blocks per SM
 constexpr int TCS_FEW = 8;     // worlds per SM up to which each has a block of its own
+constexpr int TCS_MANY = 64;   // worlds per SM from which a few large ones are solved in their blocks
 constexpr int TCS_ROWS = 32;  // rows of a world, a lane each
 constexpr int TCS_LDH = 36;   // row stride of H: float4 loads of eight rows meet no bank twice
 
@@ -447,7 +448,7 @@ __global__ void __launch_bounds__(32 * TCS_WARPS, TCS_BLOCKS) tc_k_small(const _
   int ncon = 0, nr = 0;
   const bool live = w < g.n && g.live[w];  // uniform per warp, as every condition on it below
   float dt = 0.f;
-  bool rk4 = false;
+  bool rk4 = false, here = false;
 
   // ---- forward kinematics, joint axes and levers ----
   PairGeoms first;
@@ -486,11 +487,16 @@ __global__ void __launch_bounds__(32 * TCS_WARPS, TCS_BLOCKS) tc_k_small(const _
       rows_solve_any(G, w, sv, nr, ncon, status, lane);
       return;
     }
-    if ((nr == 0 || nr > TCS_ROWS) && lane == 0 && status) atomicOr(g.status + w, status);
-    if (nr > TCS_ROWS && lane == 0) G.list[2 + atomicAdd(G.list, 1)] = w;
+    if (nr > TCS_ROWS) {
+      int before = 0;
+      if (lane == 0 && G.here > 0) before = atomicAdd(G.list + 2, 1);
+      here = __shfl_sync(FULL, before, 0) < G.here;
+      if (!here && lane == 0) G.list[3 + atomicAdd(G.list, 1)] = w;
+    }
+    if ((nr == 0 || (nr > TCS_ROWS && !here)) && lane == 0 && status) atomicOr(g.status + w, status);
   }
   bool on = nr > 0 && nr <= TCS_ROWS;  // without rows qacc stays a_free
-  if (!__syncthreads_or(on)) return;
+  if (!__syncthreads_or(on || here)) return;
 
   // ---- link COM Jacobians, world inertias and masses, lane per link; M ----
   if (on) {
@@ -715,6 +721,8 @@ __global__ void __launch_bounds__(32 * TCS_WARPS, TCS_BLOCKS) tc_k_small(const _
         done = newton_any(H, hd, nr, wf + lay.H, wf + lay.LH, reinterpret_cast<double*>(wf + lay.LHd), lay.ld, bias,
                           iters, __any_sync(FULL, facet && mu == 0.f), lane, &x, &status);
     }
+  } else if (here) {
+    rows_solve_any(G, w, sv, nr, ncon, status, lane);
   }
   __syncthreads();
 

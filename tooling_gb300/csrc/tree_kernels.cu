@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(128) tree_aba_kernel(TreeGroupDev g) {
 template <int MAXL>
 __global__ void __launch_bounds__(128) tree_integrate_kernel(TreeGroupDev g) {
   const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w < 2 && g.zero) g.zero[w] = 0;
+  if (w < 3 && g.zero) g.zero[w] = 0;
   if (w >= g.n || !g.live[w]) return;
   const bool rk4 = is_rk4(g, w);
   if (rk4 && !g.cfrc) return;  // stepped whole by the ABA stage
