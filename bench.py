@@ -52,9 +52,9 @@ PGS_FLOP_PER_CONTACT_SWEEP = 5 * 235
 # DRAM bytes (read + write) per world and env-step of pile_k_contacts and
 # pile_k_sweep, from the ncu captures summarised in
 # profiles/batched_kernels_sections.md (8192 settled worlds, one env-step:
-# 39.0 MB read + 40.3 MB written, 75.7 MB read + 1.8 MB written), scaled by
+# 39.0 MB read + 39.8 MB written, 75.7 MB read + 1.8 MB written), scaled by
 # worlds x env-steps
-BATCHED_DRAM_BYTES_PER_WORLD_STEP = (39.012608e6 + 40.318208e6 + 75.677952e6 + 1.83552e6) / 8192
+BATCHED_DRAM_BYTES_PER_WORLD_STEP = (38.992128e6 + 39.775744e6 + 75.683840e6 + 1.825280e6) / 8192
 
 
 def pinned_like(a):
@@ -583,7 +583,7 @@ def run_gpu_quadruped(args, rank, ws, local, dist):
         "config": {"workload": "quadruped: floating torso + 4x3 revolute legs on a plane, Newton <= 20 iterations, "
                                "dt 2e-3, tau ~ N(0,2) resampled every 20 steps",
                    "worlds_per_gpu": W, "dof": int(batch.nv[0]), "env_steps_per_bench_step": S,
-                   "mode": "3 kernels per env-step (ABA, warp-per-world contact solve, integrate)",
+                   "mode": "4 kernels per env-step (ABA, warp-per-world contact solve in two, integrate)",
                    "l2": "flushed between timed steps (working set also exceeds L2)",
                    "parallelism": f"replicas x{ws}", "contacts_per_world_end": contacts},
         "e2e": {"value": e2e, "unit": "env-steps/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
@@ -604,8 +604,8 @@ def run_gpu_quadruped(args, rank, ws, local, dist):
 
 def run_gpu_uneven(args, rank, ws, local, dist):
     """Uneven batch: chains and piles with 2..64 bodies (log-uniform), PGS 50,
-    dt 2e-3.  The batched form (tree persistent kernels per size bucket plus
-    one pile table over every size, captured in a CUDA graph) is timed beside
+    dt 2e-3.  The batched form (one tree launch per size bucket, two pile
+    launches per env-step and size class, in a CUDA graph) is timed beside
     the plain form (one launch per stage per size group) on the same worlds
     from the same start state."""
     from tooling_gb300 import build as B
@@ -697,7 +697,7 @@ def run_gpu_uneven(args, rank, ws, local, dist):
                    "worlds_per_gpu": W, "chains": W - n_piles, "piles": n_piles, "env_steps_per_bench_step": S,
                    "horizon": f"env-steps 0..{S * args.steps} from the start state (piles fall and settle)",
                    "autotuned": tuned,
-                   "mode": "batched: tree persistent kernels per size bucket + one pile table, CUDA graph",
+                   "mode": "batched: one tree launch per size bucket, two pile launches per env-step and size class, CUDA graph",
                    "l2": "flushed between timed steps", "parallelism": f"replicas x{ws}"},
         "plain_value": plain, "batched_over_plain": value / ws / plain,
         "plain_launches_per_bench_step": plain_launches / args.steps,
@@ -708,8 +708,8 @@ def run_gpu_uneven(args, rank, ws, local, dist):
         "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": hbm, "unit": "GB/s",
                      "frac": achieved / hbm if achieved else None, "traffic": None, "peak_source": src,
                      "algorithmic_bytes_per_launch": alg, "ms_per_launch": dom_ms,
-                     "note": "pile kernels timed live inside the graph; the tree persistent kernels run "
-                             "concurrently on a second branch"},
+                     "note": "pile kernels timed live inside the graph; the tree launches run "
+                             "concurrently on branches of their own"},
         "status_flags": int(np.bitwise_or.reduce(st)) if len(st) else 0,
     }
     eng.close()

@@ -191,18 +191,20 @@ NEWT_API int newt_gpu_set_qfrc(newt_gpu_ctx* ctx, const int32_t* slots, int32_t 
 
 /* Replaces `World::step()` (newt/src/world.rs:1459) for every live world.
  * mode NEWT_STEP_PLAIN: one launch per stage per step, fixed tiles.
- * mode NEWT_STEP_BATCHED: the whole call captured in one CUDA graph and
- *   replayed: trees run the horizon in one persistent launch per size bucket
- *   over a cost-sorted queue; pile worlds of every size run two launches per
- *   env-step and size class (contacts, then sweeps and integration, over a
- *   queue sorted by the previous call's cost, most costly first), each class
- *   on a branch of the graph; tree-contact worlds run three or four kernels per env-step on a
- *   branch of the graph.  newt_gpu_autotune may instead pick the
+ * mode NEWT_STEP_BATCHED: the call captured in a CUDA graph and replayed
+ *   (calls of more than 128 env-steps with piles or tree-contact worlds: a
+ *   graph of 128 and one of the rest): trees run the horizon in one launch per
+ *   size bucket over a queue of the largest first; pile worlds of every size
+ *   run two launches per env-step and size class (contacts, then sweeps and
+ *   integration, over a queue sorted by the previous call's cost, most costly
+ *   first), each class on a branch of the graph; tree-contact worlds run three
+ *   kernels per env-step on a branch of the graph, four with many trees of up
+ *   to 24 DoF.  newt_gpu_autotune may instead pick the
  *   island-class pipeline for piles (collide, island-class solvers on forked
  *   streams, integrate, per env-step).  Pile worlds under the Newton solver
  *   (solve_free_body_newton_impulses, newt/src/solver.rs:1295-1407) run
- *   collide, a dense Newton solve (a warp per world) and integrate per
- *   env-step in both modes. */
+ *   collide, a dense Newton solve (a block per world by its rows) and
+ *   integrate per env-step in both modes. */
 #define NEWT_STEP_PLAIN 0
 #define NEWT_STEP_BATCHED 1
 NEWT_API int newt_gpu_step(newt_gpu_ctx* ctx, int32_t n_steps, int32_t mode);
@@ -356,8 +358,9 @@ NEWT_API int newt_gpu_flush_l2(newt_gpu_ctx* ctx);                              
 NEWT_API int64_t newt_gpu_launch_count(const newt_gpu_ctx* ctx);
 /* Times the batched step's launch choices on the live worlds (piles in the
  * batched launches in each of their shapes -- 8, 16 or 32 lanes per world in
- * the sweeps, 2, 4, 6 or 8 warps per block in the contact stage -- or in the island-class pipeline with 1, 2 or 3 world-range branches; tree
- * persistent grid at full or half residency), `n_steps` env-steps per trial,
+ * the sweeps, 2, 4, 6 or 8 warps per block in the contact stage -- or in the
+ * island-class pipeline with 1, 2 or 3 world-range branches; tree blocks at
+ * full or half residency), `n_steps` env-steps per trial,
  * and keeps the fastest for later NEWT_STEP_BATCHED calls.  `horizon` is how
  * many env-steps the caller means to run next (<= 0: 8 x n_steps): every
  * choice is timed from three snapshots of every world -- as they are, and
@@ -372,7 +375,7 @@ NEWT_API int64_t newt_gpu_launch_count(const newt_gpu_ctx* ctx);
 NEWT_API int newt_gpu_autotune(newt_gpu_ctx* ctx, int32_t n_steps, int32_t horizon, int32_t* choice);
 /* Sets the batched step's launch choices directly, in newt_gpu_autotune's
  * `choice` layout: [0] pile world-range branches of the island-class
- * pipeline (0: by world count), [1] tree persistent grid percent, [2]
+ * pipeline (0: by world count), [1] tree residency percent, [2]
  * ignored, [3] 1 for the batched pile launches, 0 for the pipeline,
  * [4] its shape index (newt_gpu_autotune).  No counterpart in newt. */
 NEWT_API int newt_gpu_set_launch_choice(newt_gpu_ctx* ctx, const int32_t* choice);

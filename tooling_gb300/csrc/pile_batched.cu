@@ -53,8 +53,8 @@
 //
 // Measured (GB300, us an env-step, one warp per world for the whole horizon
 // before -> now): ten worlds of 16 bodies 206 -> 88, 8192 of 16 bodies
-// 1100 -> 505, 700 of 53 bodies 790 -> 252, 1500 of 12 capsules (RK4)
-// 196 -> 97.
+// 1100 -> 493, 700 of 53 bodies 790 -> 247, 1500 of 12 capsules (RK4)
+// 196 -> 96.
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
@@ -303,7 +303,7 @@ __device__ __noinline__ void row_update_far(float4* x, int stride, float* A, boo
 // one before it updates, its rows' bodies a round before that and its bounds
 // one more.  Contacts between boxes come in fours on the same two bodies, so
 // stacks and walls have as many rounds: us an env-step with every far row read
-// in its own round, and now (the world-persistent kernel in brackets): 1000
+// in its own round, and now (one warp per world for the whole horizon in brackets): 1000
 // walls of 8 boxes 1203, 643 (849), of 16 2135, 1474 (1544), 8192 of 16 9123,
 // 5829 (8382), 1000 stacks of 16 1655, 877 (1187).
 // The lane's world: `fit` of its nact rows lie at `mine`, all at `rec`; nr

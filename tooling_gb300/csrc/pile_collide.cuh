@@ -202,8 +202,10 @@ NEWT_D void collide(const WsLay& L, float* wf, int* wi, int lane, Put put) {
   __syncwarp();
   // ordered pair list, rows a ascending, b > a ascending: a lane per geom b
   // tests it against each a in turn and a ballot places the pairs.  Body geoms
-  // pair where their AABBs meet, of geoms 0..63; every body geom pairs with
-  // every plane.  (Sorting the geoms, scanning forward and then listing the
+  // pair where their AABBs meet, of geoms 0..63 (the width of the sort that
+  // this took the place of; a 64-body world's last body beside a plane meets
+  // planes alone, a known divergence from newt that tests hold); every body
+  // geom pairs with every plane.  (Sorting the geoms, scanning forward and then listing the
   // marked pairs took a serial scan per lane and more instructions up to the
   // largest worlds; us an env-step of the batched form, before -> now: ten
   // worlds of 16 bodies 92 -> 88, 8192 of 16 555 -> 505, 700 of 53 309 -> 289.)

@@ -181,7 +181,7 @@ struct newt_gpu_ctx {
   // island-class streams and four fork/join events
   static constexpr int PILE_BRANCHES = 3;
   // launch choices of the batched form (newt_gpu_autotune): pile branches
-  // (0: by world count), tree persistent grid in percent of full residency
+  // (0: by world count), tree blocks in percent of full residency
   int tune_branches = 0, tune_tree_grid_pct = 100;
   // pile worlds in the batched form: 1 = two launches per env-step over a
   // cost-sorted queue (pile_batched.cu), 0 = the island-class pipeline per

@@ -2,9 +2,10 @@
 //
 // Plain form (the drop-in baseline): every group is launched separately,
 // one launch per stage per env-step with fixed tiles.
-// Batched form: the whole call is captured once in a CUDA graph and
-// replayed.  Trees run their horizon in one persistent launch per size
-// bucket, pulling work items from a device queue sorted by size class;
+// Batched form: the call is captured once in a CUDA graph and replayed (a
+// long one as a graph for its pieces and one for its end).  Trees run their
+// horizon in one launch per size bucket, a block per item of a device queue
+// of the largest first;
 // pile worlds run two launches per env-step and size class over a
 // cost-sorted queue (pile_batched.cu; the island-class pipeline, one launch
 // per stage per env-step, stays available to the autotuner); tree-contact
@@ -543,8 +544,8 @@ int autotune_batched(newt_gpu_ctx* ctx, int n_steps, int horizon, int32_t* choic
     return NEWT_OK;
   };
   // piles: the batched launches in each shape (lanes per world in the
-  // sweeps, warps per block in the contact stage), or the island-class pipeline with 1, 2 or 3 world-range branches; trees: full
-  // or half persistent grid
+  // sweeps, warps per block in the contact stage), or the island-class
+  // pipeline with 1, 2 or 3 world-range branches; trees: full or half residency
   struct Cand { int fused, shape, branches, grid_pct; };
   const Cand cands[] = {{1, 0, 0, 100},  {1, 1, 0, 100}, {1, 2, 0, 100}, {1, 3, 0, 100}, {1, 4, 0, 100},
                         {1, 5, 0, 100},  {1, 6, 0, 100}, {1, 7, 0, 100}, {1, 8, 0, 100}, {1, 9, 0, 100},

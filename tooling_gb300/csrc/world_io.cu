@@ -1,14 +1,16 @@
-// Per-world state I/O: moves chosen rows of the named worlds between the
-// host mirror and the device, so a call that touches k worlds moves k worlds'
-// rows (what newt's World::apply_mujoco_qpos/qvel, newt/src/world.rs:519-623,
-// touches for one world) instead of whole groups.
+// Per-world I/O, of the named worlds' rows alone (what newt's
+// World::apply_mujoco_qpos/qvel, newt/src/world.rs:519-623, touches for one
+// world) instead of whole groups.
 //
-// One call packs every group's segment into one pinned staging buffer, makes
-// one copy and one scatter (or gather) launch per group, then synchronises
-// once; a group whose named worlds are consecutive indices skips the packing
-// and moves by one strided copy.  The packed order follows the device layout so both sides of each
-// launch are coalesced: tree groups keep fields as rows x cap (packed as
-// rows x k), pile groups keep worlds contiguous (packed as k x rows).
+// State and forces are converted on the device from and to the caller's arrays
+// (second half of this file).  Models and accelerations move between the host
+// mirror and the device: one call packs every group's segment into one pinned
+// staging buffer, makes one copy and one scatter (or gather) launch per group,
+// then synchronises once; a group whose named worlds are consecutive indices
+// skips the packing and moves by one strided copy.  The packed order follows
+// the device layout so both sides of each launch are coalesced: tree groups
+// keep fields as rows x cap (packed as rows x k), pile groups keep worlds
+// contiguous (packed as k x rows).
 #include <cuda.h>
 
 #include <algorithm>
@@ -242,8 +244,7 @@ int io_gather(newt_gpu_ctx* ctx, const std::vector<RowMove>& all) {
 // and a hinge's MuJoCo offsets equal newt's (7 and 1 coordinates, 6 and 1
 // rates), so a link's `topo` offsets index both layouts.
 //
-// What bounds a call: latency for few worlds (a copy for the plan, one per
-// array, the launch, the wait), the host's loops over the slots and the link
+// What bounds a call: latency for few worlds (the launch, the wait), the host's loops over the slots and the link
 // for many.  So
 //   * the worlds are taken as runs of consecutive indices in a group, a few
 //     of which describe most calls and travel as kernel parameters (up to
