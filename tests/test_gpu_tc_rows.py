@@ -59,8 +59,10 @@ def test_large_worlds_beside_small_ones(solver):
         tol = max(2 * np.abs(v32 - v64).max(), 1e-4 * np.abs(v64 - v[w]).max())
         assert np.abs(gv[0, w] - v64).max() <= tol, w
         assert np.abs(gq[0, w] - q64).max() <= max(2 * np.abs(q32 - q64).max(), 2e-3 * tol, 2e-7), w
-    hq, hv, _ = _step(P, q, v, 8 * 192 // WORLDS + 1)  # more than eight worlds an SM: blocks of four and the list
-    assert (hq == gq[0]).all() and (hv == gv[0]).all()
+    # more than eight worlds an SM: blocks of four and the list; more than 64: a part of them in the blocks
+    for per_sm in (8, 64):
+        hq, hv, _ = _step(P, q, v, per_sm * 192 // WORLDS + 1)
+        assert (hq == gq[0]).all() and (hv == gv[0]).all()
 
 
 def test_a_large_world_does_not_hold_up_its_neighbours():
